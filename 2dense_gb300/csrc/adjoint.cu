@@ -854,10 +854,9 @@ __global__ void __launch_bounds__(128, 3) k_char_face(AdjParams a, const double*
 #pragma unroll
                 for (int m = 0; m < 5; ++m)
                     lf[m] = fma(M[0][k], F(m, 0), fma(M[1][k], F(m, 1), fma(M[2][k], F(m, 2), M[3][k] * F(m, 3))));
-                double gd[4], d0, d1, d2;
+                double gd[4], d0, d1, d2, B[3];
                 first_differences(lf, gd);
-                betas_g(gd, d0, d1, d2);
-                const double B[3] = {fma(-3.0, gd[1], gd[0]), gd[1] + gd[2], fma(3.0, gd[2], -gd[3])};
+                betas_g(gd, d0, d1, d2, B);
                 WenoTerms wt;
                 weno_terms<true>(gd, d0, d1, d2, wt);
                 const double iN = rcp_nr(wt.N), num = weno_num(wt);
@@ -906,10 +905,9 @@ __global__ void __launch_bounds__(128, 3) k_char_face(AdjParams a, const double*
                 phi[m] = fma(HB[0], F(m, 0), fma(HB[1], F(m, 1), fma(HB[2], F(m, 2), HB[3] * F(m, 3))));
                 sur[m] = sC[8][bi][am(m)] + F(m, 1 + DIR);
             }
-            double gd[4], d0, d1, d2;
+            double gd[4], d0, d1, d2, B[3];
             first_differences(sur, gd);
-            betas_g(gd, d0, d1, d2);
-            const double B[3] = {fma(-3.0, gd[1], gd[0]), gd[1] + gd[2], fma(3.0, gd[2], -gd[3])};
+            betas_g(gd, d0, d1, d2, B);
             WenoTerms wt;
             weno_terms<true>(gd, d0, d1, d2, wt);
             const double iN = rcp_nr(wt.N);

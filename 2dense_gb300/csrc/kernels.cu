@@ -12,11 +12,12 @@
 //      against its array (chk below); one outside sets DENSE_FLAG_BOUNDS in the status word and
 //      is clamped into the array, so a bad index is reported, never dereferenced.
 //
-// All arithmetic is FP64. On GB300 the FP64 pipe, not HBM, bounds every kernel here (about
+// All values are FP64. On GB300 the FP64 pipe, not HBM, bounds what is computed with it (about
 // 4-7 kFLOP per cell-update against 256 B of compulsory traffic), so the kernels are built to
 // minimise FP64 instructions: per-cell split fluxes are computed once per tile into shared
-// memory, Roe averages and eigenvectors once per interface for both signs, and loop-invariant
-// scalars (dt/dx, dt/dy, the GLF wave speed) once per stage.
+// memory, Roe averages and eigenvectors once per interface for both signs, loop-invariant
+// scalars (dt/dx, dt/dy, the GLF wave speed) once per stage, and the fast variant's WENO
+// reconstructions run on the integer pipes (weno_fixed.cuh).
 //
 // Layout in HBM (0-based, padded with 4 ghost layers; I = i + 4, J = j + 4 for interior (i,j)):
 //   cons[v][J][I]  v = 0..3 (rho, rho u, rho v, E)       row pitch P doubles, plane NJp*P
@@ -27,6 +28,7 @@
 
 #include "fastmath.cuh"
 #include "internal.h"
+#include "weno_fixed.cuh"
 
 #ifndef DENSE_VARIANT_STRICT
 #error "DENSE_VARIANT_STRICT must be defined (0 or 1)"
@@ -153,19 +155,10 @@ __device__ __forceinline__ double upwind5(const double lf[5]) {
 
 // WENO reconstruction of a stencil no other interface shares (the characteristic fields).
 template <bool Z> __device__ __forceinline__ double weno_fast(const double lf[5]) {
-    double g[4], d0, d1, d2;
+    double g[4], d0, d1, d2, B[3];
     first_differences(lf, g);
-    betas_g(g, d0, d1, d2);
+    betas_g(g, d0, d1, d2, B);
     return weno_from_d<Z>(lf[2], g, d0, d1, d2);
-}
-
-// Second-difference term of a smoothness indicator, s = 4 ss + 13/3 A^2 (four times ss + 13/12
-// A^2) with A = lm - 2 lc + lr: it depends on one cell and its two neighbours only, so a sweep
-// computes it once per cell and sign and each of the three interfaces that use it reads it (the
-// "-" sign passes its neighbours in mirrored order, as its stencil reads them).
-__device__ __forceinline__ double ind_second(double lm, double lc, double lr) {
-    const double a = fma(-2.0, lc, lm) + lr;
-    return fma(k133 * a, a, 4.0 * kSS);
 }
 
 // The five coefficients of h = sum_k w_k q_k as one 5-point stencil: W[m] lf[m].
@@ -195,10 +188,9 @@ __device__ __forceinline__ void recon_grad(const double lf[5], double g[5]) {
         return;
     }
     constexpr bool Z = REC == DENSE_RECON_WENOZ5;
-    double gd[4], d0, d1, d2;
+    double gd[4], d0, d1, d2, B[3];
     first_differences(lf, gd);
-    betas_g(gd, d0, d1, d2);
-    const double B[3] = {fma(-3.0, gd[1], gd[0]), gd[1] + gd[2], fma(3.0, gd[2], -gd[3])};
+    betas_g(gd, d0, d1, d2, B);
     WenoTerms t;
     weno_terms<Z>(gd, d0, d1, d2, t);
     const double iN = rcp_nr(t.N);
@@ -419,8 +411,8 @@ __device__ __forceinline__ void char_weno_fast_g(const EigFast& e, const double 
     double c[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        double d0, d1, d2;
-        betas_g(gd[k], d0, d1, d2);
+        double d0, d1, d2, B[3];
+        betas_g(gd[k], d0, d1, d2, B);
         c[k] = weno_from_d<true>(lc[k], gd[k], d0, d1, d2);
     }
     const double s = c[0] + c[1] + c[3], d = c[3] - c[0];
@@ -477,16 +469,16 @@ __device__ __forceinline__ void stage_scalars(const Params& p, int irk) {
 // One thread per interface; the tile's per-cell split fluxes are staged in shared memory.
 // xi tile: TX interfaces x TY rows, cells f0+1 .. f0+TX+5; eta tile: TX columns x TY interfaces.
 // Dynamic shared memory of one block, in doubles: the split fluxes sF[8][NL][NC] (F+ of the four
-// components, then F-) and, for the WENO reconstructions of the fast variant, the indicators'
-// second-difference terms sS[8][NL][NC] and the forward differences sG[8][NL][NC] = F(k) - F(k+1)
-// along the sweep of the same cells (F+ then F-): a cell's terms serve up to four interfaces.
+// components, then F-) and, for the WENO reconstructions of the fast variant, the forward
+// differences sG[8][NL][NC] = F(k) - F(k+1) along the sweep of the same cells (F+ then F-): a
+// cell's difference serves four interfaces.
 template <int DIR, int REC, int TX, int TY>
 struct CwTile {
     static constexpr int NL = DIR == 0 ? TY : TY + 5;   // smem rows
     static constexpr int NC = DIR == 0 ? TX + 5 : TX;   // smem columns
     static constexpr int NCELL = NL * NC;
-    static constexpr bool kStageS = FAST && REC != DENSE_RECON_UPWIND5;
-    static constexpr size_t bytes = sizeof(double) * (size_t)NCELL * (kStageS ? 24 : 8);
+    static constexpr bool kStageG = FAST && REC != DENSE_RECON_UPWIND5;
+    static constexpr size_t bytes = sizeof(double) * (size_t)NCELL * (kStageG ? 16 : 8);
 };
 
 // TZ threads share an interface (threadIdx.z): they stage the tile's cells together and each
@@ -498,12 +490,11 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
     if (!p.sc->active) return;
     using L = CwTile<DIR, REC, TX, TY>;
     constexpr int NL = L::NL, NC = L::NC, NCELL = L::NCELL;
-    constexpr bool kStageS = L::kStageS;
+    constexpr bool kStageG = L::kStageG;
     extern __shared__ __align__(16) double dsm[];
     double* const sF = dsm;
-    double* const sS = dsm + 8 * NCELL;
-    double* const sG = dsm + 16 * NCELL;
-    (void)sS; (void)sG; (void)NL;
+    double* const sG = dsm + 8 * NCELL;
+    (void)sG; (void)NL;
     auto at = [&](int r, int c) { return chk(p, r, NL) * NC + chk(p, c, NC); };
     // the thread's place in the tile from its linear index (a TX x TY x TZ block, or the
     // persistent kernel's one-dimensional block of as many threads)
@@ -549,21 +540,15 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
     }
     __syncthreads();
 
-    // phase 1b (fast WENO): the indicators' second-difference terms, once per cell and sign for
-    // the cells with both neighbours in the tile ("+" reads a cell's neighbours as k-1, k, k+1,
-    // "-" as k+1, k, k-1), and the forward differences of the cells with a next neighbour
-    if constexpr (kStageS) {
+    // phase 1b (fast WENO): the forward differences of the cells with a next neighbour
+    if constexpr (kStageG) {
         constexpr int KN = DIR == 0 ? TX + 5 : TY + 5;   // cells along the sweep
+        constexpr int st = DIR == 0 ? 1 : NC;            // neighbour along the sweep
         const int tid = tx + ty * TX + tz * TX * TY;
         for (int e = tid; e < 8 * NCELL; e += TX * TY * TZ) {
-            const int q = e / NCELL, o = e - q * NCELL;
+            const int o = e % NCELL;
             const int k = DIR == 0 ? o % NC : o / NC;
-            if (k == KN - 1) continue;
-            const int st = DIR == 0 ? 1 : NC;             // neighbour along the sweep
-            const double* F = sF + q * NCELL + o;
-            sG[e] = F[0] - F[st];
-            if (k == 0) continue;
-            sS[e] = q < 4 ? ind_second(F[-st], F[0], F[st]) : ind_second(F[st], F[0], F[-st]);
+            if (k < KN - 1) sG[e] = sF[e] - sF[e + st];
         }
         __syncthreads();
     }
@@ -583,17 +568,16 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
                                   fidx<DIR>(p, 0, line, f);
     (void)tape_at;
     [[maybe_unused]] const long long ts = DIR == 0 ? (long long)p.nj * (p.ni + 1) : (long long)(p.nj + 1) * p.ni;
-#pragma unroll
+    // one component's code in a loop: eight copies of the integer reconstruction would not fit the
+    // instruction cache
+#pragma unroll 1
     for (int vz = 0; vz < 4 / TZ; ++vz) {
         const int v = tz + vz * TZ;
         double h;
-        if constexpr (kStageS) {
-            // "+": lf(m) = F+(tile cell t+m), g_m = G+(t+m), substencils centred on t+1, t+2, t+3;
-            // "-": lf(m) = F-(tile cell t+5-m), g_m = F-(t+5-m) - F-(t+4-m) = -G-(t+4-m),
-            // substencils centred on t+4, t+3, t+2
+        if constexpr (kStageG) {
+            // "+": lf(m) = F+(tile cell t+m), g_m = G+(t+m); "-": lf(m) = F-(tile cell t+5-m), g_m =
+            // F-(t+5-m) - F-(t+4-m) = -G-(t+4-m)
             constexpr bool Z = REC == DENSE_RECON_WENOZ5;
-            const double* Sp = sS + v * NCELL;
-            const double* Sm = sS + (4 + v) * NCELL;
             const double* Gp = sG + v * NCELL;
             const double* Gm = sG + (4 + v) * NCELL;
             double gp[4], gm[4];
@@ -602,32 +586,22 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
                 gp[m] = Gp[atk(t + m)];
                 gm[m] = -Gm[atk(t + 4 - m)];
             }
-            const double lp2 = sF[v * NCELL + atk(t + 2)], lm2 = sF[(4 + v) * NCELL + atk(t + 3)];
-            // the value, and for the tape its gradient from the same terms (stencil slot m0:
-            // 0 "+", 5 "-")
-            auto recon_taped = [&](double lf2, const double gd[4], const double B[3], double d0, double d1,
-                                   double d2, int m0) -> double {
-                if constexpr (TAPE) {
+            h = fx::pair<Z>(sF[v * NCELL + atk(t + 2)], gp, sF[(4 + v) * NCELL + atk(t + 3)], gm);
+            if constexpr (TAPE) {
+                // the gradients of the two reconstructions (stencil slots 0 "+" and 5 "-")
+                auto tape_grad = [&](const double gd[4], int m0) {
+                    double d0, d1, d2, B[3], g[5];
+                    betas_g(gd, d0, d1, d2, B);
                     WenoTerms tt;
                     weno_terms<Z>(gd, d0, d1, d2, tt);
                     const double iN = rcp_nr(tt.N);
-                    const double num = weno_num(tt);
-                    double g[5];
-                    weno_grad<Z>(gd, B, d0, d1, d2, tt, num * iN, iN, g);
+                    weno_grad<Z>(gd, B, d0, d1, d2, tt, weno_num(tt) * iN, iN, g);
 #pragma unroll
                     for (int m = 0; m < 5; ++m) tape_at[((m0 + m) * 4 + v) * ts] = g[m];
-                    return fma(num, iN, lf2);
-                } else {
-                    (void)m0; (void)B;
-                    return weno_from_d<Z>(lf2, gd, d0, d1, d2);
-                }
-            };
-            double d0, d1, d2, B[3];
-            betas_staged(gp, Sp[atk(t + 1)], Sp[atk(t + 2)], Sp[atk(t + 3)], d0, d1, d2, B);
-            const double hp = recon_taped(lp2, gp, B, d0, d1, d2, 0);
-            betas_staged(gm, Sm[atk(t + 4)], Sm[atk(t + 3)], Sm[atk(t + 2)], d0, d1, d2, B);
-            const double hm = recon_taped(lm2, gm, B, d0, d1, d2, 5);
-            h = hp + hm;
+                };
+                tape_grad(gp, 0);
+                tape_grad(gm, 5);
+            }
         } else {
             double lp[5], lm[5];
 #pragma unroll

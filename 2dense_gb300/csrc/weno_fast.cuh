@@ -20,23 +20,13 @@ constexpr double kSS = (double)1.0e-6f;       // ss = 1.0e-6, a default-real lit
 // d_k, which that exact binary scale leaves unchanged.
 constexpr double k133 = 13.0 / 3.0;   // 4 x 13/12 (exactly, in binary)
 
-// d_k = 4 (ss + beta_k) from the first differences and the terms s_k = 4 ss + 13/3 A_k^2 (staged
-// once per cell by the component-wise sweeps, whose neighbouring interfaces share them); B[k]
-// the first-order combinations.
-__device__ __forceinline__ void betas_staged(const double g[4], double s0, double s1, double s2, double& d0,
-                                             double& d1, double& d2, double B[3]) {
-    B[0] = fma(-3.0, g[1], g[0]); B[1] = g[1] + g[2]; B[2] = fma(3.0, g[2], -g[3]);
-    d0 = fma(B[0], B[0], s0);
-    d1 = fma(B[1], B[1], s1);
-    d2 = fma(B[2], B[2], s2);
-}
-// The same from the first differences alone (a stencil no other interface shares).
-__device__ __forceinline__ void betas_g(const double g[4], double& d0, double& d1, double& d2) {
+// d_k = 4 (ss + beta_k) from the first differences; B[k] the first-order combinations.
+__device__ __forceinline__ void betas_g(const double g[4], double& d0, double& d1, double& d2, double B[3]) {
     const double A0 = g[0] - g[1], A1 = g[1] - g[2], A2 = g[2] - g[3];
-    const double B0 = fma(-3.0, g[1], g[0]), B1 = g[1] + g[2], B2 = fma(3.0, g[2], -g[3]);
-    d0 = fma(k133 * A0, A0, fma(B0, B0, 4.0 * kSS));
-    d1 = fma(k133 * A1, A1, fma(B1, B1, 4.0 * kSS));
-    d2 = fma(k133 * A2, A2, fma(B2, B2, 4.0 * kSS));
+    B[0] = fma(-3.0, g[1], g[0]); B[1] = g[1] + g[2]; B[2] = fma(3.0, g[2], -g[3]);
+    d0 = fma(k133 * A0, A0, fma(B[0], B[0], 4.0 * kSS));
+    d1 = fma(k133 * A1, A1, fma(B[1], B[1], 4.0 * kSS));
+    d2 = fma(k133 * A2, A2, fma(B[2], B[2], 4.0 * kSS));
 }
 __device__ __forceinline__ void first_differences(const double lf[5], double g[4]) {
 #pragma unroll

@@ -1,0 +1,43 @@
+"""The integer WENO reconstructions (csrc/weno_fixed.cuh), compiled for the host, against long
+double and beside the FP64 form (csrc/weno_fast.cuh): no less exact over smooth, discontinuous and
+rough stencils, and the same answers in every form an input can take."""
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def lines(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("wf") / "driver")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-o", exe,
+                    os.path.join(HERE, "weno_fixed_driver.cpp")], check=True)
+    out = subprocess.run([exe], check=True, stdout=subprocess.PIPE).stdout.decode()
+    return [x.split() for x in out.splitlines()]
+
+
+def test_reciprocal(lines):
+    (worst,) = [float(x[1]) for x in lines if x[0] == "reciprocal"]
+    assert worst <= 2.0 ** -58
+
+
+@pytest.mark.parametrize("kind", range(5))
+@pytest.mark.parametrize("z", [0, 1])
+def test_accuracy(lines, kind, z):
+    """In units of the stencils' largest value S: the centres' sum rounds by 2^-52, the result (at
+    most 4.3 S) by 2.2 x 2^-52, the differences by 2^-52 each with sensitivities of 4 in all: 16 x
+    2^-53. The rms no larger than the FP64 form's on the same stencils."""
+    _, _, _, worst, rms, worst64, rms64 = [x for x in lines if x[0] == "accuracy" and x[1:3] == [str(z), str(kind)]][0]
+    assert float(worst) <= 16 * 2.0 ** -53
+    assert float(rms) <= float(rms64)
+
+
+@pytest.mark.parametrize("z", [0, 1])
+def test_forms(lines, z):
+    """Signs and the two stencils' order leave the bits alone, flat stencils give their centre, a
+    NaN or infinity gives NaN, and magnitudes from 1e-180 to 1e90 keep their accuracy."""
+    _, _, odd, swap, flat, bad, n, scale_err = [x for x in lines if x[0] == "forms" and x[1] == str(z)][0]
+    assert (int(odd), int(swap), int(flat), int(bad)) == (0, 0, 0, 0)
+    assert int(n) > 1000 and float(scale_err) <= 1.0

@@ -1,0 +1,145 @@
+// The integer reconstructions of csrc/weno_fixed.cuh on the host, beside the FP64 form of
+// csrc/weno_fast.cuh, both against long double. Prints one line a check; see test_weno_fixed.py.
+#include <algorithm>
+#include <cmath>
+#include <cstdio>
+#include <limits>
+#include <random>
+
+#include "../2dense_gb300/csrc/weno_fixed.cuh"
+
+#define __device__
+#define __forceinline__ inline
+namespace f64 {
+double rcp_nr(double d) { return 1.0 / d; }
+#include "../2dense_gb300/csrc/weno_fast.cuh"
+template <bool Z> double recon(double lf2, const double g[4]) {
+    double d0, d1, d2, B[3];
+    betas_g(g, d0, d1, d2, B);
+    return weno_from_d<Z>(lf2, g, d0, d1, d2);
+}
+}  // namespace f64
+
+typedef long double ld;
+
+// the reconstruction as weno_mod.f90 writes it
+template <bool Z> ld exact(const double f[5]) {
+    const ld a = f[0], b = f[1], c = f[2], d = f[3], e = f[4], ss = (double)1.0e-6f;
+    const ld is[3] = {13 * (a - 2 * b + c) * (a - 2 * b + c) / 12 + (a - 4 * b + 3 * c) * (a - 4 * b + 3 * c) / 4,
+                      13 * (b - 2 * c + d) * (b - 2 * c + d) / 12 + (b - d) * (b - d) / 4,
+                      13 * (c - 2 * d + e) * (c - 2 * d + e) / 12 + (3 * c - 4 * d + e) * (3 * c - 4 * d + e) / 4};
+    const ld q[3] = {(2 * a - 7 * b + 11 * c) / 6, (-b + 5 * c + 2 * d) / 6, (2 * c + 5 * d - e) / 6};
+    const ld cs[3] = {1, 6, 3}, tau = is[2] - is[0];
+    ld num = 0, den = 0;
+    for (int k = 0; k < 3; ++k) {
+        const ld s = (ss + is[k]) * (ss + is[k]), w = Z ? cs[k] * (1 + tau * tau / s) : cs[k] / s;
+        num += w * q[k];
+        den += w;
+    }
+    return num / den;
+}
+
+struct Stencils {
+    double fp[5], fm[5], gp[4], gm[4];
+    void differences() {
+        for (int m = 0; m < 4; ++m) { gp[m] = fp[m] - fp[m + 1]; gm[m] = fm[m] - fm[m + 1]; }
+    }
+    double size() const {
+        double s = 0;
+        for (int m = 0; m < 5; ++m) s = std::max(s, std::max(std::fabs(fp[m]), std::fabs(fm[m])));
+        return s;
+    }
+};
+
+// kind 0 smooth, 1 one jump of 0.03 to 30 times the level, 2 rough, 3 a flat side beside a jump of up
+// to 3e4 times the level, 4 the same beside 1e12 times the level
+Stencils draw(std::mt19937_64& r, int kind) {
+    std::uniform_real_distribution<double> u(-1, 1);
+    Stencils s;
+    const double level = std::pow(10.0, 2 * u(r)), amp = level * std::pow(10.0, -4 + 4 * u(r));
+    for (double* f : {s.fp, s.fm}) {
+        const double a = u(r), b = u(r), c = u(r), jump = level * std::pow(10.0, 1.5 * u(r));
+        const int j = 1 + (int)(r() % 4);
+        for (int m = 0; m < 5; ++m) {
+            const double x = m - 2.0;
+            f[m] = level * (f == s.fp ? 1.0 : -0.7) + amp * (a * x + 0.3 * b * x * x + 0.1 * c * x * x * x);
+            if (kind == 1 && m >= j) f[m] += jump;
+            if (kind == 2) f[m] += level * u(r);
+            if (kind >= 3) f[m] = m < j ? level : f[m] + jump * (kind == 3 ? 1e3 * u(r) : 1e12);
+        }
+    }
+    s.differences();
+    return s;
+}
+
+template <bool Z> void accuracy(int kind) {
+    std::mt19937_64 r(11 + kind);
+    double worst = 0, worst64 = 0, sum = 0, sum64 = 0;
+    const int n = 100000;
+    for (int t = 0; t < n; ++t) {
+        const Stencils s = draw(r, kind);
+        const ld ref = exact<Z>(s.fp) + exact<Z>(s.fm);
+        const double h = dense::fx::pair<Z>(s.fp[2], s.gp, s.fm[2], s.gm);
+        const double h64 = f64::recon<Z>(s.fp[2], s.gp) + f64::recon<Z>(s.fm[2], s.gm);
+        const double e = (double)fabsl(h - ref) / s.size(), e64 = (double)fabsl(h64 - ref) / s.size();
+        worst = std::max(worst, e); worst64 = std::max(worst64, e64);
+        sum += e * e; sum64 += e64 * e64;
+    }
+    printf("accuracy %d %d %.17g %.17g %.17g %.17g\n", (int)Z, kind, worst, std::sqrt(sum / n), worst64, std::sqrt(sum64 / n));
+}
+
+template <bool Z> void forms() {
+    std::mt19937_64 r(5);
+    int odd = 0, swap = 0, flat = 0, bad = 0, n = 0;
+    double scale_err = 0;
+    for (int t = 0; t < 20000; ++t) {
+        Stencils s = draw(r, t % 5);
+        const double cp = s.fp[2], cm = s.fm[2], h = dense::fx::pair<Z>(cp, s.gp, cm, s.gm);
+        double np[4], nm[4];
+        for (int m = 0; m < 4; ++m) { np[m] = -s.gp[m]; nm[m] = -s.gm[m]; }
+        odd += dense::fx::pair<Z>(-cp, np, -cm, nm) != -h;
+        swap += dense::fx::pair<Z>(cm, s.gm, cp, s.gp) != h;
+        const double zero[4] = {0, -0.0, 0, 0};
+        flat += dense::fx::pair<Z>(cp, zero, cm, zero) != cp + cm;
+        for (double x : {std::numeric_limits<double>::quiet_NaN(), std::numeric_limits<double>::infinity(),
+                         -std::numeric_limits<double>::infinity()}) {
+            Stencils b = s;
+            (t & 1 ? b.gp : b.gm)[(t >> 1) & 3] = x;
+            bad += !std::isnan(dense::fx::pair<Z>(cp, b.gp, cm, b.gm));
+        }
+        // the same differences at any scale: far above ss the weights do not depend on it, far below
+        // they are the linear ones
+        if (t % 5 == 0) {
+            const double p = std::ldexp(1.0, (int)(r() % 900) - 700);
+            Stencils b;
+            for (int m = 0; m < 5; ++m) { b.fp[m] = s.fp[m] * p; b.fm[m] = s.fm[m] * p; }
+            if (b.size() < 1e90 && b.size() > 1e-180) {
+                b.differences();
+                double g = 0;
+                for (int m = 0; m < 4; ++m) g = std::max(g, std::max(std::fabs(b.gp[m]), std::fabs(b.gm[m])));
+                const ld ref = (exact<Z>(b.fp) - b.fp[2]) + (exact<Z>(b.fm) - b.fm[2]);
+                // the differences themselves carry the rounding of their level
+                const double tol = 64 * (std::ldexp(b.size(), -53) + std::ldexp(g, -53));
+                scale_err = std::max(scale_err, (double)(fabsl(dense::fx::pair<Z>(0.0, b.gp, 0.0, b.gm) - ref) / tol));
+                ++n;
+            }
+        }
+    }
+    printf("forms %d %d %d %d %d %d %.17g\n", (int)Z, odd, swap, flat, bad, n, scale_err);
+}
+
+int main() {
+    std::mt19937_64 r(3);
+    double worst = 0;
+    for (int t = 0; t < 2000000; ++t) {
+        dense::fx::u64 n = (r() >> 2) | (1ull << 62);
+        if (t < 64) n = (1ull << 62) + (dense::fx::u64)t;
+        else if (t < 128) n = (1ull << 63) - 1 - (dense::fx::u64)t;
+        const ld e = (ld)dense::fx::reciprocal(n) * (ld)n / ((ld)(1ull << 62) * (ld)(1ull << 63)) - 1;
+        worst = std::max(worst, (double)fabsl(e));
+    }
+    printf("reciprocal %.17g\n", worst);
+    for (int k = 0; k < 5; ++k) { accuracy<false>(k); accuracy<true>(k); }
+    forms<false>();
+    forms<true>();
+}
