@@ -343,95 +343,83 @@ __device__ __forceinline__ void char_weno(const Eig& e, const double F[5][4], do
 // FAST characteristic machinery. The Roe state of the two cells next to an interface from
 // their sqrt(rho) and total enthalpy H = gamma/(gamma-1) p/rho + |u|^2/2 (staged once per cell),
 // with one reciprocal for the three weighted means and one inverse square root giving both
-// alpha0 and 1/alpha0; 1/hh0 = (gamma-1)/alpha0^2. The eigenvector products use the zero and
-// unit entries of the matrices of get_l_r_vec_xi/_eta (scheme_weno5th_SC.f90:277-328, 607-658):
-// the tangential-shear characteristic is F_t - u_t0 F_0, and the back-projection is
+// alpha0 and 1/alpha0; 1/hh0 = (gamma-1)/alpha0^2. With n the normal and t the tangential momentum
+// component, the projection on the left eigenvectors of get_l_r_vec_xi/_eta
+// (scheme_weno5th_SC.f90:277-328, 607-658) is
+//   w = f_n - u_n0 f_0,  q = f_t - u_t0 f_0,  z = f_3 - uu0 f_0 - u_n0 w - u_t0 q,
+//   l_0 = z/(2 hh0) - w/(2 a0),  l_1 = f_0 - z/hh0,  l_2 = q,  l_3 = z/(2 hh0) + w/(2 a0)
+// (9 operations where the rows' products take 13), and the back-projection
 //   h_0 = c0 + c1 + c3,  h_n = u_n0 h_0 + a0 (c3 - c0),  h_t = u_t0 h_0 + c2,
-//   h_3 = H0 (c0 + c3) + a0 u_n0 (c3 - c0) + uu0 c1 + u_t0 c2,
-// with n the normal and t the tangential momentum component.
+//   h_3 = H0 (c0 + c3) + a0 u_n0 (c3 - c0) + uu0 c1 + u_t0 c2.
 struct EigFast {
-    double un0, ut0, a0, h0, uu0, a0un0;
-    double l00, l10, l20, l30;  // column 0 (acoustic, u_n - a)
-    double l01, l11, l21, l31;  // column 1 (entropy)
-    double l03, l13, l23;       // column 3 (acoustic, u_n + a); l33 == l30
+    double un0, ut0, a0, h0, uu0;
+    double ia5, ih, ihh;  // 1/(2 a0), 1/(2 hh0), 1/hh0
 };
 
 template <int DIR>
 __device__ __forceinline__ bool roe_eig_fast(double g1, double sl, double sr, double ul, double ur,
                                              double vl, double vr, double hl, double hr, EigFast& e) {
-    const double r = rcp_nr(sl + sr);
-    const double u0 = fma(sr, ur, sl * ul) * r;
-    const double v0 = fma(sr, vr, sl * vl) * r;
-    const double h0 = fma(sr, hr, sl * hl) * r;
-    const double uu0 = 0.5 * fma(u0, u0, v0 * v0);
-    const double c2 = g1 * (h0 - uu0);
+    const double w = sr * rcp_nr(sl + sr);
+    const double u0 = fma(w, ur - ul, ul);
+    const double v0 = fma(w, vr - vl, vl);
+    e.h0 = fma(w, hr - hl, hl);
+    e.uu0 = 0.5 * fma(u0, u0, v0 * v0);
+    const double c2 = g1 * (e.h0 - e.uu0);
     const double ia = rsqrt_nr(c2);
-    const double a0 = c2 * ia;
-    const double ihh = g1 * ia * ia;
-    const double un0 = DIR == 0 ? u0 : v0, ut0 = DIR == 0 ? v0 : u0;
-    e.un0 = un0; e.ut0 = ut0; e.a0 = a0; e.h0 = h0; e.uu0 = uu0; e.a0un0 = a0 * un0;
-    const double hu = 0.5 * uu0 * ihh, nu = 0.5 * un0 * ia, ia5 = 0.5 * ia;
-    const double pn = 0.5 * un0 * ihh, pt = 0.5 * ut0 * ihh, ih = 0.5 * ihh;
-    // rows of the normal (n) and tangential (t) momentum components
-    const double ln0 = -pn - ia5, ln3 = -pn + ia5;
-    if (DIR == 0) {
-        e.l00 = hu + nu; e.l10 = ln0; e.l20 = -pt;
-        e.l03 = hu - nu; e.l13 = ln3; e.l23 = -pt;
-    } else {
-        e.l00 = hu + nu; e.l10 = -pt; e.l20 = ln0;
-        e.l03 = hu - nu; e.l13 = -pt; e.l23 = ln3;
-    }
-    e.l30 = ih;
-    e.l01 = fma(-uu0, ihh, 1.0); e.l11 = u0 * ihh; e.l21 = v0 * ihh; e.l31 = -ihh;
+    e.a0 = c2 * ia;
+    e.ia5 = 0.5 * ia;
+    e.ih = g1 * ia * e.ia5;
+    e.ihh = 2.0 * e.ih;
+    e.un0 = DIR == 0 ? u0 : v0;
+    e.ut0 = DIR == 0 ? v0 : u0;
     return c2 > 0.0;
 }
 
-// Characteristic-wise WENO-Z at one interface and one sign from the stencil's centre split flux
-// Fc and its first differences dF[m] = F[m] - F[m+1] (m = 0..3): the projection is linear, so the
-// characteristic fields' first differences are the projected differences, and each field's
-// reconstruction works from them directly (weno_from_d).
+// Characteristic fields of a flux (or flux difference) f.
 template <int DIR>
-__device__ __forceinline__ void char_weno_fast_g(const EigFast& e, const double Fc[4], const double dF[4][4],
-                                                 double h[4]) {
-    auto proj = [&](const double f[4], double l[4]) {
-        l[0] = fma(e.l00, f[0], fma(e.l10, f[1], fma(e.l20, f[2], e.l30 * f[3])));
-        l[1] = fma(e.l01, f[0], fma(e.l11, f[1], fma(e.l21, f[2], e.l31 * f[3])));
-        l[2] = fma(-e.ut0, f[0], DIR == 0 ? f[2] : f[1]);
-        l[3] = fma(e.l03, f[0], fma(e.l13, f[1], fma(e.l23, f[2], e.l30 * f[3])));
-    };
-    double lc[4], gd[4][4];
-    proj(Fc, lc);
+__device__ __forceinline__ void project_fast(const EigFast& e, const double f[4], double l[4]) {
+    const double w = fma(-e.un0, f[0], f[1 + DIR]), q = fma(-e.ut0, f[0], f[2 - DIR]);
+    const double z = fma(-e.ut0, q, fma(-e.un0, w, fma(-e.uu0, f[0], f[3])));
+    const double m = e.ia5 * w;
+    l[0] = fma(e.ih, z, -m);
+    l[1] = fma(-e.ihh, z, f[0]);
+    l[2] = q;
+    l[3] = fma(e.ih, z, m);
+}
+
+// Characteristic-wise WENO-Z. The projection is linear, so a field's first differences are the
+// projected differences of the split flux; and the projected centre value, projected back, is the
+// centre flux itself, so that only the reconstructions' corrections pass through the fields:
+//   h = F+(centre) + F-(centre) + sum_k r_k (c_k+ + c_k-),
+// one back-projection for both signs and none of the centres' projections. c[k] takes 6 c_k (added,
+// the "-" stencil's differences read in mirrored order with the opposite sign: neg).
+template <int DIR>
+__device__ __forceinline__ void char_corrections(const EigFast& e, const double dF[4][4], bool neg, double c[4]) {
+    double g[4][4];
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
         double l[4];
-        proj(dF[m], l);
+        project_fast<DIR>(e, dF[m], l);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) gd[k][m] = l[k];
+        for (int k = 0; k < 4; ++k) g[k][m] = l[k];
     }
-    double c[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        double d0, d1, d2, B[3];
-        betas_g(gd[k], d0, d1, d2, B);
-        c[k] = weno_from_d<true>(lc[k], gd[k], d0, d1, d2);
+        // a correction is odd in its differences, to the bit
+        const double x = fx::correction<true>(g[k]);
+        c[k] += neg ? -x : x;
     }
-    const double s = c[0] + c[1] + c[3], d = c[3] - c[0];
-    const double hn = fma(e.un0, s, e.a0 * d);
-    const double ht = fma(e.ut0, s, c[2]);
-    h[0] = s;
-    h[1 + DIR] = hn;
-    h[2 - DIR] = ht;
-    h[3] = fma(e.h0, c[0] + c[3], fma(e.a0un0, d, fma(e.uu0, c[1], e.ut0 * c[2])));
 }
-// The same from the stencil's five split fluxes F[m][c].
 template <int DIR>
-__device__ __forceinline__ void char_weno_fast(const EigFast& e, const double F[5][4], double h[4]) {
-    double dF[4][4];
-#pragma unroll
-    for (int m = 0; m < 4; ++m)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) dF[m][c] = F[m][c] - F[m + 1][c];
-    char_weno_fast_g<DIR>(e, F[2], dF, h);
+__device__ __forceinline__ void back_project_fast(const EigFast& e, const double c[4], const double centre[4],
+                                                  double h[4]) {
+    const double s = c[0] + c[3], d = c[3] - c[0], h0 = s + c[1], ad = e.a0 * d;
+    const double hn = fma(e.un0, h0, ad), ht = fma(e.ut0, h0, c[2]);
+    const double h3 = fma(e.h0, s, fma(e.un0, ad, fma(e.uu0, c[1], e.ut0 * c[2])));
+    h[0] = fma(1.0 / 6.0, h0, centre[0]);
+    h[1 + DIR] = fma(1.0 / 6.0, hn, centre[1 + DIR]);
+    h[2 - DIR] = fma(1.0 / 6.0, ht, centre[2 - DIR]);
+    h[3] = fma(1.0 / 6.0, h3, centre[3]);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -845,13 +833,6 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
 #pragma unroll
             for (int c = 0; c < 4; ++c) F[m][c] = s == 0 ? SF(c, t0 + m, ox, oy) : SF(4 + c, t0 + 5 - m, ox, oy);
     };
-    auto char_recon = [&](const EigT& e, const double F[5][4], double h[4]) {
-#if FAST
-        char_weno_fast<DIR>(e, F, h);
-#else
-        char_weno(e, F, h);
-#endif
-    };
     auto store = [&](const double hsum[4]) {
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
@@ -878,31 +859,37 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
         EigT e;
         eig_at(tx, ty, e);
         double hsum[4];
+#if FAST
+        // "+": centre F+(t+2), differences F+(t+m) - F+(t+m+1) = DF+(t+m); "-": centre
+        // F-(t+3), differences F-(t+5-m) - F-(t+4-m) = -DF-(t+4-m)
+        const int t = DIR == 0 ? tx : ty;
+        double c6[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+        for (int s = 0; s < 2; ++s) {
+            double dF[4][4];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                const int o = atk(s == 0 ? t + m : t + 4 - m, tx, ty);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) dF[m][c] = sDF[(4 * s + c) * NCELL + o];
+            }
+            char_corrections<DIR>(e, dF, s != 0, c6);
+        }
+        double centre[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) centre[c] = SF(c, t + 2, tx, ty) + SF(4 + c, t + 3, tx, ty);
+        back_project_fast<DIR>(e, c6, centre, hsum);
+#else
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
             double h[4];
-#if FAST
-            // "+": centre F+(t+2), differences F+(t+m) - F+(t+m+1) = DF+(t+m); "-": centre
-            // F-(t+3), differences F-(t+5-m) - F-(t+4-m) = -DF-(t+4-m)
-            const int t = DIR == 0 ? tx : ty;
-            double Fc[4], dF[4][4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                Fc[c] = s == 0 ? SF(c, t + 2, tx, ty) : SF(4 + c, t + 3, tx, ty);
-#pragma unroll
-                for (int m = 0; m < 4; ++m)
-                    dF[m][c] = s == 0 ? sDF[c * NCELL + atk(t + m, tx, ty)]
-                                      : -sDF[(4 + c) * NCELL + atk(t + 4 - m, tx, ty)];
-            }
-            char_weno_fast_g<DIR>(e, Fc, dF, h);
-#else
             double F[5][4];
             stencil(tx, ty, s, F);
-            char_recon(e, F, h);
-#endif
+            char_weno(e, F, h);
 #pragma unroll
             for (int c = 0; c < 4; ++c) hsum[c] = s == 0 ? h[c] : hsum[c] + h[c];
         }
+#endif
         store(hsum);
     } else {
         // 105, phase 2a: the AdaWENO indicator from the scalar surrogate rho + F+-(normal
@@ -1063,7 +1050,17 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
             eig_at(ox, oy, e);
             double F[5][4], h[4];
             stencil(ox, oy, s, F);
-            char_recon(e, F, h);
+#if FAST
+            double dF[4][4], c6[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) dF[m][c] = F[m][c] - F[m + 1][c];
+            char_corrections<DIR>(e, dF, false, c6);
+            back_project_fast<DIR>(e, c6, F[2], h);
+#else
+            char_weno(e, F, h);
+#endif
 #pragma unroll
             for (int c = 0; c < 4; ++c) hbuf(s, c, owner) = h[c];
         }
@@ -1485,16 +1482,19 @@ __device__ __forceinline__ void bc_block(const Params& p, int bx) {
 // Kernels of one block (instance) of the solver: block coordinates are the launch's own.
 // Resident blocks the register allocation of a characteristic sweep is sized for. AdaWENO's
 // blocks stall on the barriers of their work queue, which a third block per SM hides (80
-// registers instead of 94, a few bytes spilled: the xi sweep 2 % faster on the 1920 x 480 double
-// Mach reflection); the 104 eta sweep lost 4 % that way and keeps its natural 96 registers.
-constexpr int char_min_blocks(bool adapt) { return adapt ? 3 : 1; }
+// registers, a few bytes spilled; at two blocks the xi sweep of the 1920 x 480 double Mach
+// reflection takes 0.292 instead of 0.282 ms). The 104 sweeps' four inlined integer
+// reconstructions would take 160 registers; at 1024 resident threads (64 registers) the sweeps of
+// the 256 x 1024 Rayleigh-Taylor case take 0.127 (xi) and 0.111 ms (eta), at 768 0.131 and 0.113,
+// unbounded 0.141 and 0.158 -- and 0.340 and 0.293 with the reconstructions in FP64.
+constexpr int char_min_blocks(bool adapt, int nt) { return adapt ? 3 : 1024 / nt; }
 template <int DIR, int SPL, int REC, int TX, int TY, bool TAPE = false, int TZ = 1>
 __global__ void __launch_bounds__(TX* TY* TZ) k_flux_cw(Params p, int irk) {
     grid_dependency_wait();
     flux_cw_block<DIR, SPL, REC, TX, TY, TAPE, TZ>(p, irk, blockIdx.x, blockIdx.y);
 }
 template <int DIR, bool ADAPT, int TX, int TY>
-__global__ void __launch_bounds__(TX* TY, char_min_blocks(ADAPT)) k_flux_char(Params p, int irk) {
+__global__ void __launch_bounds__(TX* TY, char_min_blocks(ADAPT, TX* TY)) k_flux_char(Params p, int irk) {
     grid_dependency_wait();
     flux_char_block<DIR, ADAPT, TX, TY>(p, irk, blockIdx.x, blockIdx.y);
 }
@@ -1536,7 +1536,7 @@ __global__ void __launch_bounds__(TX* TY) kb_flux_cw(const Params* tab, const in
     flux_cw_block<DIR, SPL, REC, TX, TY>(sp, irk, m.y, m.z);
 }
 template <int DIR, bool ADAPT, int TX, int TY>
-__global__ void __launch_bounds__(TX* TY, char_min_blocks(ADAPT)) kb_flux_char(const Params* tab, const int3* map, int irk) {
+__global__ void __launch_bounds__(TX* TY, char_min_blocks(ADAPT, TX* TY)) kb_flux_char(const Params* tab, const int3* map, int irk) {
     DENSE_BATCH_PROLOGUE
     flux_char_block<DIR, ADAPT, TX, TY>(sp, irk, m.y, m.z);
 }

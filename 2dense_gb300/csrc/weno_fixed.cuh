@@ -286,12 +286,12 @@ DENSE_FX double pair(double lp, const double gp[4], double lm, const double gm[4
     const bool first = ap < am || (ap == am && bits(lp) == ap);  // of two opposite ones, the positive
     return fma(c, 1.0 / 6.0, first ? lp : lm) + (first ? lm : lp);
 }
-// One reconstruction.
+// 6 (h - lf_2) of one reconstruction.
 template <bool Z>
-DENSE_FX double single(double centre, const double g[4]) {
+DENSE_FX double correction(const double g[4]) {
     u32 top = 0;
     const u32 eh = scale_of(g, top);
-    return fma(to_double(correction6<Z>(g, eh), eh, top), 1.0 / 6.0, centre);
+    return to_double(correction6<Z>(g, eh), eh, top);
 }
 
 }  // namespace fx
