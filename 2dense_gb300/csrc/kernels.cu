@@ -153,31 +153,15 @@ __device__ __forceinline__ double upwind5(const double lf[5]) {
 // (rcp_nr and rsqrt_nr: fastmath.cuh)
 
 
-// WENO reconstruction of a stencil no other interface shares (the characteristic fields).
-template <bool Z> __device__ __forceinline__ double weno_fast(const double lf[5]) {
-    double g[4], d0, d1, d2, B[3];
-    first_differences(lf, g);
+// AdaWENO's indicator theta = 1/(1 + (sum alpha - 1)^2) from a surrogate's first differences, for the
+// saved indicator (the switch itself: fx::surrogate): sum alpha - 1 = tau^2 Q / D, Q = sum c_k P_k.
+__device__ __forceinline__ double theta_of(const double g[4]) {
+    double d0, d1, d2, B[3];
     betas_g(g, d0, d1, d2, B);
-    return weno_from_d<Z>(lf[2], g, d0, d1, d2);
-}
-
-// The five coefficients of h = sum_k w_k q_k as one 5-point stencil: W[m] lf[m].
-__device__ __forceinline__ void stencil_from_weights(double w0, double w1, double w2, double W[5]) {
-    W[0] = w0 * a300;
-    W[1] = fma(w1, a310, w0 * a301);
-    W[2] = fma(w2, a320, fma(w1, a311, w0 * a302));
-    W[3] = fma(w2, a321, w1 * a312);
-    W[4] = w2 * a322;
-}
-
-// The same 5-point stencil from u0 = w0/c0 and u2 = w2/c2 of WENO-Z weights that sum to one
-// (w1 = 1 - w0 - w2): the linear weights c_k and the candidates' coefficients fold into constants.
-__device__ __forceinline__ void stencil_from_u(double u0, double u2, double W[5]) {
-    W[0] = (c30 * a300) * u0;
-    W[1] = fma(c30 * (a301 - a310), u0, fma(-c32 * a310, u2, a310));
-    W[2] = fma(c30 * (a302 - a311), u0, fma(c32 * (a320 - a311), u2, a311));
-    W[3] = fma(-c30 * a312, u0, fma(c32 * (a321 - a312), u2, a312));
-    W[4] = (c32 * a322) * u2;
+    WenoTerms t;
+    weno_terms<true>(g, d0, d1, d2, t);
+    const double sm1 = t.tau * t.tau * fma(c31, t.P[1], fma(c30, t.P[0], c32 * t.P[2])) / t.D;
+    return 1.0 / (1.0 + sm1 * sm1);
 }
 
 // The gradient of a stencil's reconstruction alone (upwind5's is constant), its terms recomputed.
@@ -197,14 +181,12 @@ __device__ __forceinline__ void recon_grad(const double lf[5], double g[5]) {
     weno_grad<Z>(gd, B, d0, d1, d2, t, weno_num(t) * iN, iN, g);
 }
 
+// One reconstruction (the fast variant's WENO ones: weno_fixed.cuh).
 template <int REC> __device__ __forceinline__ double recon5(const double lf[5]) {
+    static_assert(!FAST || REC == DENSE_RECON_UPWIND5, "fast WENO reconstructions work from differences");
     if (REC == DENSE_RECON_UPWIND5) return upwind5(lf);
-#if FAST
-    return weno_fast<REC == DENSE_RECON_WENOZ5>(lf);
-#else
     if (REC == DENSE_RECON_WENOJS5) return weno5js(lf);
     return weno5z(lf);
-#endif
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -641,12 +623,15 @@ __global__ void k_flux_noop(Params p, int irk) {
 // branch would hold whole warps for the sake of one or two lanes; instead each thread does its
 // smooth signs and queues its characteristic (interface, sign) items in shared memory, and the
 // whole block then works through the queue on full warps.
+// What bounds it: the FP64 pipe. The surrogate's weights and the smooth branch run on the integer
+// pipes (weno_fixed.cuh), which leaves some 55 FP64 instructions an interface of 150 and took the
+// 1920 x 480 double Mach reflection's sweeps from 0.282 and 0.305 ms to 0.159 and 0.180.
 // Dynamic shared memory of one characteristic sweep block, in doubles: the tile's split fluxes
-// sF[8][NL][NC] and primitives sQ[4][NL][NC]; per-cell sqrt(rho) sS (104, fast); and one region
-// R that AdaWENO uses three times over: the scalar surrogates sur[2][NL][NC] and, from them,
-// the staged indicator terms (fast: second differences D2, ss + 13/12 D2^2 and first differences
-// per sign, 6 x [NL][NC]), read by the interfaces; then, after a barrier, the per-sign results
-// hbuf[2][4][NT].
+// sF[8][NL][NC] and primitives sQ[4][NL][NC]; per-cell sqrt(rho) sS (104, fast); the split fluxes'
+// forward differences along the sweep sDF[8][NL][NC] (fast); and one region R that AdaWENO uses
+// twice over: the scalar surrogates sur[2][NL][NC] (fast: their forward differences), read by the
+// interfaces; then, after a barrier, the per-sign results hbuf[2][4][NT] of the interfaces with a
+// characteristic sign.
 template <int DIR, bool ADAPT, int TX, int TY>
 struct CharTile {
     // interfaces of a tile along the sweep (KW): a one-row xi tile of TX threads covers TX - 5
@@ -661,14 +646,11 @@ struct CharTile {
     static constexpr int NT = TX * TY;
     static constexpr int NCELL = NL * NC;
     static constexpr bool kStageHS = FAST && !ADAPT;
-    static constexpr bool kStageInd = FAST && ADAPT;
     static constexpr int kF = 0, kQ = kF + 8 * NCELL, kS = kQ + 4 * NCELL;
-    // 104, fast: the forward differences of the split fluxes along the sweep, F(k) - F(k+1)
+    // fast: the forward differences of the split fluxes along the sweep, F(k) - F(k+1)
     static constexpr int kDF = kS + (kStageHS ? NCELL : 0);
-    static constexpr int kR = kDF + (kStageHS ? 8 * NCELL : 0);
-    static constexpr int kRSize = !ADAPT ? 0
-                                  : (kStageInd ? (8 * NCELL > 8 * NT ? 8 * NCELL : 8 * NT)
-                                               : (2 * NCELL > 8 * NT ? 2 * NCELL : 8 * NT));
+    static constexpr int kR = kDF + (FAST ? 8 * NCELL : 0);
+    static constexpr int kRSize = !ADAPT ? 0 : (2 * NCELL > 8 * NT ? 2 * NCELL : 8 * NT);
     static constexpr size_t bytes = sizeof(double) * (size_t)(kR + kRSize);
 };
 
@@ -677,7 +659,7 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
     if (!p.sc->active) return;
     using L = CharTile<DIR, ADAPT, TX, TY>;
     constexpr int NL = L::NL, NC = L::NC, NT = L::NT, NCELL = L::NCELL;
-    constexpr bool kStageHS = L::kStageHS, kStageInd = L::kStageInd;
+    constexpr bool kStageHS = L::kStageHS;
     extern __shared__ __align__(16) double dsm[];
     double* const sF = dsm + L::kF;
     double* const sQ = dsm + L::kQ;
@@ -717,7 +699,7 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
             sF[(4 + v) * NCELL + at(r, c)] = fm[v];
             sQ[v * NCELL + at(r, c)] = q[v];
         }
-        if constexpr (ADAPT) {  // AdaWENO's scalar surrogates rho + F+-(normal momentum)
+        if constexpr (ADAPT && !FAST) {  // AdaWENO's scalar surrogates rho + F+-(normal momentum)
             sR[at(r, c)] = q[0] + fp[1 + DIR];
             sR[NCELL + at(r, c)] = q[0] + fm[1 + DIR];
         }
@@ -739,46 +721,33 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
     }
     __syncthreads();
 
-    // phase 1b (104, fast): the split fluxes' forward differences along the sweep, once per cell
-    // and sign for the cells with a next neighbour in the tile (each serves four interfaces)
+    // phase 1b (fast): the split fluxes' forward differences along the sweep, once per cell and
+    // sign for the cells with a next neighbour in the tile (each serves four interfaces), and
+    // AdaWENO's surrogates' rho + F+-(normal momentum)
     double* const sDF = dsm + L::kDF;
-    if constexpr (kStageHS) {
+    (void)sDF;
+    if constexpr (FAST) {
         constexpr int KN = L::KW + 5;
         constexpr int st = DIR == 0 ? 1 : NC;            // neighbour along the sweep
-        for (int e = tid; e < 8 * NCELL; e += NT) {
-            const int o = e % NCELL;
-            const int k = DIR == 0 ? o % NC : o / NC;
-            if (k < KN - 1) sDF[e] = sF[e] - sF[e + st];
-        }
-        __syncthreads();
-    }
-
-    // phase 1b (AdaWENO, fast): per cell and sign, the surrogate's second difference
-    // A = sur(k-1) + sur(k+1) - 2 sur(k) (symmetric, so the same for both stencil directions),
-    // four times the squared-difference term ss + 13/12 A^2 of the smoothness indicators, and
-    // the first difference sur(k+1) - sur(k); an interface's indicators then need only their
-    // first-order terms. With the factor 4 (exact in binary) the interfaces add B_k^2 in the
-    // indicator's FMA with no 1/4 product; the weights and the switch compare homogeneous
-    // products of the d_k, which that scale leaves unchanged.
-    double* const sD2 = sR + 2 * NCELL;   // [2][NCELL]: A
-    double* const sA2 = sR + 4 * NCELL;   // [2][NCELL]: 4 (ss + 13/12 A^2)
-    double* const sDl = sR + 6 * NCELL;   // [2][NCELL]: sur(k+1) - sur(k)
-    if constexpr (kStageInd) {
-        constexpr int KN = L::KW + 5;                    // cells along the sweep
-        constexpr int KL = DIR == 0 ? TY : TX;           // lines
-        constexpr double k133 = 13.0 / 3.0;
-        for (int e = tid; e < KL * (KN - 2); e += NT) {
-            const int line = e / (KN - 2), k = 1 + e % (KN - 2);
-            const int o = DIR == 0 ? at(line, k) : at(k, line);
-            const int om = DIR == 0 ? at(line, k - 1) : at(k - 1, line);
-            const int op = DIR == 0 ? at(line, k + 1) : at(k + 1, line);
+        if constexpr (!ADAPT) {
+            for (int e = tid; e < 8 * NCELL; e += NT) {
+                const int o = e % NCELL;
+                const int k = DIR == 0 ? o % NC : o / NC;
+                if (k < KN - 1) sDF[e] = sF[e] - sF[e + st];
+            }
+        } else {
+            for (int o = tid; o < NCELL; o += NT) {
+                const int k = DIR == 0 ? o % NC : o / NC;
+                if (k == KN - 1) continue;
+                double d[8];
 #pragma unroll
-            for (int sg = 0; sg < 2; ++sg) {
-                const double* su = sR + sg * NCELL;
-                const double a = fma(-2.0, su[o], su[om] + su[op]);
-                sD2[sg * NCELL + o] = a;
-                sA2[sg * NCELL + o] = fma(k133 * a, a, 4.0 * kSS);
-                sDl[sg * NCELL + o] = su[op] - su[o];
+                for (int q = 0; q < 8; ++q) {
+                    d[q] = sF[q * NCELL + o] - sF[q * NCELL + o + st];
+                    sDF[q * NCELL + o] = d[q];
+                }
+                const double dr = sQ[o] - sQ[o + st];
+                sR[o] = dr + d[1 + DIR];
+                sR[NCELL + o] = dr + d[5 + DIR];
             }
         }
         __syncthreads();
@@ -833,19 +802,19 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
 #pragma unroll
             for (int c = 0; c < 4; ++c) F[m][c] = s == 0 ? SF(c, t0 + m, ox, oy) : SF(4 + c, t0 + 5 - m, ox, oy);
     };
-    auto store = [&](const double hsum[4]) {
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            (DIR == 0 ? p.hx : p.he)[fidx<DIR>(p, v, line, f)] = hsum[v];
-        }
+    auto store_one = [&](int v, double h) {
+        (DIR == 0 ? p.hx : p.he)[fidx<DIR>(p, v, line, f)] = h;
         if (p.tape) {  // the adjoint's taping recompute: the face fluxes, the last 4 planes a direction
             constexpr int NP = ADAPT ? 5 : 4;
             const long long xs = (long long)p.nj * (p.ni + 1), ts = DIR == 0 ? xs : (long long)(p.nj + 1) * p.ni;
-            double* T = p.tape + (DIR == 0 ? 0 : NP * xs) + (NP - 4) * ts + fidx<DIR>(p, 0, line, f);
-#pragma unroll
-            for (int v = 0; v < 4; ++v) T[v * ts] = hsum[v];
+            p.tape[(DIR == 0 ? 0 : NP * xs) + (NP - 4 + v) * ts + fidx<DIR>(p, 0, line, f)] = h;
         }
     };
+    auto store = [&](const double hsum[4]) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) store_one(v, hsum[v]);
+    };
+    (void)store;
     auto hbuf = [&](int s, int c, int i) -> double& { return sR[(s * 4 + c) * NT + chk(p, i, (int)NT)]; };
     // the indicator of a valid interface and sign into Params::theta (get_theta_*, SC.f90:1-64)
     auto theta_out = [&](int s, double th) {
@@ -897,47 +866,25 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
         // 1-64,330-393), the smooth branch (SC.f90:110-124), and the queue of the rest
         const int t = DIR == 0 ? tx : ty;
         bool smooth[2] = {true, true};
+#if FAST
+        fx::u64 f0[2], f2[2];
+#else
         double wsur[2][3];
+#endif
         if (valid) {
 #if FAST
-#pragma unroll
+            // differences of sign s: "+" g_m = D(t+m), "-" g_m = -D(t+4-m)
+#pragma unroll 1
             for (int s = 0; s < 2; ++s) {
-                // "+": substencils centred on cells t+1, t+2, t+3; "-": on t+4, t+3, t+2
-                const int c0 = s == 0 ? t + 1 : t + 4, c2 = s == 0 ? t + 3 : t + 2, cm = t + 2;
-                const double* D2 = sD2 + s * NCELL;
-                const double* A2 = sA2 + s * NCELL;
-                const double* Dl = sDl + s * NCELL;
-                const double A0 = D2[atk(c0, tx, ty)], A2c = D2[atk(c2, tx, ty)];
-                const double dl1 = Dl[atk(s == 0 ? t + 1 : t + 3, tx, ty)];
-                const double dl2 = Dl[atk(t + 2, tx, ty)];
-                // B0 = lf0 - 4 lf1 + 3 lf2 = A0 +- 2 dl1, B1 = lf1 - lf3 = -+(dl1 + dl2),
-                // B2 = 3 lf2 - 4 lf3 + lf4 = A2 -+ 2 dl2 (upper signs "+", lower "-"); d_k here
-                // is 4 (ss + beta_k)
-                const double B0 = fma(s == 0 ? 2.0 : -2.0, dl1, A0);
-                const double B1 = dl1 + dl2;
-                const double B2 = fma(s == 0 ? -2.0 : 2.0, dl2, A2c);
-                const double d0 = fma(B0, B0, A2[atk(c0, tx, ty)]);
-                const double d1 = fma(B1, B1, A2[atk(cm + (s == 0 ? 0 : 1), tx, ty)]);
-                const double d2 = fma(B2, B2, A2[atk(c2, tx, ty)]);
-                // WENO-Z over the common denominator D = prod d_k^2, P_k = D/d_k^2, T = tau^2:
-                // alpha_k D = c_k (D + T P_k); since sum c_k = 1, N = (sum alpha) D = D + T Q with
-                // Q = sum c_k P_k, and theta > delta <=> D > theta_c N. Both sides are positive,
-                // so the test compares their bit patterns on the integer pipe.
-                const double e0 = d0 * d0, e1 = d1 * d1, e2 = d2 * d2;
-                const double P0 = e1 * e2, P1 = e0 * e2, P2 = e0 * e1;
-                const double D = e0 * P0;
-                const double dd = d2 - d0, T = dd * dd;
-                const double Q = fma(c31, P1, c30 * P0) + c32 * P2;
-                const double N = fma(T, Q, D);
-                smooth[s] = __double_as_longlong(D) > __double_as_longlong(p.theta_c * N);
-                const double r = rcp_nr(N);
-                // u_k = alpha_k / (c_k sum alpha); the weights are w_k = c_k u_k, w1 = 1 - w0 - w2
-                wsur[s][0] = fma(T, P0, D) * r;
-                wsur[s][2] = fma(T, P2, D) * r;
-                if (p.theta) {  // theta = 1/(1 + (sum alpha - 1)^2), sum alpha - 1 = T Q / D
-                    const double sm1 = T * Q / D;
-                    theta_out(s, 1.0 / (1.0 + sm1 * sm1));
-                }
+                double g[4];
+#pragma unroll
+                for (int m = 0; m < 4; ++m) g[m] = sR[s * NCELL + atk(s == 0 ? t + m : t + 4 - m, tx, ty)];
+                // (the weights do not see the differences' common sign)
+                fx::u64 a, b;
+                const bool sm = fx::surrogate(g, p.theta_c, a, b);
+                if (s == 0) { smooth[0] = sm; f0[0] = a; f2[0] = b; }
+                else        { smooth[1] = sm; f0[1] = a; f2[1] = b; }
+                if (p.theta) theta_out(s, theta_of(g));
             }
 #else
             double lp[5], lm[5];
@@ -977,44 +924,31 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
             }
         }
 #if FAST
-        // The smooth results are computed by every lane (uniform, no divergence) and kept only
-        // where the smooth branch is taken; the lanes past a fitted xi tile's last interface read
-        // that interface's stencils. The "-" sign's stencil sum continues the "+" sign's FMA
-        // chain, so a lane smooth in both signs has h = h+ + h- with no separate sum; a lane
-        // smooth in "-" only keeps (h+ + h-) - h+.
-        {
-            const int ox = DIR == 0 && tx >= L::KW ? L::KW - 1 : tx;
-            const int oy = DIR == 1 && ty >= L::KW ? L::KW - 1 : ty;
-            double F[5][4], W[5], hp[4], hs[4];
-            stencil(ox, oy, 0, F);
-            stencil_from_u(wsur[0][0], wsur[0][2], W);
+        // The smooth signs' share of each component: both signs' corrections in one exponent, one
+        // conversion back; a sign that is not smooth contributes nothing. An interface smooth in
+        // both signs is done (most are); the others keep theirs for the characteristic sign's.
+        if (valid) {
+            const bool both = smooth[0] && smooth[1];
+            if (smooth[0] || smooth[1]) {
+#pragma unroll 1
+                for (int c = 0; c < 4; ++c) {
+                    double gp[4], gm[4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-                hp[c] = fma(W[4], F[4][c], fma(W[3], F[3][c], fma(W[2], F[2][c], fma(W[1], F[1][c], W[0] * F[0][c]))));
-            stencil(ox, oy, 1, F);
-            stencil_from_u(wsur[1][0], wsur[1][2], W);
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                hs[c] = fma(W[4], F[4][c], fma(W[3], F[3][c], fma(W[2], F[2][c], fma(W[1], F[1][c], fma(W[0], F[0][c], hp[c])))));
-            if (valid) {
-                if (smooth[0] && smooth[1]) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) hbuf(0, c, tid) = hs[c];
-                } else {
-                    if (smooth[0]) {
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) hbuf(0, c, tid) = hp[c];
-                    } else {
-                        queue[chk(p, atomicAdd(&qn, 1), (int)(2 * NT))] = 2 * tid;
+                    for (int m = 0; m < 4; ++m) {
+                        gp[m] = sDF[c * NCELL + atk(t + m, tx, ty)];
+                        gm[m] = sDF[(4 + c) * NCELL + atk(t + 4 - m, tx, ty)];
                     }
-                    if (smooth[1]) {
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) hbuf(1, c, tid) = hs[c] - hp[c];
-                    } else {
-                        queue[chk(p, atomicAdd(&qn, 1), (int)(2 * NT))] = 2 * tid + 1;
-                    }
+                    const fx::u32 ep = smooth[0] ? fx::exponent_of(gp) : 0u, em = smooth[1] ? fx::exponent_of(gm) : 0u;
+                    const fx::u32 top = fx::umax(ep, em), eh = fx::umax(top, fx::kExpMin);
+                    const fx::i64 kp = fx::correction6_by(gp, eh, f0[0], f2[0]), km = fx::correction6_by(gm, eh, f0[1], f2[1]);
+                    const double h = fx::about(smooth[0] ? SF(c, t + 2, tx, ty) : 0.0, smooth[1] ? SF(4 + c, t + 3, tx, ty) : 0.0,
+                                               fx::to_double((smooth[0] ? kp : 0) - (smooth[1] ? km : 0), eh, top));
+                    if (both) store_one(c, h);
+                    else hbuf(smooth[0] ? 0 : 1, c, tid) = h;
                 }
             }
+            if (!smooth[0]) queue[chk(p, atomicAdd(&qn, 1), (int)(2 * NT))] = 2 * tid;
+            if (!smooth[1]) queue[chk(p, atomicAdd(&qn, 1), (int)(2 * NT))] = 2 * tid + 1;
         }
 #else
 #pragma unroll
@@ -1048,17 +982,21 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
             const int ox = owner % TX, oy = owner / TX;
             EigT e;
             eig_at(ox, oy, e);
-            double F[5][4], h[4];
-            stencil(ox, oy, s, F);
+            double h[4];
 #if FAST
-            double dF[4][4], c6[4] = {0.0, 0.0, 0.0, 0.0};
+            const int t0 = DIR == 0 ? ox : oy;
+            double dF[4][4], centre[4], c6[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-            for (int m = 0; m < 4; ++m)
+            for (int c = 0; c < 4; ++c) {
+                centre[c] = SF(4 * s + c, t0 + 2 + s, ox, oy);
 #pragma unroll
-                for (int c = 0; c < 4; ++c) dF[m][c] = F[m][c] - F[m + 1][c];
-            char_corrections<DIR>(e, dF, false, c6);
-            back_project_fast<DIR>(e, c6, F[2], h);
+                for (int m = 0; m < 4; ++m) dF[m][c] = sDF[(4 * s + c) * NCELL + atk(s == 0 ? t0 + m : t0 + 4 - m, ox, oy)];
+            }
+            char_corrections<DIR>(e, dF, s != 0, c6);
+            back_project_fast<DIR>(e, c6, centre, h);
 #else
+            double F[5][4];
+            stencil(ox, oy, s, F);
             char_weno(e, F, h);
 #endif
 #pragma unroll
@@ -1066,16 +1004,9 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
         }
         __syncthreads();
         // phase 2c: h = h+ + h- (sum_field, field_op.f90:1-21)
-        if (valid) {
-            double hsum[4];
-#if FAST
-            const bool both = smooth[0] && smooth[1];
-#else
-            const bool both = false;
-#endif
+        if (valid && !(FAST && smooth[0] && smooth[1])) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) hsum[c] = both ? hbuf(0, c, tid) : hbuf(0, c, tid) + hbuf(1, c, tid);
-            store(hsum);
+            for (int c = 0; c < 4; ++c) store_one(c, hbuf(0, c, tid) + hbuf(1, c, tid));
         }
     }
 }
@@ -1482,8 +1413,9 @@ __device__ __forceinline__ void bc_block(const Params& p, int bx) {
 // Kernels of one block (instance) of the solver: block coordinates are the launch's own.
 // Resident blocks the register allocation of a characteristic sweep is sized for. AdaWENO's
 // blocks stall on the barriers of their work queue, which a third block per SM hides (80
-// registers, a few bytes spilled; at two blocks the xi sweep of the 1920 x 480 double Mach
-// reflection takes 0.292 instead of 0.282 ms). The 104 sweeps' four inlined integer
+// registers, a few bytes spilled; sweeps of the 1920 x 480 double Mach reflection, xi and eta:
+// 0.159 and 0.180 ms at three blocks, 0.180 and 0.203 at two, 0.162 and 0.188 at four). The 104
+// sweeps' four inlined integer
 // reconstructions would take 160 registers; at 1024 resident threads (64 registers) the sweeps of
 // the 256 x 1024 Rayleigh-Taylor case take 0.127 (xi) and 0.111 ms (eta), at 768 0.131 and 0.113,
 // unbounded 0.141 and 0.158 -- and 0.340 and 0.293 with the reconstructions in FP64.

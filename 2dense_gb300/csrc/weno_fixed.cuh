@@ -209,16 +209,26 @@ DENSE_FX u64 indicator(i64 A, i64 B, int e2, int& x) {
     return d << z;
 }
 
+// The three of a stencil.
+DENSE_FX void indicators(i64 A0, i64 A1, i64 A2, i64 G1, i64 G2, u32 eh, u64 M[3], int x[3]) {
+    const int e2 = 2 * (int)(eh >> 20) - 2014;
+    M[0] = indicator(A0, A0 - 2 * G1, e2, x[0]);
+    M[1] = indicator(A1, G1 + G2, e2, x[1]);
+    M[2] = indicator(A2, A2 + 2 * G2, e2, x[2]);
+}
+
 // The weights' shares 2 w_0 and w_2 and their sum n = sum of all c_k v_k, from the indicators:
 // u0/n = 2 w_0, u2/n = w_2, n in [2^62, 2^63). JS: v_k = P_k, the product of the other two
-// squares; Z: v_k = D + tau^2 P_k (weno_terms). The linear weights are 1, 6 and 3 tenths.
+// squares; Z: v_k = D + tau^2 P_k (weno_terms), and lin = 10 D on the scale of n. The linear
+// weights are 1, 6 and 3 tenths.
 template <bool Z>
-DENSE_FX void weights(const u64 M[3], const int x[3], u64& u0, u64& u2, u64& n) {
+DENSE_FX void weights(const u64 M[3], const int x[3], u64& u0, u64& u2, u64& n, u64& lin) {
     int a0 = 2 * x[0], a1 = 2 * x[1], a2 = 2 * x[2];
     const u64 q0 = norm1(sqhi(M[0]), a0), q1 = norm1(sqhi(M[1]), a1), q2 = norm1(sqhi(M[2]), a2);
     const u64 P0 = mulhi(q1, q2), P1 = mulhi(q0, q2), P2 = mulhi(q0, q1);  // at least 2^62 - 2
     const int am = imin(imin(a0, a1), a2);
     u64 v0, v1, v2;
+    lin = 0;
     // v_k below 2^59 (10 x 2^59 < 2^63), the largest at least 2^56 (JS) or 2^55 (Z)
     if (!Z) {
         v0 = shr(P0, a0 - am + 5);
@@ -233,6 +243,7 @@ DENSE_FX void weights(const u64 M[3], const int x[3], u64& u0, u64& u2, u64& n) 
         const u64 D = mulhi(q0, P0);
         const int X = imax(0, at - am) + 6;
         const u64 ds = shr(D, X);
+        lin = 10 * ds;
         v0 = ds + shr(mulhi(T, P0), X - (at - a0));
         v1 = ds + shr(mulhi(T, P1), X - (at - a1));
         v2 = ds + shr(mulhi(T, P2), X - (at - a2));
@@ -243,6 +254,7 @@ DENSE_FX void weights(const u64 M[3], const int x[3], u64& u0, u64& u2, u64& n) 
     u0 = v0 << (c + 1);
     u2 = v2 << c;
     n <<= c;
+    lin <<= c;
 }
 
 // u C / 2^64, truncated towards zero
@@ -261,30 +273,31 @@ DENSE_FX i64 weighted(u64 u0, u64 u2, u64 n, i64 C0, i64 C2) {
 // 6 (h - lf_2) of one stencil in units of 2^(E - 1081), from its first differences
 template <bool Z>
 DENSE_FX i64 correction6(const double g[4], u32 eh) {
-    const int e2 = 2 * (int)(eh >> 20) - 2014;
     const i64 G1 = to_fixed(g[1], eh), G2 = to_fixed(g[2], eh);
     const i64 A0 = to_fixed(g[0], eh) - G1, A1 = G1 - G2, A2 = G2 - to_fixed(g[3], eh);
-    u64 M[3], u0, u2, n;
+    u64 M[3], u0, u2, n, lin;
     int x[3];
-    M[0] = indicator(A0, A0 - 2 * G1, e2, x[0]);
-    M[1] = indicator(A1, G1 + G2, e2, x[1]);
-    M[2] = indicator(A2, A2 + 2 * G2, e2, x[2]);
-    weights<Z>(M, x, u0, u2, n);
+    indicators(A0, A1, A2, G1, G2, eh, M, x);
+    weights<Z>(M, x, u0, u2, n, lin);
     return weighted(u0, u2, n, A0 - A1, A1 - A2) - G1 - 2 * G2;
 }
 
-// The sum of two reconstructions about lp and lm. The corrections share their exponent and the
-// conversion back; their sum goes to the smaller centre first, so that the two FP64 roundings
-// are no larger than those of two values and their sum, and the same in either order.
+// lp + lm + c/6, c on the smaller one first: the two FP64 roundings are no larger than those of two
+// values and their sum, and the same in either order.
+DENSE_FX double about(double lp, double lm, double c) {
+    constexpr u64 kAbs = 0x7fffffffffffffffull;
+    const u64 ap = bits(lp) & kAbs, am = bits(lm) & kAbs;
+    const bool first = ap < am || (ap == am && bits(lp) == ap);  // of two opposite ones, the positive
+    return fma(c, 1.0 / 6.0, first ? lp : lm) + (first ? lm : lp);
+}
+// The sum of two reconstructions about lp and lm, whose corrections share their exponent and the
+// conversion back.
 template <bool Z>
 DENSE_FX double pair(double lp, const double gp[4], double lm, const double gm[4]) {
     u32 top = 0;
     const u32 ep = scale_of(gp, top), eh = umax(ep, scale_of(gm, top));
     const double c = to_double(correction6<Z>(gp, eh) + correction6<Z>(gm, eh), eh, top);
-    constexpr u64 kAbs = 0x7fffffffffffffffull;
-    const u64 ap = bits(lp) & kAbs, am = bits(lm) & kAbs;
-    const bool first = ap < am || (ap == am && bits(lp) == ap);  // of two opposite ones, the positive
-    return fma(c, 1.0 / 6.0, first ? lp : lm) + (first ? lm : lp);
+    return about(lp, lm, c);
 }
 // 6 (h - lf_2) of one reconstruction.
 template <bool Z>
@@ -292,6 +305,39 @@ DENSE_FX double correction(const double g[4]) {
     u32 top = 0;
     const u32 eh = scale_of(g, top);
     return to_double(correction6<Z>(g, eh), eh, top);
+}
+
+// AdaWENO: the WENO-Z weights of a scalar surrogate, from its first differences, as fractions
+// 2 w_0 = f0/2^62 and w_2 = f2/2^62, and its switch theta > delta, which is 10 D > theta_c n
+// (Params::theta_c; 0 always, 1 never). A NaN or infinity is not smooth.
+DENSE_FX bool surrogate(const double g[4], double theta_c, u64& f0, u64& f2) {
+    u32 top = 0;
+    const u32 eh = scale_of(g, top);
+    const i64 G1 = to_fixed(g[1], eh), G2 = to_fixed(g[2], eh);
+    const i64 A0 = to_fixed(g[0], eh) - G1, A1 = G1 - G2, A2 = G2 - to_fixed(g[3], eh);
+    u64 M[3], u0, u2, n, lin;
+    int x[3];
+    indicators(A0, A1, A2, G1, G2, eh, M, x);
+    weights<true>(M, x, u0, u2, n, lin);
+    const u64 r = reciprocal(n);
+    f0 = mulhi63(u0 >> 1, r) << 2;
+    f2 = mulhi63(u2, r) << 1;
+    const u64 tb = bits(theta_c);
+    const u32 te = (u32)(tb >> 52);  // theta_c in [0, 1]: its exponent field is at most 1023
+    const u64 tc = shr((tb << 11) | 0x8000000000000000ull, 1022u - te);
+    const bool smooth = te == 0 || (te < 1023u && lin > mulhi(n, tc));
+    return smooth && top < kExpMax;
+}
+// 6 (h - lf_2) of another stencil by a surrogate's weights, in units of 2^(E - 1081), E at least
+// the exponent of its differences (the weights are not its own: nothing is clipped).
+DENSE_FX i64 correction6_by(const double g[4], u32 eh, u64 f0, u64 f2) {
+    const i64 G1 = to_fixed(g[1], eh), G2 = to_fixed(g[2], eh);
+    const i64 A0 = to_fixed(g[0], eh) - G1, A1 = G1 - G2, A2 = G2 - to_fixed(g[3], eh);
+    return scaled(f0, (A0 - A1) * 4) + scaled(f2, (A1 - A2) * 4) - G1 - 2 * G2;
+}
+// The largest exponent of a stencil's differences.
+DENSE_FX u32 exponent_of(const double g[4]) {
+    return umax(umax(exponent(g[0]), exponent(g[1])), umax(exponent(g[2]), exponent(g[3])));
 }
 
 }  // namespace fx

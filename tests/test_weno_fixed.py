@@ -41,3 +41,13 @@ def test_forms(lines, z):
     _, _, odd, swap, flat, bad, n, scale_err = [x for x in lines if x[0] == "forms" and x[1] == str(z)][0]
     assert (int(odd), int(swap), int(flat), int(bad)) == (0, 0, 0, 0)
     assert int(n) > 1000 and float(scale_err) <= 1.0
+
+
+def test_adaptive(lines):
+    """AdaWENO's switch equals theta > delta away from the threshold (within the rounding of the
+    surrogate's values), delta's two ends and a NaN decide it, and a stencil reconstructed with the
+    surrogate's weights is exact to a few roundings."""
+    n, wrong, near, ends, nans, smooth, worst = [float(v) for v in [x for x in lines if x[0] == "adaptive"][0][1:]]
+    assert (wrong, ends, nans) == (0, 0, 0)
+    assert near < 0.1 * n and 0.05 * n < smooth < 0.95 * n
+    assert worst <= 16 * 2.0 ** -53

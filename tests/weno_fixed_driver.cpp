@@ -128,6 +128,54 @@ template <bool Z> void forms() {
     printf("forms %d %d %d %d %d %d %.17g\n", (int)Z, odd, swap, flat, bad, n, scale_err);
 }
 
+// AdaWENO's surrogate: its switch against theta > delta, and another stencil reconstructed with its
+// weights against long double
+void adaptive() {
+    std::mt19937_64 r(9);
+    std::uniform_real_distribution<double> u(0, 1);
+    int wrong = 0, near = 0, ends = 0, smooth = 0, nans = 0;
+    double worst = 0;
+    const int n = 50000;
+    for (int t = 0; t < n; ++t) {
+        const Stencils s = draw(r, t % 4);
+        const double delta = t % 3 ? u(r) : 0.5, k = std::sqrt(delta / (1.0 - delta)), theta_c = k / (1.0 + k);
+        const ld a = s.fp[0], b = s.fp[1], c = s.fp[2], d = s.fp[3], e = s.fp[4], ss = (double)1.0e-6f;
+        const ld is[3] = {13 * (a - 2 * b + c) * (a - 2 * b + c) / 12 + (a - 4 * b + 3 * c) * (a - 4 * b + 3 * c) / 4,
+                          13 * (b - 2 * c + d) * (b - 2 * c + d) / 12 + (b - d) * (b - d) / 4,
+                          13 * (c - 2 * d + e) * (c - 2 * d + e) / 12 + (3 * c - 4 * d + e) * (3 * c - 4 * d + e) / 4};
+        ld al[3], sum = 0;
+        const ld tau = is[2] - is[0], cs[3] = {0.1L, 0.6L, 0.3L};
+        for (int i = 0; i < 3; ++i) { al[i] = cs[i] * (1 + tau * tau / ((ss + is[i]) * (ss + is[i]))); sum += al[i]; }
+        const ld theta = 1 / (1 + (sum - 1) * (sum - 1));
+        dense::fx::u64 f0, f2;
+        const bool got = dense::fx::surrogate(s.gp, theta_c, f0, f2);
+        smooth += got;
+        // the surrogate's differences carry the rounding of its values: 2^-53 of them, amplified by the
+        // indicators' sensitivity to the smallest difference (or sqrt(ss))
+        ld small = std::sqrt((double)ss);
+        ld sens = 64 * s.size() * 0x1p-53L;
+        for (int m = 0; m < 4; ++m) if (s.gp[m] != 0) small = std::min(small, (ld)std::fabs(s.gp[m]));
+        if (fabsl(theta - delta) <= 1e-9L + sens / small) ++near;
+        else wrong += got != (theta > delta);
+        ends += !dense::fx::surrogate(s.gp, 0.0, f0, f2) || dense::fx::surrogate(s.gp, 1.0, f0, f2);
+        double bad[4] = {s.gp[0], s.gp[1], s.gp[2], s.gp[3]};
+        bad[t & 3] = t & 4 ? std::numeric_limits<double>::quiet_NaN() : std::numeric_limits<double>::infinity();
+        dense::fx::u64 x, y;
+        nans += dense::fx::surrogate(bad, 0.0, x, y);
+        // the other stencil (s.fm) with these weights: the weights are taken as they are (an error of
+        // theirs counts with the third differences), the arithmetic is compared
+        const ld w0 = ldexpl((ld)f0, -63), w2 = ldexpl((ld)f2, -62), w1 = 1 - w0 - w2;
+        const ld q0 = (2 * (ld)s.fm[0] - 7 * (ld)s.fm[1] + 11 * (ld)s.fm[2]) / 6, q1 = (-(ld)s.fm[1] + 5 * (ld)s.fm[2] + 2 * (ld)s.fm[3]) / 6,
+                 q2 = (2 * (ld)s.fm[2] + 5 * (ld)s.fm[3] - (ld)s.fm[4]) / 6;
+        const dense::fx::u32 eh = dense::fx::umax(dense::fx::exponent_of(s.gm), dense::fx::kExpMin);
+        const double h = dense::fx::about(s.fm[2], 0.0, dense::fx::to_double(dense::fx::correction6_by(s.gm, eh, f0, f2), eh, eh));
+        worst = std::max(worst, (double)(fabsl(h - (w0 * q0 + w1 * q1 + w2 * q2)) / s.size()));
+        // and the weights
+        worst = std::max(worst, (double)(fabsl(w0 - al[0] / sum) > 1e-9L + sens / small));
+    }
+    printf("adaptive %d %d %d %d %d %d %.17g\n", n, wrong, near, ends, nans, smooth, worst);
+}
+
 int main() {
     std::mt19937_64 r(3);
     double worst = 0;
@@ -142,4 +190,5 @@ int main() {
     for (int k = 0; k < 5; ++k) { accuracy<false>(k); accuracy<true>(k); }
     forms<false>();
     forms<true>();
+    adaptive();
 }
