@@ -388,8 +388,7 @@ __device__ __forceinline__ void char_corrections(const EigFast& e, const double 
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         // a correction is odd in its differences, to the bit
-        const double x = fx::correction<true>(g[k]);
-        c[k] += neg ? -x : x;
+        c[k] += fx::from_bits(fx::bits(fx::correction<true>(g[k])) ^ (neg ? 0x8000000000000000ull : 0ull));
     }
 }
 template <int DIR>
@@ -546,7 +545,7 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
         double h;
         if constexpr (kStageG) {
             // "+": lf(m) = F+(tile cell t+m), g_m = G+(t+m); "-": lf(m) = F-(tile cell t+5-m), g_m =
-            // F-(t+5-m) - F-(t+4-m) = -G-(t+4-m)
+            // F-(t+5-m) - F-(t+4-m) = -G-(t+4-m), its sign left to fx::pair
             constexpr bool Z = REC == DENSE_RECON_WENOZ5;
             const double* Gp = sG + v * NCELL;
             const double* Gm = sG + (4 + v) * NCELL;
@@ -554,7 +553,7 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
                 gp[m] = Gp[atk(t + m)];
-                gm[m] = -Gm[atk(t + 4 - m)];
+                gm[m] = Gm[atk(t + 4 - m)];
             }
             h = fx::pair<Z>(sF[v * NCELL + atk(t + 2)], gp, sF[(4 + v) * NCELL + atk(t + 3)], gm);
             if constexpr (TAPE) {
@@ -570,6 +569,8 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
                     for (int m = 0; m < 5; ++m) tape_at[((m0 + m) * 4 + v) * ts] = g[m];
                 };
                 tape_grad(gp, 0);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) gm[m] = -gm[m];
                 tape_grad(gm, 5);
             }
         } else {
@@ -625,7 +626,7 @@ __global__ void k_flux_noop(Params p, int irk) {
 // whole block then works through the queue on full warps.
 // What bounds it: the FP64 pipe. The surrogate's weights and the smooth branch run on the integer
 // pipes (weno_fixed.cuh), which leaves some 55 FP64 instructions an interface of 150 and took the
-// 1920 x 480 double Mach reflection's sweeps from 0.282 and 0.305 ms to 0.159 and 0.180.
+// 1920 x 480 double Mach reflection's sweeps from 0.282 and 0.305 ms to 0.149 and 0.174.
 // Dynamic shared memory of one characteristic sweep block, in doubles: the tile's split fluxes
 // sF[8][NL][NC] and primitives sQ[4][NL][NC]; per-cell sqrt(rho) sS (104, fast); the split fluxes'
 // forward differences along the sweep sDF[8][NL][NC] (fast); and one region R that AdaWENO uses
@@ -1414,11 +1415,13 @@ __device__ __forceinline__ void bc_block(const Params& p, int bx) {
 // Resident blocks the register allocation of a characteristic sweep is sized for. AdaWENO's
 // blocks stall on the barriers of their work queue, which a third block per SM hides (80
 // registers, a few bytes spilled; sweeps of the 1920 x 480 double Mach reflection, xi and eta:
-// 0.159 and 0.180 ms at three blocks, 0.180 and 0.203 at two, 0.162 and 0.188 at four). The 104
+// 0.149 and 0.174 ms at three blocks; before its weights' last trimming 0.159 and 0.180 at three,
+// 0.180 and 0.203 at two, 0.162 and 0.188 at four). The 104
 // sweeps' four inlined integer
 // reconstructions would take 160 registers; at 1024 resident threads (64 registers) the sweeps of
-// the 256 x 1024 Rayleigh-Taylor case take 0.127 (xi) and 0.111 ms (eta), at 768 0.131 and 0.113,
-// unbounded 0.141 and 0.158 -- and 0.340 and 0.293 with the reconstructions in FP64.
+// the 256 x 1024 Rayleigh-Taylor case took 0.127 (xi) and 0.111 ms (eta), at 768 0.131 and 0.113,
+// unbounded 0.141 and 0.158 (0.123 and 0.104 after that trimming, and 0.340 and 0.293 with the
+// reconstructions in FP64).
 constexpr int char_min_blocks(bool adapt, int nt) { return adapt ? 3 : 1024 / nt; }
 template <int DIR, int SPL, int REC, int TX, int TY, bool TAPE = false, int TZ = 1>
 __global__ void __launch_bounds__(TX* TY* TZ) k_flux_cw(Params p, int irk) {

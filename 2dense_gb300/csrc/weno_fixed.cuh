@@ -1,26 +1,26 @@
 // weno_fixed.cuh -- WENO-JS5 / WENO-Z5 reconstructions on the integer pipes, for the fast sweeps.
 //
-// GB300 issues an FP64 instruction of a warp every 16 to 20 cycles of an SM, and in that time up
-// to 64 others: measured per warp and SM, DFMA 16.9 cycles, DADD and DMUL 20.0, against 0.6 for a
-// 32-bit IMAD or LOP, 1.0 for a 32x32+64-bit IMAD.WIDE, 0.6 for a 64-bit shift and 4.5 for the
-// upper half of a 64x64-bit product. A reconstruction in FP64 is about 34 instructions, 556 (JS)
-// to 668 (Z) cycles with the integer pipes idle; the same value in 64-bit integers takes 206 and
-// 238, and leaves the FP64 pipe to the split fluxes of other warps. The component-wise xi sweep of
-// a 2048 x 2048 LLF stage went from 2.414 to 0.776 ms (JS) and from 2.773 to 0.877 ms (Z), the
-// eta sweep from 2.301 to 0.776 and from 2.657 to 0.856 ms. Nothing is computed in fewer bits than
-// before: the words carry 57 to 64 significant bits where a double carries 53.
-//
+// GB300 issues an FP64 instruction of a warp every 16 cycles of an SM, and in that time up to 64
+// others: measured per warp and SM, DFMA 16.9 cycles, against 0.6 for a 32-bit IMAD or LOP, 1.0 for a
+// 32x32+64-bit IMAD.WIDE, 0.6 for a 64-bit shift and 4.5 for the upper half of a 64x64-bit
+// product. A reconstruction in FP64 is about 34 instructions, 556 (JS) to 668 (Z) cycles with the
+// integer pipes idle; the same value in 64-bit integers takes 172 and 205, and leaves the FP64 pipe
+// to the split fluxes of other warps. The component-wise xi sweep of a 2048 x 2048 LLF stage went
+// from 2.414 to 0.684 ms (JS) and from 2.773 to 0.778 ms (Z), the eta sweep from 2.301 to 0.663 and
+// from 2.657 to 0.772 ms; what bounds them now is the integer ALU (72 % busy, 340 instructions a
+// reconstruction before its last trimming). Nothing is computed in fewer bits than before: the
+// words carry 57 to 64 significant bits where a double carries 53.
 // The value. With g_m = lf_m - lf_(m+1), A_k = g_k - g_(k+1), B_0 = A_0 - 2 g_1, B_1 = g_1 + g_2,
 // B_2 = A_2 + 2 g_2 and d_k = 4 (ss + beta_k) = 4 ss + 13/3 A_k^2 + B_k^2 (weno_fast.cuh), the
 // candidates differ by third differences, so that with weights of sum one
 //   6 (h - lf_2) = -(g_1 + 2 g_2) + 2 w_0 (A_0 - A_1) + w_2 (A_1 - A_2).
 // The representation:
 //  * the first differences become fixed-point integers of one exponent for the stencils of a face
-//    value, below 2^59: their sums and differences are exact. The exponent is the largest
+//    value, below 2^58: their sums and differences are exact. The exponent is the largest
 //    difference's, but at most kCap above that of the smoothest substencil (of sqrt(ss), where that
 //    is more): past a jump of 2^kCap times the rest, the weights leave 2^-3kCap of the rest to the
 //    substencils that contain it, whatever it is, so it may as well be clipped, and the rest keeps
-//    58 - kCap bits or more beside any jump;
+//    57 - kCap bits or more beside any jump;
 //  * the indicators 3 d_k = 12 ss + 13 A_k^2 + 3 B_k^2 and everything made of them are positive
 //    floating-point numbers of a 64-bit mantissa and an integer exponent, whose products need
 //    no normalising between them; the weights' common denominators are those of weno_terms;
@@ -133,12 +133,6 @@ DENSE_FX u64 mulhi63(u64 a, u64 b) {
     return wide(hi32(a), hi32(b)) + hi32(m);
 }
 DENSE_FX u64 sqhi(u64 a) { return wide(hi32(a), hi32(a)) + (wide(hi32(a), (u32)a) >> 31); }
-// the top bit set, for a at least 2^62; x counts the shift
-DENSE_FX u64 norm1(u64 a, int& x) {
-    const u32 c = (hi32(a) >> 31) ^ 1u;
-    x -= (int)c;
-    return a << c;
-}
 
 // 2^125 / n for n in [2^62, 2^63), relative error below 2^-59: x0 = 2^61 / (n / 2^32) to 22 bits
 // from the hardware's reciprocal, e = 1 - x0 n, and 1/n = x0 (1 + e + e^2 + ...), as rcp_nr has it
@@ -169,7 +163,7 @@ DENSE_FX u32 scale_of(const double g[4], u32& top) {
     return umax(umin(most, umax(least, kExpSS) + (kCap << 20)), kExpMin);
 }
 
-// A double as a fixed-point integer in units of 2^(E - 1081) (E in place in eh): below 2^59,
+// A double as a fixed-point integer in units of 2^(E - 1080) (E in place in eh): below 2^58,
 // truncated; a larger one clipped to E.
 DENSE_FX i64 to_fixed(double g, u32 eh) {
     const u64 b = bits(g);
@@ -177,44 +171,44 @@ DENSE_FX i64 to_fixed(double g, u32 eh) {
     const int sh = (int)(eh - (h & kExpMask)) >> 20;
     // 1.m in [2^62, 2^63); where the exponent is zero the shift leaves nothing of it
     const u64 m = ((u64)((((h << 10) | ((u32)b >> 22)) & 0x3fffffffu) | 0x40000000u) << 32) | (u32)((u32)b << 10);
-    const u64 a = shr(m, (u32)imax(sh, 0) + 4);
+    const u64 a = shr(m, (u32)imax(sh, 0) + 5);
     const u64 s = (u64)(i64)((int)h >> 31);
     return (i64)((a ^ s) - s);
 }
-// c 2^(E - 1081) rounded to nearest, |c| below 2^63; NaN for top from kExpMax on
+// c 2^(E - 1080) rounded to nearest, |c| below 2^63; NaN for top from kExpMax on
 DENSE_FX double to_double(i64 c, u32 eh, u32 top) {
     const u64 a = abs64(c);
     const int n = clz64(a) & 63;
-    u64 r = ((u64)c & 0x8000000000000000ull) | (((u64)((eh >> 20) + 4 - n) << 52) + (((a << n) + 0x400) >> 11));
+    u64 r = ((u64)c & 0x8000000000000000ull) | (((u64)((eh >> 20) + 5 - n) << 52) + (((a << n) + 0x400) >> 11));
     if (a == 0) r = 0;
     if (top >= kExpMax) r = 0x7ff8000000000000ull;
     return from_bits(r);
 }
 
+// a^2 / 2^64 for a below 2^61, at most 2 below its floor
+DENSE_FX u64 sq61(u64 a) { return wide(hi32(a), hi32(a)) + hi32(wide(2 * hi32(a), (u32)a)); }
 // 3 d_k = 12 ss + 13 A^2 + 3 B^2 as M 2^x (up to a power of two common to all), M with its top
-// bit set; A below 2^61, B below 2^62 in units of 2^(E - 1081), e2 = 2 E - 2014.
-DENSE_FX u64 indicator(i64 A, i64 B, int e2, int& x) {
+// bit set; |A| and |B| at most 2^60. A and B are scaled up by 2^n first, so that a small
+// indicator keeps its bits, but not past the unit of 12 ss, where nothing is left to keep: the
+// squares' unit is then 2^up of it (or, where all differences are that small, 2^-down).
+DENSE_FX u64 indicator(i64 A, i64 B, u32 nmax, u32 down, int& x) {
     constexpr u64 kS = (u64)(12.0 * (double)1.0e-6f * 302231454903657293676544.0);  // 12 ss 2^78
     u64 a = abs64(A), b = abs64(B);
-    const u64 o = a | b;
-    const int n = clz64(o) & 63;
+    const u32 n = umin((u32)clz64(a | b) - 3u, nmax), up = 2 * (nmax - n);
     a <<= n;
     b <<= n;
-    const u64 q = 13 * (sqhi(a) >> 6) + 3 * (sqhi(b) >> 6);  // below 2^62, units of 2^(e2 - 2n - 78)
-    const int t = o ? e2 - 2 * n : 0;                        // A = B = 0: 12 ss alone
-    const int up = imax(t, 0), down = imax(-t, 0);
-    const u64 d = shr(q, down) + shr(kS, up);                // units of 2^(up - 78); at least 2^57
+    const u64 d = shr(13 * sq61(a) + 3 * sq61(b), down) + shr(kS, up);  // below 2^63, at least 2^57
     const int z = clz32(hi32(d));
-    x = up - z;
+    x = (int)up - z;
     return d << z;
 }
-
-// The three of a stencil.
+// The three of a stencil. A square's unit is 2^(2 (E - 1080 - n) + 64), that of 12 ss 2^-78.
 DENSE_FX void indicators(i64 A0, i64 A1, i64 A2, i64 G1, i64 G2, u32 eh, u64 M[3], int x[3]) {
-    const int e2 = 2 * (int)(eh >> 20) - 2014;
-    M[0] = indicator(A0, A0 - 2 * G1, e2, x[0]);
-    M[1] = indicator(A1, G1 + G2, e2, x[1]);
-    M[2] = indicator(A2, A2 + 2 * G2, e2, x[2]);
+    const int e = (int)(eh >> 20) - 1009;
+    const u32 nmax = (u32)imax(e, 0), down = (u32)imax(-2 * e, 0);
+    M[0] = indicator(A0, A0 - 2 * G1, nmax, down, x[0]);
+    M[1] = indicator(A1, G1 + G2, nmax, down, x[1]);
+    M[2] = indicator(A2, A2 + 2 * G2, nmax, down, x[2]);
 }
 
 // The weights' shares 2 w_0 and w_2 and their sum n = sum of all c_k v_k, from the indicators:
@@ -223,13 +217,12 @@ DENSE_FX void indicators(i64 A0, i64 A1, i64 A2, i64 G1, i64 G2, u32 eh, u64 M[3
 // weights are 1, 6 and 3 tenths.
 template <bool Z>
 DENSE_FX void weights(const u64 M[3], const int x[3], u64& u0, u64& u2, u64& n, u64& lin) {
-    int a0 = 2 * x[0], a1 = 2 * x[1], a2 = 2 * x[2];
-    const u64 q0 = norm1(sqhi(M[0]), a0), q1 = norm1(sqhi(M[1]), a1), q2 = norm1(sqhi(M[2]), a2);
-    const u64 P0 = mulhi(q1, q2), P1 = mulhi(q0, q2), P2 = mulhi(q0, q1);  // at least 2^62 - 2
-    const int am = imin(imin(a0, a1), a2);
+    const int a0 = 2 * x[0], a1 = 2 * x[1], a2 = 2 * x[2], am = imin(imin(a0, a1), a2);
+    const u64 q0 = sqhi(M[0]), q1 = sqhi(M[1]), q2 = sqhi(M[2]);           // at least 2^62
+    const u64 P0 = mulhi(q1, q2), P1 = mulhi(q0, q2), P2 = mulhi(q0, q1);  // at least 2^60 - 2
     u64 v0, v1, v2;
     lin = 0;
-    // v_k below 2^59 (10 x 2^59 < 2^63), the largest at least 2^56 (JS) or 2^55 (Z)
+    // v_k below 2^59 (10 x 2^59 < 2^63), the largest at least 2^54 (JS) or 2^57 (Z)
     if (!Z) {
         v0 = shr(P0, a0 - am + 5);
         v1 = shr(P1, a1 - am + 5);
@@ -238,15 +231,16 @@ DENSE_FX void weights(const u64 M[3], const int x[3], u64& u0, u64& u2, u64& n, 
         const int xm = imax(x[0], x[2]);
         const u64 dd = abs64((i64)(shr(M[2], xm - x[2] + 1) - shr(M[0], xm - x[0] + 1)));
         const int c = clz64(dd) & 63;
-        int at = dd ? 2 * (xm + 1 - c) : -100000;  // tau = 0 leaves every v_k = D
-        const u64 T = norm1(sqhi(dd << c), at);
-        const u64 D = mulhi(q0, P0);
-        const int X = imax(0, at - am) + 6;
+        const int at = dd ? 2 * (xm + 1 - c) : -100000;  // tau = 0 leaves every v_k = D
+        const u64 T = sqhi(dd << c);
+        const u64 D = mulhi(q0, P0), t0 = mulhi(T, P0), t1 = mulhi(T, P1), t2 = mulhi(T, P2);
+        // all below 2^(64 - z), z at most 6: the alignment shifts by that much less
+        const int X = imax(0, at - am) + 6 - clz32(hi32(D | t0 | t1 | t2));
         const u64 ds = shr(D, X);
         lin = 10 * ds;
-        v0 = ds + shr(mulhi(T, P0), X - (at - a0));
-        v1 = ds + shr(mulhi(T, P1), X - (at - a1));
-        v2 = ds + shr(mulhi(T, P2), X - (at - a2));
+        v0 = ds + shr(t0, X - (at - a0));
+        v1 = ds + shr(t1, X - (at - a1));
+        v2 = ds + shr(t2, X - (at - a2));
     }
     v2 *= 3;
     n = v0 + 6 * v1 + v2;
@@ -270,7 +264,7 @@ DENSE_FX i64 weighted(u64 u0, u64 u2, u64 n, i64 C0, i64 C2) {
     return (i64)((q ^ s) - s);
 }
 
-// 6 (h - lf_2) of one stencil in units of 2^(E - 1081), from its first differences
+// 6 (h - lf_2) of one stencil in units of 2^(E - 1080), from its first differences
 template <bool Z>
 DENSE_FX i64 correction6(const double g[4], u32 eh) {
     const i64 G1 = to_fixed(g[1], eh), G2 = to_fixed(g[2], eh);
@@ -285,18 +279,18 @@ DENSE_FX i64 correction6(const double g[4], u32 eh) {
 // lp + lm + c/6, c on the smaller one first: the two FP64 roundings are no larger than those of two
 // values and their sum, and the same in either order.
 DENSE_FX double about(double lp, double lm, double c) {
-    constexpr u64 kAbs = 0x7fffffffffffffffull;
-    const u64 ap = bits(lp) & kAbs, am = bits(lm) & kAbs;
-    const bool first = ap < am || (ap == am && bits(lp) == ap);  // of two opposite ones, the positive
+    const u64 ap = bits(lp) << 1, am = bits(lm) << 1;          // (an FP64 absolute value would take that pipe)
+    const bool first = ap < am || (ap == am && (i64)bits(lp) >= 0);  // of two opposite ones, the positive
     return fma(c, 1.0 / 6.0, first ? lp : lm) + (first ? lm : lp);
 }
 // The sum of two reconstructions about lp and lm, whose corrections share their exponent and the
-// conversion back.
+// conversion back. gm: the second's differences with the opposite sign, as a sweep has them (a
+// correction is odd in its differences, to the bit; negating doubles would take the FP64 pipe).
 template <bool Z>
 DENSE_FX double pair(double lp, const double gp[4], double lm, const double gm[4]) {
     u32 top = 0;
     const u32 ep = scale_of(gp, top), eh = umax(ep, scale_of(gm, top));
-    const double c = to_double(correction6<Z>(gp, eh) + correction6<Z>(gm, eh), eh, top);
+    const double c = to_double(correction6<Z>(gp, eh) - correction6<Z>(gm, eh), eh, top);
     return about(lp, lm, c);
 }
 // 6 (h - lf_2) of one reconstruction.
@@ -328,7 +322,7 @@ DENSE_FX bool surrogate(const double g[4], double theta_c, u64& f0, u64& f2) {
     const bool smooth = te == 0 || (te < 1023u && lin > mulhi(n, tc));
     return smooth && top < kExpMax;
 }
-// 6 (h - lf_2) of another stencil by a surrogate's weights, in units of 2^(E - 1081), E at least
+// 6 (h - lf_2) of another stencil by a surrogate's weights, in units of 2^(E - 1080), E at least
 // the exponent of its differences (the weights are not its own: nothing is clipped).
 DENSE_FX i64 correction6_by(const double g[4], u32 eh, u64 f0, u64 f2) {
     const i64 G1 = to_fixed(g[1], eh), G2 = to_fixed(g[2], eh);
