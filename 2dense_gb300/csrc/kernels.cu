@@ -130,9 +130,15 @@ __device__ __forceinline__ void weno5z_omega_theta(const double lf[5], double& w
     theta = 1.0 / (1.0 + sq(s - 1.0));
 }
 
-// upwind5 (scheme_upwind5_general.f90:86-90)
+// upwind5 (scheme_upwind5_general.f90:86-90). Fast: the 60 folded into the coefficients, the
+// smallest ones first; five operations where the divide alone costs ten (sweeps of a 1024 x 1024
+// GLF stage: xi 0.276 -> 0.155 ms, eta 0.250 -> 0.131 ms).
 __device__ __forceinline__ double upwind5(const double lf[5]) {
+#if FAST
+    return fma(47.0 / 60.0, lf[2], fma(27.0 / 60.0, lf[3], fma(-13.0 / 60.0, lf[1], fma(-3.0 / 60.0, lf[4], 2.0 / 60.0 * lf[0]))));
+#else
     return (2.0 * lf[0] - 13.0 * lf[1] + 47.0 * lf[2] + 27.0 * lf[3] - 3.0 * lf[4]) / 60.0;
+#endif
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -234,6 +240,34 @@ template <int DIR>
 __device__ __forceinline__ void sw_split(double rho, double u, double v, double alpha, double gamma,
                                          double fp[4], double fm[4]) {
     const double epsl2 = 0.125 * 0.125;
+#if FAST
+    // With p_k = l_k +- sqrt(l_k^2 + eps^2) (twice the split eigenvalues), l_2,3 = u_n -+ a, c =
+    // rho / (4 gamma), S = p_2 + p_3 and D = c a (p_3 - p_2), the components factor into
+    //   f_0 = c (2 (gamma-1) p_1 + S),  f_n = u_n f_0 + D,  f_t = u_t f_0,
+    //   f_3 = (u^2 + v^2)/2 f_0 + u_n D + c a^2/(gamma-1) S:
+    // 53 operations for both signs, the square roots from rsqrt_nr, where the form below spends
+    // three IEEE square roots and eight divides (481 x 479 WENO-Z sweeps: xi 0.190 -> 0.080 ms, eta
+    // 0.148 -> 0.076 ms). Every sum of a product is an explicit FMA, so that the plain and taping
+    // sweeps round alike.
+    const double un = DIR == 0 ? u : v, ut = DIR == 0 ? v : u;
+    const double l2 = un - alpha, l3 = un + alpha;
+    const double x1 = fma(un, un, epsl2), x2 = fma(l2, l2, epsl2), x3 = fma(l3, l3, epsl2);
+    const double r1 = rsqrt_nr(x1), r2 = rsqrt_nr(x2), r3 = rsqrt_nr(x3);
+    const double c = rho * (0.25 / gamma), ca = c * alpha, k = ca * (alpha * (1.0 / (gamma - 1.0)));
+    const double half_q2 = 0.5 * fma(un, un, ut * ut), two_g1 = 2.0 * (gamma - 1.0);
+#pragma unroll
+    for (int sgn = 0; sgn < 2; ++sgn) {
+        const double p1 = fma(sgn == 0 ? x1 : -x1, r1, un);
+        const double p2 = fma(sgn == 0 ? x2 : -x2, r2, l2);
+        const double p3 = fma(sgn == 0 ? x3 : -x3, r3, l3);
+        double* f = sgn == 0 ? fp : fm;
+        const double S = p2 + p3, D = ca * (p3 - p2);
+        f[0] = c * fma(two_g1, p1, S);
+        f[1 + DIR] = fma(un, f[0], D);
+        f[2 - DIR] = ut * f[0];
+        f[3] = fma(half_q2, f[0], fma(un, D, k * S));
+    }
+#else
     const double g1 = gamma - 1.0, two_g1 = 2.0 * (gamma - 1.0), two_g = 2.0 * gamma;
     const double uu2 = u * u + v * v;
     const double un = DIR == 0 ? u : v, ut = DIR == 0 ? v : u;
@@ -256,6 +290,7 @@ __device__ __forceinline__ void sw_split(double rho, double u, double v, double 
         f[2 - DIR] = ft;
         f[3] = (lp1 * g1 * uu2 + lp2 * 0.5 * q2 + lp3 * 0.5 * q3 + wii) * rho / two_g;
     }
+#endif
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -10,6 +10,7 @@
 // from 2.657 to 0.772 ms; what bounds them now is the integer ALU (72 % busy, 340 instructions a
 // reconstruction before its last trimming). Nothing is computed in fewer bits than before: the
 // words carry 57 to 64 significant bits where a double carries 53.
+//
 // The value. With g_m = lf_m - lf_(m+1), A_k = g_k - g_(k+1), B_0 = A_0 - 2 g_1, B_1 = g_1 + g_2,
 // B_2 = A_2 + 2 g_2 and d_k = 4 (ss + beta_k) = 4 ss + 13/3 A_k^2 + B_k^2 (weno_fast.cuh), the
 // candidates differ by third differences, so that with weights of sum one
