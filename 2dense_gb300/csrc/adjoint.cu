@@ -113,14 +113,14 @@ struct Prim {
 };
 __device__ __forceinline__ Prim prim_of(const double U[4], double gamma) {
     Prim q;
-    q.ir = rcp_nr(U[0]);
+    q.ir = fx::rcp(U[0]);
     q.u = U[1] * q.ir;
     q.v = U[2] * q.ir;
     q.p = (gamma - 1.0) * (U[3] - 0.5 * U[0] * (q.u * q.u + q.v * q.v));
     q.floored = q.p < 0.0;
     if (q.floored) q.p = kPFloor;
     const double a2 = gamma * q.p * q.ir;
-    q.rs = rsqrt_nr(a2);
+    q.rs = fx::rsqrt(a2);
     q.a = a2 * q.rs;
     return q;
 }
@@ -230,12 +230,12 @@ __device__ __forceinline__ Dual operator-(Dual a, Dual b) { return {a.v - b.v, a
 __device__ __forceinline__ Dual operator*(Dual a, Dual b) { return {a.v * b.v, fma(a.d, b.v, a.v * b.d)}; }
 __device__ __forceinline__ Dual operator*(double c, Dual a) { return {c * a.v, c * a.d}; }
 __device__ __forceinline__ Dual operator/(Dual a, Dual b) {
-    const double r = rcp_nr(b.v), q = a.v * r;
+    const double r = fx::rcp(b.v), q = a.v * r;
     return {q, (a.d - q * b.d) * r};
 }
 __device__ __forceinline__ Dual operator/(Dual a, double c) { return {a.v / c, a.d / c}; }
 __device__ __forceinline__ Dual dsqrt(Dual a) {
-    const double rs = rsqrt_nr(a.v), s = a.v * rs;
+    const double rs = fx::rsqrt(a.v), s = a.v * rs;
     return {s, 0.5 * a.d * rs};
 }
 
@@ -859,7 +859,7 @@ __global__ void __launch_bounds__(128, 3) k_char_face(AdjParams a, const double*
                 betas_g(gd, d0, d1, d2, B);
                 WenoTerms wt;
                 weno_terms<true>(gd, d0, d1, d2, wt);
-                const double iN = rcp_nr(wt.N), num = weno_num(wt);
+                const double iN = fx::rcp(wt.N), num = weno_num(wt);
                 const double cv = fma(num, iN, lf[2]);
                 double G[5];
                 weno_grad<true>(gd, B, d0, d1, d2, wt, num * iN, iN, G);
@@ -910,7 +910,7 @@ __global__ void __launch_bounds__(128, 3) k_char_face(AdjParams a, const double*
             betas_g(gd, d0, d1, d2, B);
             WenoTerms wt;
             weno_terms<true>(gd, d0, d1, d2, wt);
-            const double iN = rcp_nr(wt.N);
+            const double iN = fx::rcp(wt.N);
             const double w0 = c30 * wt.v[0] * iN, w1 = c31 * wt.v[1] * iN, w2 = c32 * wt.v[2] * iN;
             const double Q0 = fma(a300, phi[0], fma(a301, phi[1], a302 * phi[2]));
             const double Q1 = fma(a310, phi[1], fma(a311, phi[2], a312 * phi[3]));

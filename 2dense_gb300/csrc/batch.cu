@@ -398,7 +398,7 @@ int dense_batch_create(int n, const dense_config_t* cfgs, dense_batch_t** out) {
         q += align256((size_t)(2 * c.ni + c.nj) * sizeof(double));
         p.sc = (Scalars*)q;
         p.ni = c.ni; p.nj = c.nj; p.P = P; p.plane = (long long)plane;
-        p.gamma = c.gamma; p.cfl = c.cfl; p.delta = c.delta; p.dx = c.dx; p.dy = c.dy; p.dt_const = c.dt;
+        dense::set_gamma(p, c.gamma); p.cfl = c.cfl; p.delta = c.delta; p.dx = c.dx; p.dy = c.dy; p.dt_const = c.dt;
         p.theta_c = dense::theta_c_of(c.delta);
         p.if_const_dt = c.if_const_dt;
         p.bodyforce = c.if_bodyforce && (c.benchmark == DENSE_BENCH_RT || c.benchmark == DENSE_BENCH_RT_REFLECT);

@@ -5,6 +5,7 @@
 #include <cstdint>
 
 #include "../../include/dense2d.h"
+#include "weno_fixed.cuh"
 
 namespace dense {
 
@@ -19,7 +20,8 @@ constexpr int tape_planes(int recon) { return recon == DENSE_RECON_UPWIND5 ? 4 :
 struct Scalars {
     double maxeig[3][2];  // slot s = stage (0..2) that reads it: (max_eig_i, max_eig_j)
     double dt;            // flow_general::dt
-    double dtdx, dtdy;    // dt/dx, dt/dy (time_advance_general.f90:49)
+    double dtdx, dtdy;    // dt/dx, dt/dy (time_advance_general.f90:49); strict kernels
+    fx::Rates rates;      // the same times the stage's factor 1, 1/4 or 2/3; fast kernels
     double t;             // current_time
     double elasp;         // elasp_time
     double t_end;         // loop bound on time (general_main.f90:23)
@@ -55,6 +57,9 @@ struct Params {
     int P;           // row pitch of the padded arrays, in doubles
     long long plane; // doubles per variable plane = NJp * P
     double gamma, cfl, delta, dx, dy, dt_const;
+    // of gamma, for the fast kernels (set_gamma; a divide in every thread would take the FP64 pipe
+    // ten issue slots): gamma - 1, 1/(gamma-1), gamma/(gamma-1), 1/(4 gamma)
+    double g1, ig1, kg, i4g;
     // AdaWENO switch theta > delta written without a divide (fast kernels): with
     // theta = 1/(1 + (sum alpha - 1)^2), N = (sum alpha) D and N - D = tau^2 Q >= 0 (common
     // denominator D), theta > delta <=> D > k (N - D) with k = sqrt(delta/(1-delta))
@@ -86,6 +91,14 @@ inline double theta_c_of(double delta) {
     if (delta >= 1.0) return 1.0;
     const double k = __builtin_sqrt(delta / (1.0 - delta));
     return k / (1.0 + k);
+}
+
+inline void set_gamma(Params& p, double gamma) {
+    p.gamma = gamma;
+    p.g1 = gamma - 1.0;
+    p.ig1 = 1.0 / (gamma - 1.0);
+    p.kg = gamma / (gamma - 1.0);
+    p.i4g = 0.25 / gamma;
 }
 
 // Whether the update of a configuration writes the periodic ghost images (Params::periodic_ghosts).

@@ -144,11 +144,7 @@ __device__ __forceinline__ double upwind5(const double lf[5]) {
 // ---------------------------------------------------------------------------------------------
 // FAST arithmetic. On GB300 an IEEE double divide costs about ten FMA slots of the FP64 pipe,
 // and the reference's WENO weights spend seven divides per stencil. The fast variant
-//  * takes reciprocals and inverse square roots from the hardware seeds (rcp.approx.ftz.f64,
-//    rsqrt.approx.ftz.f64) refined by one third-order step each (with e = 1 - d r, 1/d =
-//    r (1 + e + e^2 + ...); with e = 1 - x y^2, 1/sqrt(x) = y (1 + e/2 + 3e^2/8 + ...)), which
-//    lands within 2 ulp of the correctly rounded result for the positive normal arguments
-//    used here;
+//  * takes reciprocals and square roots from the integer pipes (fastmath.cuh);
 //  * writes the WENO weights over a common denominator: with d_k = ss + beta_k,
 //    P_k = prod_{j != k} d_j^2 and D = prod_j d_j^2,
 //      WENO-JS: alpha_k D = c_k P_k,   WENO-Z: alpha_k D = c_k (D + tau^2 P_k),
@@ -156,7 +152,6 @@ __device__ __forceinline__ double upwind5(const double lf[5]) {
 //    and the AdaWENO test theta > delta becomes sqrt(1-delta) D > sqrt(delta) (N - D) with
 //    N = sum alpha_k D (theta = 1/(1+(sum alpha - 1)^2)), which needs no divide at all.
 // Products of squared d_k stay far inside the double range for d_k in [1e-6, 1e40].
-// (rcp_nr and rsqrt_nr: fastmath.cuh)
 
 
 // AdaWENO's indicator theta = 1/(1 + (sum alpha - 1)^2) from a surrogate's first differences, for the
@@ -183,7 +178,7 @@ __device__ __forceinline__ void recon_grad(const double lf[5], double g[5]) {
     betas_g(gd, d0, d1, d2, B);
     WenoTerms t;
     weno_terms<Z>(gd, d0, d1, d2, t);
-    const double iN = rcp_nr(t.N);
+    const double iN = fx::rcp(t.N);
     weno_grad<Z>(gd, B, d0, d1, d2, t, weno_num(t) * iN, iN, g);
 }
 
@@ -237,7 +232,7 @@ __device__ __forceinline__ void lf_split(const double U[4], double un, double p,
 
 // Steger-Warming (flux_splitting_SW.f90:42-91 xi, :110-160 eta)
 template <int DIR>
-__device__ __forceinline__ void sw_split(double rho, double u, double v, double alpha, double gamma,
+__device__ __forceinline__ void sw_split(const Params& p, double rho, double u, double v, double alpha,
                                          double fp[4], double fm[4]) {
     const double epsl2 = 0.125 * 0.125;
 #if FAST
@@ -245,16 +240,16 @@ __device__ __forceinline__ void sw_split(double rho, double u, double v, double 
     // rho / (4 gamma), S = p_2 + p_3 and D = c a (p_3 - p_2), the components factor into
     //   f_0 = c (2 (gamma-1) p_1 + S),  f_n = u_n f_0 + D,  f_t = u_t f_0,
     //   f_3 = (u^2 + v^2)/2 f_0 + u_n D + c a^2/(gamma-1) S:
-    // 53 operations for both signs, the square roots from rsqrt_nr, where the form below spends
-    // three IEEE square roots and eight divides (481 x 479 WENO-Z sweeps: xi 0.190 -> 0.080 ms, eta
-    // 0.148 -> 0.076 ms). Every sum of a product is an explicit FMA, so that the plain and taping
+    // 53 operations for both signs, the square roots from fx::rsqrt, where the form below spends
+    // three IEEE square roots and eight divides (481 x 479 WENO-Z sweeps: xi 0.190 -> 0.069 ms, eta
+    // 0.148 -> 0.070 ms). Every sum of a product is an explicit FMA, so that the plain and taping
     // sweeps round alike.
     const double un = DIR == 0 ? u : v, ut = DIR == 0 ? v : u;
     const double l2 = un - alpha, l3 = un + alpha;
     const double x1 = fma(un, un, epsl2), x2 = fma(l2, l2, epsl2), x3 = fma(l3, l3, epsl2);
-    const double r1 = rsqrt_nr(x1), r2 = rsqrt_nr(x2), r3 = rsqrt_nr(x3);
-    const double c = rho * (0.25 / gamma), ca = c * alpha, k = ca * (alpha * (1.0 / (gamma - 1.0)));
-    const double half_q2 = 0.5 * fma(un, un, ut * ut), two_g1 = 2.0 * (gamma - 1.0);
+    const double r1 = fx::rsqrt(x1), r2 = fx::rsqrt(x2), r3 = fx::rsqrt(x3);
+    const double c = rho * p.i4g, ca = c * alpha, k = ca * (alpha * p.ig1);
+    const double half_q2 = 0.5 * fma(un, un, ut * ut), two_g1 = 2.0 * p.g1;
 #pragma unroll
     for (int sgn = 0; sgn < 2; ++sgn) {
         const double p1 = fma(sgn == 0 ? x1 : -x1, r1, un);
@@ -268,6 +263,7 @@ __device__ __forceinline__ void sw_split(double rho, double u, double v, double 
         f[3] = fma(half_q2, f[0], fma(un, D, k * S));
     }
 #else
+    const double gamma = p.gamma;
     const double g1 = gamma - 1.0, two_g1 = 2.0 * (gamma - 1.0), two_g = 2.0 * gamma;
     const double uu2 = u * u + v * v;
     const double un = DIR == 0 ? u : v, ut = DIR == 0 ? v : u;
@@ -376,13 +372,13 @@ struct EigFast {
 template <int DIR>
 __device__ __forceinline__ bool roe_eig_fast(double g1, double sl, double sr, double ul, double ur,
                                              double vl, double vr, double hl, double hr, EigFast& e) {
-    const double w = sr * rcp_nr(sl + sr);
+    const double w = sr * fx::rcp(sl + sr);
     const double u0 = fma(w, ur - ul, ul);
     const double v0 = fma(w, vr - vl, vl);
     e.h0 = fma(w, hr - hl, hl);
     e.uu0 = 0.5 * fma(u0, u0, v0 * v0);
     const double c2 = g1 * (e.h0 - e.uu0);
-    const double ia = rsqrt_nr(c2);
+    const double ia = fx::rsqrt(c2);
     e.a0 = c2 * ia;
     e.ia5 = 0.5 * ia;
     e.ih = g1 * ia * e.ia5;
@@ -461,8 +457,14 @@ __device__ __forceinline__ void stage_scalars(const Params& p, int irk) {
         const double dt_eta = p.dy / sc->maxeig[slot][1];
         sc->dt = p.cfl * dt_xi * dt_eta / (dt_xi + dt_eta);
     }
+#if FAST
+    // with the stage's factor of the flux differences (stage 2: 1/4, stage 3: 2/3) folded in
+    const double kb = irk == 1 ? 1.0 : irk == 2 ? 1.0 / 4.0 : 2.0 / 3.0;
+    sc->rates = fx::rates_of(kb * (sc->dt / p.dx), kb * (sc->dt / p.dy));
+#else
     sc->dtdx = sc->dt / p.dx;
     sc->dtdy = sc->dt / p.dy;
+#endif
     const int next = irk % 3;
     sc->maxeig[next][0] = 0.0;
     sc->maxeig[next][1] = 0.0;
@@ -521,8 +523,7 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
             const double lam = p.splitting == DENSE_SPLIT_LLF ? fabs(un) + p.prim[4 * p.plane + o] : lam_g;
             lf_split<DIR>(U, un, pr, lam, fp, fm);
         } else {
-            sw_split<DIR>(p.prim[o], p.prim[p.plane + o], p.prim[2 * p.plane + o], p.prim[4 * p.plane + o],
-                          p.gamma, fp, fm);
+            sw_split<DIR>(p, p.prim[o], p.prim[p.plane + o], p.prim[2 * p.plane + o], p.prim[4 * p.plane + o], fp, fm);
         }
 #pragma unroll
         for (int v = 0; v < 4; ++v) { sF[v * NCELL + at(r, c)] = fp[v]; sF[(4 + v) * NCELL + at(r, c)] = fm[v]; }
@@ -598,7 +599,7 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
                     betas_g(gd, d0, d1, d2, B);
                     WenoTerms tt;
                     weno_terms<Z>(gd, d0, d1, d2, tt);
-                    const double iN = rcp_nr(tt.N);
+                    const double iN = fx::rcp(tt.N);
                     weno_grad<Z>(gd, B, d0, d1, d2, tt, weno_num(tt) * iN, iN, g);
 #pragma unroll
                     for (int m = 0; m < 5; ++m) tape_at[((m0 + m) * 4 + v) * ts] = g[m];
@@ -661,7 +662,7 @@ __global__ void k_flux_noop(Params p, int irk) {
 // whole block then works through the queue on full warps.
 // What bounds it: the FP64 pipe. The surrogate's weights and the smooth branch run on the integer
 // pipes (weno_fixed.cuh), which leaves some 55 FP64 instructions an interface of 150 and took the
-// 1920 x 480 double Mach reflection's sweeps from 0.282 and 0.305 ms to 0.149 and 0.174.
+// 1920 x 480 double Mach reflection's sweeps from 0.282 and 0.305 ms to 0.149 and 0.172.
 // Dynamic shared memory of one characteristic sweep block, in doubles: the tile's split fluxes
 // sF[8][NL][NC] and primitives sQ[4][NL][NC]; per-cell sqrt(rho) sS (104, fast); the split fluxes'
 // forward differences along the sweep sDF[8][NL][NC] (fast); and one region R that AdaWENO uses
@@ -708,7 +709,7 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
     if (DIR == 0 && bx == 0 && by == 0 && tid == 0) stage_scalars(p, irk);
     const double lam = p.sc->maxeig[slot][DIR];
     const int NIp = p.ni + 2 * kB, NJp = p.nj + 2 * kB;
-    const double g1 = p.gamma - 1.0, kg = p.gamma / (p.gamma - 1.0);
+    const double g1 = p.g1, kg = p.kg;
     if (ADAPT && tid == 0) qn = 0;
     (void)g1; (void)kg; (void)NL;
     // tile cell (r, c) -> offset; k runs along the sweep, (ox, oy) is the interface's tile position
@@ -725,9 +726,9 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
         for (int v = 0; v < 4; ++v) q[v] = p.prim[v * p.plane + o];
         lf_split<DIR>(U, q[1 + DIR], q[3], lam, fp, fm);
         if constexpr (kStageHS) {
-            const double ir = rcp_nr(q[0]);
+            const double ir = fx::rcp(q[0]);
             q[3] = fma(kg * q[3], ir, 0.5 * fma(q[1], q[1], q[2] * q[2]));
-            sS[at(r, c)] = q[0] * rsqrt_nr(q[0]);
+            sS[at(r, c)] = fx::sqrt_normal(q[0]);
         }
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
@@ -815,10 +816,10 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
             const double rl = SQ(0, kl, ox, oy), rr = SQ(0, kr, ox, oy);
             const double ul = SQ(1, kl, ox, oy), ur = SQ(1, kr, ox, oy);
             const double vl = SQ(2, kl, ox, oy), vr = SQ(2, kr, ox, oy);
-            hl = fma(kg * SQ(3, kl, ox, oy), rcp_nr(rl), 0.5 * fma(ul, ul, vl * vl));
-            hr = fma(kg * SQ(3, kr, ox, oy), rcp_nr(rr), 0.5 * fma(ur, ur, vr * vr));
-            sl = rl * rsqrt_nr(rl);
-            sr = rr * rsqrt_nr(rr);
+            hl = fma(kg * SQ(3, kl, ox, oy), fx::rcp(rl), 0.5 * fma(ul, ul, vl * vl));
+            hr = fma(kg * SQ(3, kr, ox, oy), fx::rcp(rr), 0.5 * fma(ur, ur, vr * vr));
+            sl = fx::sqrt_normal(rl);
+            sr = fx::sqrt_normal(rr);
         }
         const bool ok = roe_eig_fast<DIR>(g1, sl, sr, SQ(1, kl, ox, oy), SQ(1, kr, ox, oy),
                                           SQ(2, kl, ox, oy), SQ(2, kr, ox, oy), hl, hr, e);
@@ -1076,7 +1077,7 @@ __device__ __forceinline__ void prim_cell(const Params& p, long long o, const do
                                           double& e2, unsigned& flags, double pv[5]) {
     const double rho = q[0];
 #if FAST
-    const double ir = rcp_nr(rho);
+    const double ir = fx::rcp(rho);
     const double u = q[1] * ir;
     const double v = q[2] * ir;
 #else
@@ -1085,7 +1086,7 @@ __device__ __forceinline__ void prim_cell(const Params& p, long long o, const do
 #endif
 #if FAST
     // rho (u^2 + v^2) = m_u u + m_v v
-    double pr = (p.gamma - 1.0) * fma(-0.5, fma(q[1], u, q[2] * v), q[3]);
+    double pr = p.g1 * fma(-0.5, fma(q[1], u, q[2] * v), q[3]);
 #else
     double pr = (p.gamma - 1.0) * (q[3] - 0.5 * rho * (u * u + v * v));
 #endif
@@ -1095,7 +1096,7 @@ __device__ __forceinline__ void prim_cell(const Params& p, long long o, const do
     const long long pb = __double_as_longlong(pr), pm = pb & 0x7fffffffffffffffLL;
     if (pb < 0 && pm != 0 && pm <= 0x7ff0000000000000LL) { pr = kPFloor; flags |= DENSE_FLAG_P_FLOOR; }
     const double a2 = p.gamma * pr * ir;
-    const double alpha = __double_as_longlong(a2) > 0 ? a2 * rsqrt_nr(a2) : sqrt(a2);
+    const double alpha = __double_as_longlong(a2) > 0 ? fx::sqrt_normal(a2) : sqrt(a2);
 #else
     if (pr < 0.0) { pr = kPFloor; flags |= DENSE_FLAG_P_FLOOR; }
     const double alpha = sqrt(p.gamma * pr / rho);
@@ -1145,7 +1146,12 @@ __device__ __forceinline__ void update_block(const Params& p, int i, int j) {
     unsigned flags = 0;
     if (i < p.ni && j < p.nj) {
         const Scalars* sc = p.sc;
-        const double dtdx = sc->dtdx, dtdy = sc->dtdy, dt = sc->dt;
+        const double dt = sc->dt;
+#if FAST
+        const fx::Rates rates = sc->rates;
+#else
+        const double dtdx = sc->dtdx, dtdy = sc->dtdy;
+#endif
         const long long o = cidx(p, i + kB, j + kB);
         // the cell's faces: xi left/right, eta bottom/top; planes hxs, hes apart
         const long long hxs = (long long)p.nj * (p.ni + 1), hes = (long long)(p.nj + 1) * p.ni;
@@ -1155,29 +1161,35 @@ __device__ __forceinline__ void update_block(const Params& p, int i, int j) {
 #if FAST
         // stage 2: 3/4 q0 + 1/4 (...); stage 3: 1/3 q0 + 2/3 (...)
         const double ka = IRK == 2 ? 3.0 / 4.0 : 1.0 / 3.0, kb = IRK == 2 ? 1.0 / 4.0 : 2.0 / 3.0;
-        const double cx = kb * dtdx, cy = kb * dtdy;
-        (void)ka; (void)cx; (void)cy;
+        (void)ka; (void)kb;
 #endif
         double q[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-            const double dh_dxi = p.hx[v * hxs + hxr] - p.hx[v * hxs + hxl];
-            const double dh_deta = p.he[v * hes + her] - p.he[v * hes + hel];
             const double qc = p.cons[v * p.plane + o];
             double qn;
+#if FAST
+            // a q0 + b (qc - (dt/dx dh_xi + dt/dy dh_eta)), b folded into the rates
+            const double d = fx::flux_change(p.hx[v * hxs + hxl], p.hx[v * hxs + hxr], p.he[v * hes + hel],
+                                             p.he[v * hes + her], rates);
+            if (IRK == 1) {
+                p.cons0[v * p.plane + o] = qc;
+                qn = qc - d;
+            } else {
+                qn = fma(ka, p.cons0[v * p.plane + o], fma(kb, qc, -d));
+            }
+#else
+            const double dh_dxi = p.hx[v * hxs + hxr] - p.hx[v * hxs + hxl];
+            const double dh_deta = p.he[v * hes + her] - p.he[v * hes + hel];
             if (IRK == 1) {
                 p.cons0[v * p.plane + o] = qc;
                 qn = qc - dtdx * dh_dxi - dtdy * dh_deta;
             } else {
                 const double q0 = p.cons0[v * p.plane + o];
-#if FAST
-                // a q0 + b (qc - (dt/dx dh_xi + dt/dy dh_eta)), b folded into dt/dx and dt/dy
-                qn = fma(ka, q0, fma(kb, qc, -fma(cx, dh_dxi, cy * dh_deta)));
-#else
                 if (IRK == 2) qn = 3.0 / 4.0 * q0 + 1.0 / 4.0 * qc - 1.0 / 4.0 * (dtdx * dh_dxi + dtdy * dh_deta);
                 else          qn = 1.0 / 3.0 * q0 + 2.0 / 3.0 * qc - 2.0 / 3.0 * (dtdx * dh_dxi + dtdy * dh_deta);
-#endif
             }
+#endif
             q[v] = qn;
         }
         if (p.bodyforce) {
@@ -1450,13 +1462,13 @@ __device__ __forceinline__ void bc_block(const Params& p, int bx) {
 // Resident blocks the register allocation of a characteristic sweep is sized for. AdaWENO's
 // blocks stall on the barriers of their work queue, which a third block per SM hides (80
 // registers, a few bytes spilled; sweeps of the 1920 x 480 double Mach reflection, xi and eta:
-// 0.149 and 0.174 ms at three blocks; before its weights' last trimming 0.159 and 0.180 at three,
+// 0.149 and 0.172 ms at three blocks; before its weights' last trimming 0.159 and 0.180 at three,
 // 0.180 and 0.203 at two, 0.162 and 0.188 at four). The 104
 // sweeps' four inlined integer
 // reconstructions would take 160 registers; at 1024 resident threads (64 registers) the sweeps of
 // the 256 x 1024 Rayleigh-Taylor case took 0.127 (xi) and 0.111 ms (eta), at 768 0.131 and 0.113,
-// unbounded 0.141 and 0.158 (0.123 and 0.104 after that trimming, and 0.340 and 0.293 with the
-// reconstructions in FP64).
+// unbounded 0.141 and 0.158 (now 0.106 and 0.098, the roots on the integer pipes too; 0.340 and
+// 0.293 with the reconstructions in FP64).
 constexpr int char_min_blocks(bool adapt, int nt) { return adapt ? 3 : 1024 / nt; }
 template <int DIR, int SPL, int REC, int TX, int TY, bool TAPE = false, int TZ = 1>
 __global__ void __launch_bounds__(TX* TY* TZ) k_flux_cw(Params p, int irk) {
@@ -1472,8 +1484,13 @@ __global__ void k_prim(Params p, int slot) {
     grid_dependency_wait();
     prim_block(p, slot, blockIdx.x, blockIdx.y);
 }
+// Update: six resident blocks (42 registers). What bounded it was the FP64 pipe (50 instructions a
+// cell); with the reciprocal and root of get_primary on the integer pipes 0.356 -> 0.283 ms of a 2048 x
+// 2048 stage, with the flux change there too 0.236, with a sixth block 0.201 (200 B a cell at the
+// copy rate: 0.124 ms).
+constexpr int kUpdateBlocks = 6;
 template <int IRK>
-__global__ void k_update(Params p) {
+__global__ void __launch_bounds__(256, kUpdateBlocks) k_update(Params p) {
     grid_dependency_wait();
     update_block<IRK>(p, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y);
 }
@@ -1515,7 +1532,7 @@ __global__ void kb_prim(const Params* tab, const int3* map, int slot) {
     prim_block(sp, slot, m.y, m.z);
 }
 template <int IRK>
-__global__ void kb_update(const Params* tab, const int3* map) {
+__global__ void __launch_bounds__(256, kUpdateBlocks) kb_update(const Params* tab, const int3* map) {
     DENSE_BATCH_PROLOGUE
     update_block<IRK>(sp, m.y * blockDim.x + threadIdx.x, m.z * blockDim.y + threadIdx.y);
 }
@@ -2105,15 +2122,15 @@ const KernelTable* kernels_fast() {
 
 #if !DENSE_VARIANT_STRICT && !DENSE_CHECK
 // Accuracy check of the fast reciprocal and inverse square root against CUDA's IEEE divide and
-// square root: out[4k..4k+3] = (rcp_nr(x), 1/x, rsqrt_nr(x), 1/sqrt(x)) for each x[k].
+// square root: out[4k..4k+3] = (fx::rcp(x), 1/x, fx::rsqrt(x), 1/sqrt(x)) for each x[k].
 namespace {
 __global__ void k_fastmath(const double* x, double* out, int n) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const double v = x[k];
-    out[4 * k + 0] = dense::rcp_nr(v);
+    out[4 * k + 0] = dense::fx::rcp(v);
     out[4 * k + 1] = 1.0 / v;
-    out[4 * k + 2] = dense::rsqrt_nr(v);
+    out[4 * k + 2] = dense::fx::rsqrt(v);
     out[4 * k + 3] = 1.0 / sqrt(v);
 }
 }  // namespace

@@ -157,7 +157,7 @@ extern "C" int dense_stage_noalloc(const dense_config_t* cfg, int irk, double cu
     p.sc = ptr.sc;
     p.ni = cfg->ni; p.nj = cfg->nj; p.P = (NIp + 1) & ~1;
     p.plane = (long long)NJp * p.P;
-    p.gamma = cfg->gamma; p.cfl = cfg->cfl; p.delta = cfg->delta; p.dx = cfg->dx; p.dy = cfg->dy;
+    dense::set_gamma(p, cfg->gamma); p.cfl = cfg->cfl; p.delta = cfg->delta; p.dx = cfg->dx; p.dy = cfg->dy;
     p.dt_const = cfg->dt;
     p.theta_c = dense::theta_c_of(cfg->delta);
     p.if_const_dt = cfg->if_const_dt;

@@ -1,6 +1,6 @@
 // weno_fast.cuh -- the WENO-JS5 / WENO-Z5 reconstruction terms of the fast kernels and their
 // stencil gradient, shared by the sweeps (kernels.cu) and the discrete adjoint's face-level
-// reverse (adjoint.cu). Included inside each file's own namespace (both need dense::rcp_nr).
+// reverse (adjoint.cu). Included inside each file's own namespace (both see dense::fx).
 #pragma once
 
 // weno module constants (source/inv_scheme/weno_mod.f90:3-14,37)
@@ -70,7 +70,7 @@ template <bool Z>
 __device__ __forceinline__ double weno_from_d(double lf2, const double g[4], double d0, double d1, double d2) {
     WenoTerms t;
     weno_terms<Z>(g, d0, d1, d2, t);
-    return weno_value(t, rcp_nr(t.N), lf2);
+    return weno_value(t, fx::rcp(t.N), lf2);
 }
 
 // Gradient of the WENO reconstruction with respect to its stencil, g[m] = dW/dlf[m], for the
@@ -96,7 +96,7 @@ __device__ __forceinline__ void weno_grad(const double gd[4], const double B[3],
         E[k] = fma(-cs[k], corr, t.r[k]);  // (q_k - W) c_k
         u[k] = t.v[k] * iN;                // w_k / c_k
     }
-    const double iD = 4.0 * rcp_nr(t.D);
+    const double iD = 4.0 * fx::rcp(t.D);
     const double id0 = d0 * (t.P[0] * iD), id1 = d1 * (t.P[1] * iD), id2 = d2 * (t.P[2] * iD);  // 1/(ss + beta_k)
     const double A0 = gd[0] - gd[1], B0 = B[0];
     const double A1 = gd[1] - gd[2], B1 = B[1];
@@ -145,7 +145,7 @@ template <bool Z>
 __device__ __forceinline__ void weno_weight_grad(const double gd[4], const double B[3], double d0, double d1,
                                                  double d2, const WenoTerms& t, const double E[3], double iN,
                                                  double g[5]) {
-    const double iD = 4.0 * rcp_nr(t.D);
+    const double iD = 4.0 * fx::rcp(t.D);
     const double id0 = d0 * (t.P[0] * iD), id1 = d1 * (t.P[1] * iD), id2 = d2 * (t.P[2] * iD);  // 1/(ss + beta_k)
     const double A0 = gd[0] - gd[1], A1 = gd[1] - gd[2], A2 = gd[2] - gd[3];
     double r0, r1, r2;

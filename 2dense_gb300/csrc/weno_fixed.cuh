@@ -36,117 +36,10 @@
 //
 // The functions compile for the host too, where the tests compare them with long double.
 #pragma once
-#include <cstdint>
-#ifndef __CUDACC__
-#include <cmath>
-#include <cstring>
-#define DENSE_FX inline
-#else
-#define DENSE_FX __host__ __device__ __forceinline__
-#endif
+#include "fastmath.cuh"
 
 namespace dense {
 namespace fx {
-
-typedef uint32_t u32;
-typedef uint64_t u64;
-typedef int64_t i64;
-
-DENSE_FX u32 hi32(u64 a) { return (u32)(a >> 32); }
-DENSE_FX u64 wide(u32 a, u32 b) { return (u64)a * b; }
-DENSE_FX int imax(int a, int b) { return a > b ? a : b; }
-DENSE_FX int imin(int a, int b) { return a < b ? a : b; }
-DENSE_FX u32 umax(u32 a, u32 b) { return a > b ? a : b; }
-DENSE_FX u32 umin(u32 a, u32 b) { return a < b ? a : b; }
-DENSE_FX u64 abs64(i64 a) {
-    const u64 s = (u64)(a >> 63);
-    return ((u64)a ^ s) - s;
-}
-// a >> n with 0 for n > 63, as PTX defines it
-DENSE_FX u64 shr(u64 a, u32 n) {
-#ifdef __CUDA_ARCH__
-    u64 r;
-    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(a), "r"(n));
-    return r;
-#else
-    return n > 63 ? 0 : a >> n;
-#endif
-}
-DENSE_FX int clz32(u32 a) {
-#ifdef __CUDA_ARCH__
-    return __clz((int)a);
-#else
-    return a ? __builtin_clz(a) : 32;
-#endif
-}
-DENSE_FX int clz64(u64 a) {
-#ifdef __CUDA_ARCH__
-    return __clzll((long long)a);
-#else
-    return a ? __builtin_clzll(a) : 64;
-#endif
-}
-DENSE_FX u64 bits(double d) {
-#ifdef __CUDA_ARCH__
-    return (u64)__double_as_longlong(d);
-#else
-    u64 r;
-    memcpy(&r, &d, 8);
-    return r;
-#endif
-}
-DENSE_FX double from_bits(u64 b) {
-#ifdef __CUDA_ARCH__
-    return __longlong_as_double((long long)b);
-#else
-    double r;
-    memcpy(&r, &b, 8);
-    return r;
-#endif
-}
-DENSE_FX u32 float_bits(float f) {
-#ifdef __CUDA_ARCH__
-    return __float_as_uint(f);
-#else
-    u32 r;
-    memcpy(&r, &f, 4);
-    return r;
-#endif
-}
-DENSE_FX float rcp_seed(float x) {
-#ifdef __CUDA_ARCH__
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-#else
-    return 1.0f / x;
-#endif
-}
-
-// a b / 2^64, at most 2 below its floor: the product of the lower halves is left out
-DENSE_FX u64 mulhi(u64 a, u64 b) {
-    const u64 m1 = wide(hi32(a), (u32)b), m2 = wide((u32)a, hi32(b));
-    return wide(hi32(a), hi32(b)) + hi32(m1) + hi32(m2);
-}
-// the same for a below 2^63 and b at most 2^63, whose middle products add up within a word
-DENSE_FX u64 mulhi63(u64 a, u64 b) {
-    const u64 m = wide(hi32(a), (u32)b) + wide((u32)a, hi32(b));
-    return wide(hi32(a), hi32(b)) + hi32(m);
-}
-DENSE_FX u64 sqhi(u64 a) { return wide(hi32(a), hi32(a)) + (wide(hi32(a), (u32)a) >> 31); }
-
-// 2^125 / n for n in [2^62, 2^63), relative error below 2^-59: x0 = 2^61 / (n / 2^32) to 22 bits
-// from the hardware's reciprocal, e = 1 - x0 n, and 1/n = x0 (1 + e + e^2 + ...), as rcp_nr has it
-DENSE_FX u64 reciprocal(u64 n) {
-    const u32 nh = hi32(n);
-    // 2^53 (1 - 2^-22) x + 2^23 holds 2^53 x0 in its mantissa, below the next binade
-    const float t = fmaf(rcp_seed((float)nh), 9007199254740992.0f * (1.0f - 1.0f / 4194304.0f), 8388608.0f);
-    const u32 x0 = (float_bits(t) & 0x7fffffu) << 8;
-    const i64 e = (i64)((1ull << 61) - (wide(x0, nh) + hi32(wide(x0, (u32)n))));  // 2^61 (1 - x0 n), below 2^42
-    const int es = (int)(e >> 11);
-    const i64 f = e + (i64)((u64)((i64)es * es) >> 39);  // 2^61 (e + e^2)
-    return ((u64)x0 << 32) + (u64)(((i64)(int)x0 * (int)(f >> 11)) >> 18) + (wide(x0, (u32)f & 0x7ffu) >> 29);
-}
 
 // Exponents of doubles in place (bits 20..30 of the upper word).
 constexpr u32 kExpMask = 0x7ff00000u;
@@ -333,6 +226,38 @@ DENSE_FX i64 correction6_by(const double g[4], u32 eh, u64 f0, u64 f2) {
 // The largest exponent of a stencil's differences.
 DENSE_FX u32 exponent_of(const double g[4]) {
     return umax(umax(exponent(g[0]), exponent(g[1])), umax(exponent(g[2]), exponent(g[3])));
+}
+
+// dt/dx and dt/dy as fixed-point factors of one exponent, below 2^62 (in units of 2^-shift), and
+// dt's sign; shift kNoShift where one is not finite.
+constexpr int kNoShift = 1 << 20;
+struct Rates {
+    u64 x, y;
+    int shift;
+    u32 sign;  // 0 or the sign bit of an upper word
+};
+DENSE_FX Rates rates_of(double dtdx, double dtdy) {
+    const u64 bx = bits(dtdx), by = bits(dtdy), top = 0x2000000000000000ull;
+    const u32 ex = (hi32(bx) >> 20) & 0x7ffu, ey = (hi32(by) >> 20) & 0x7ffu, e = umax(ex, ey);
+    Rates r;
+    r.x = shr(((bx << 9) & (top - 1)) | top, e - ex);
+    r.y = shr(((by << 9) & (top - 1)) | top, e - ey);
+    r.shift = e == 0x7ffu ? kNoShift : 61 + 1023 - (int)e;
+    r.sign = hi32(bx) & 0x80000000u;
+    return r;
+}
+// dt/dx (xr - xl) + dt/dy (yr - yl): the differences exact in fixed point, their products with the rates
+// and the sum truncated below 2^-57 of the largest flux times the larger rate, rounded once.
+DENSE_FX double flux_change(double xl, double xr, double yl, double yr, const Rates& r) {
+    const u32 top = umax(umax(exponent(xl), exponent(xr)), umax(exponent(yl), exponent(yr)));
+    const u32 eh = umax(top, kExpMin);
+    const i64 X = to_fixed(xr, eh) - to_fixed(xl, eh), Y = to_fixed(yr, eh) - to_fixed(yl, eh);  // below 2^59
+    const i64 t = scaled(r.x, X * 8) + scaled(r.y, Y * 8);     // 2^(shift - 61) of the sum, below 2^61
+    const int e = (int)(eh >> 20) + 61 - r.shift;
+    double d = to_double(t, (u32)imax(e, 64) << 20, top);
+    if (e < 64) d = 0.0;                                       // below 2^-950: also where a rate is 0
+    if (r.shift == kNoShift) d = from_bits(0x7ff8000000000000ull);
+    return from_bits(bits(d) ^ ((u64)r.sign << 32));
 }
 
 }  // namespace fx

@@ -51,3 +51,18 @@ def test_adaptive(lines):
     assert (wrong, ends, nans) == (0, 0, 0)
     assert near < 0.1 * n and 0.05 * n < smooth < 0.95 * n
     assert worst <= 16 * 2.0 ** -53
+
+
+def test_roots(lines):
+    """Reciprocal, inverse square root and square root: values good to 2^-58, rounded once, so half an
+    ulp and 2^-5 of one; a NaN outside their ranges."""
+    (row,) = [x[1:] for x in lines if x[0] == "roots"]
+    assert max(float(v) for v in row[:3]) <= 0.5 + 2.0 ** -5 and int(row[3]) == 0
+
+
+def test_flux_change(lines):
+    """The update's dt/dx dh_xi + dt/dy dh_eta: the rates' own rounding aside, truncations of 2^-57 and
+    one rounding of the result, half an ulp; twice that bounds it. Odd in the fluxes and under a
+    mirror image, zero for equal fluxes, NaN for what is not finite."""
+    ((worst, odd, bad),) = [x[1:] for x in lines if x[0] == "change"]
+    assert float(worst) <= 2.0 and int(odd) == 0 and int(bad) == 0

@@ -11,7 +11,9 @@
 #define __device__
 #define __forceinline__ inline
 namespace f64 {
-double rcp_nr(double d) { return 1.0 / d; }
+namespace fx {  // the FP64 form with an IEEE reciprocal
+static double rcp(double d) { return 1.0 / d; }
+}
 #include "../2dense_gb300/csrc/weno_fast.cuh"
 template <bool Z> double recon(double lf2, const double g[4]) {
     double d0, d1, d2, B[3];
@@ -177,7 +179,69 @@ void adaptive() {
     printf("adaptive %d %d %d %d %d %d %.17g\n", n, wrong, near, ends, nans, smooth, worst);
 }
 
+// rcp, rsqrt and sqrt_normal: the largest error in ulp over mantissas and exponents, and the arguments
+// outside their range
+void roots() {
+    std::mt19937_64 r(21);
+    double worst[3] = {0, 0, 0};
+    for (int t = 0; t < 1000000; ++t) {
+        double x;
+        if (t < 1000) x = 1.0 + t * 0x1p-52;
+        else if (t < 2000) x = 2.0 - (t - 999) * 0x1p-52;
+        else if (t < 3000) x = 4.0 - (t - 1999) * 0x1p-51;
+        else x = std::ldexp(1.0 + (double)(r() >> 12) * 0x1p-52, (int)(r() % 2000) - 1000);
+        const ld want[3] = {1.0L / x, 1.0L / sqrtl(x), sqrtl(x)};
+        const double got[3] = {dense::fx::rcp(x), dense::fx::rsqrt(x), dense::fx::sqrt_normal(x)};
+        for (int k = 0; k < 3; ++k) {
+            const double w = (double)want[k], ulp = std::nextafter(w, 1e308) - w;
+            worst[k] = std::max(worst[k], (double)(fabsl(got[k] - want[k]) / ulp));
+        }
+    }
+    int bad = dense::fx::rcp(-8.0) != -0.125;
+    const double inf = std::numeric_limits<double>::infinity(), nan = std::numeric_limits<double>::quiet_NaN();
+    for (double x : {0.0, -0.0, inf, -inf, nan, 1e-310}) bad += !std::isnan(dense::fx::rcp(x));
+    for (double x : {0.0, -1.0, inf, nan, 1e-310})
+        bad += !std::isnan(dense::fx::rsqrt(x)) + !std::isnan(dense::fx::sqrt_normal(x));
+    printf("roots %.17g %.17g %.17g %d\n", worst[0], worst[1], worst[2], bad);
+}
+
+// the update's flux change against long double, in units of 2^-53 of the largest flux times the larger
+// rate; its oddness; what is not finite
+void change() {
+    std::mt19937_64 r(31);
+    std::uniform_real_distribution<double> u(-1, 1);
+    double worst = 0;
+    int odd = 0, bad = 0;
+    const double inf = std::numeric_limits<double>::infinity(), nan = std::numeric_limits<double>::quiet_NaN();
+    for (int t = 0; t < 200000; ++t) {
+        const double size = std::pow(10.0, 6 * u(r)), small = std::pow(10.0, -8 * std::fabs(u(r)));
+        double h[4];
+        const double bx = u(r), by = u(r);
+        for (int k = 0; k < 4; ++k) h[k] = size * ((k < 2 ? bx : by) + small * u(r));
+        const double dtdx = std::pow(10.0, -2 + 2 * u(r)), dtdy = dtdx * std::pow(10.0, 3 * u(r)), sg = t & 1 ? -1.0 : 1.0;
+        const dense::fx::Rates q = dense::fx::rates_of(sg * dtdx, sg * dtdy);
+        const ld want = (ld)(sg * dtdx) * ((ld)h[1] - h[0]) + (ld)(sg * dtdy) * ((ld)h[3] - h[2]);
+        const double got = dense::fx::flux_change(h[0], h[1], h[2], h[3], q);
+        double big = 0;
+        for (double x : h) big = std::max(big, std::fabs(x));
+        worst = std::max(worst, (double)(fabsl(got - want) / (0x1p-53L * (big * std::max(dtdx, dtdy) + fabsl(want)))));
+        odd += dense::fx::flux_change(-h[0], -h[1], -h[2], -h[3], q) != -got;
+        odd += dense::fx::flux_change(h[1], h[0], h[3], h[2], q) != -got;
+        const double x = t % 3 == 0 ? nan : t % 3 == 1 ? inf : -inf, keep = h[t & 3];
+        h[t & 3] = x;
+        bad += !std::isnan(dense::fx::flux_change(h[0], h[1], h[2], h[3], q));
+        h[t & 3] = keep;
+        bad += !std::isnan(dense::fx::flux_change(h[0], h[1], h[2], h[3], dense::fx::rates_of(x, dtdy)));
+        bad += !std::isnan(dense::fx::flux_change(h[0], h[1], h[2], h[3], dense::fx::rates_of(dtdx, x)));
+        bad += dense::fx::flux_change(h[0], h[1], h[2], h[3], dense::fx::rates_of(0.0, 0.0)) != 0.0;
+        bad += dense::fx::flux_change(h[0], h[0], h[2], h[2], q) != 0.0;
+    }
+    printf("change %.17g %d %d\n", worst, odd, bad);
+}
+
 int main() {
+    roots();
+    change();
     std::mt19937_64 r(3);
     double worst = 0;
     for (int t = 0; t < 2000000; ++t) {
