@@ -73,7 +73,7 @@ DENSE_FX i64 to_fixed(double g, u32 eh) {
 DENSE_FX double to_double(i64 c, u32 eh, u32 top) {
     const u64 a = abs64(c);
     const int n = clz64(a) & 63;
-    u64 r = ((u64)c & 0x8000000000000000ull) | (((u64)((eh >> 20) + 5 - n) << 52) + (((a << n) + 0x400) >> 11));
+    u64 r = ((u64)c & 0x8000000000000000ull) | (((u64)((eh >> 20) + 5 - n) << 52) + ((((a << n) >> 10) + 1) >> 1));
     if (a == 0) r = 0;
     if (top >= kExpMax) r = 0x7ff8000000000000ull;
     return from_bits(r);

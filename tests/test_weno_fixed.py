@@ -66,3 +66,8 @@ def test_flux_change(lines):
     mirror image, zero for equal fluxes, NaN for what is not finite."""
     ((worst, odd, bad),) = [x[1:] for x in lines if x[0] == "change"]
     assert float(worst) <= 2.0 and int(odd) == 0 and int(bad) == 0
+
+
+def test_conversion(lines):
+    """Fixed point to double is a nearest rounding at every width, up to the next power of two too."""
+    assert [x[1] for x in lines if x[0] == "conversion"] == ["0"]

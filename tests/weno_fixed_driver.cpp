@@ -239,7 +239,25 @@ void change() {
     printf("change %.17g %d %d\n", worst, odd, bad);
 }
 
+// to_double against the host's own rounding of an integer: every width, and the values that round up
+// to the next power of two
+void conversion() {
+    std::mt19937_64 r(41);
+    int bad = 0;
+    for (int k = 1; k < 63; ++k)
+        for (int t = 0; t < 4000; ++t) {
+            dense::fx::i64 c = (dense::fx::i64)(t < 2100 ? (1ull << k) - (unsigned long long)t : r() >> (64 - k));
+            if (c <= 0) continue;
+            if (t & 1) c = -c;
+            const double want = std::ldexp((double)c, 3), got = dense::fx::to_double(c, 1083u << 20, 0);
+            // halves go away from zero here, to even there
+            if (got != want && std::fabs((double)((ld)got / 8 - c)) > std::fabs((double)((ld)want / 8 - c))) ++bad;
+        }
+    printf("conversion %d\n", bad);
+}
+
 int main() {
+    conversion();
     roots();
     change();
     std::mt19937_64 r(3);
