@@ -854,15 +854,15 @@ __global__ void __launch_bounds__(128, 3) k_char_face(AdjParams a, const double*
 #pragma unroll
                 for (int m = 0; m < 5; ++m)
                     lf[m] = fma(M[0][k], F(m, 0), fma(M[1][k], F(m, 1), fma(M[2][k], F(m, 2), M[3][k] * F(m, 3))));
-                double gd[4], d0, d1, d2, B[3];
+                // the field's value and gradient on the integer pipes, as the taping sweeps take them
+                double gd[4], G[5];
                 first_differences(lf, gd);
-                betas_g(gd, d0, d1, d2, B);
-                WenoTerms wt;
-                weno_terms<true>(gd, d0, d1, d2, wt);
-                const double iN = fx::rcp(wt.N), num = weno_num(wt);
-                const double cv = fma(num, iN, lf[2]);
-                double G[5];
-                weno_grad<true>(gd, B, d0, d1, d2, wt, num * iN, iN, G);
+                fx::u32 top = 0;
+                const fx::u32 eh = fx::scale_of(gd, top);
+                fx::Gradient q;
+                const double cv = fma(fx::to_double(fx::correction6_taped<true>(gd, eh, q), eh, top), 1.0 / 6.0, lf[2]);
+                if (fx::rough(gd)) weno_grad_of<true>(gd, G);
+                else fx::gradient_out(q, top, G);
 #pragma unroll
                 for (int m = 0; m < 5; ++m) sL[k * 5 + m][tid] = cb[k] * G[m];
                 // the back-projection's own sensitivities, linear in the field values: with

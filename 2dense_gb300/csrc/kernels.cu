@@ -173,13 +173,9 @@ __device__ __forceinline__ void recon_grad(const double lf[5], double g[5]) {
         return;
     }
     constexpr bool Z = REC == DENSE_RECON_WENOZ5;
-    double gd[4], d0, d1, d2, B[3];
+    double gd[4];
     first_differences(lf, gd);
-    betas_g(gd, d0, d1, d2, B);
-    WenoTerms t;
-    weno_terms<Z>(gd, d0, d1, d2, t);
-    const double iN = fx::rcp(t.N);
-    weno_grad<Z>(gd, B, d0, d1, d2, t, weno_num(t) * iN, iN, g);
+    weno_grad_of<Z>(gd, g);
 }
 
 // One reconstruction (the fast variant's WENO ones: weno_fixed.cuh).
@@ -591,23 +587,29 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
                 gp[m] = Gp[atk(t + m)];
                 gm[m] = Gm[atk(t + 4 - m)];
             }
-            h = fx::pair<Z>(sF[v * NCELL + atk(t + 2)], gp, sF[(4 + v) * NCELL + atk(t + 3)], gm);
-            if constexpr (TAPE) {
-                // the gradients of the two reconstructions (stencil slots 0 "+" and 5 "-")
-                auto tape_grad = [&](const double gd[4], int m0) {
-                    double d0, d1, d2, B[3], g[5];
-                    betas_g(gd, d0, d1, d2, B);
-                    WenoTerms tt;
-                    weno_terms<Z>(gd, d0, d1, d2, tt);
-                    const double iN = fx::rcp(tt.N);
-                    weno_grad<Z>(gd, B, d0, d1, d2, tt, weno_num(tt) * iN, iN, g);
+            const double lp = sF[v * NCELL + atk(t + 2)], lm = sF[(4 + v) * NCELL + atk(t + 3)];
+            if constexpr (!TAPE) {
+                h = fx::pair<Z>(lp, gp, lm, gm);
+            } else {
+                // pair's value, to the bit, and the gradients of the two reconstructions (stencil
+                // slots 0 "+" and 5 "-"; they are even in the differences)
+                fx::u32 top = 0;
+                const fx::u32 ep = fx::scale_of(gp, top), eh = fx::umax(ep, fx::scale_of(gm, top));
+                fx::i64 c = 0;
+#pragma unroll 1
+                for (int s = 0; s < 2; ++s) {
+                    double gd[4], g[5];
 #pragma unroll
-                    for (int m = 0; m < 5; ++m) tape_at[((m0 + m) * 4 + v) * ts] = g[m];
-                };
-                tape_grad(gp, 0);
+                    for (int m = 0; m < 4; ++m) gd[m] = s == 0 ? Gp[atk(t + m)] : Gm[atk(t + 4 - m)];
+                    fx::Gradient q;
+                    const fx::i64 cs = fx::correction6_taped<Z>(gd, eh, q);
+                    c += s == 0 ? cs : -cs;
+                    if (fx::rough(gd)) weno_grad_of<Z>(gd, g);
+                    else fx::gradient_out(q, top, g);
 #pragma unroll
-                for (int m = 0; m < 4; ++m) gm[m] = -gm[m];
-                tape_grad(gm, 5);
+                    for (int m = 0; m < 5; ++m) tape_at[((5 * s + m) * 4 + v) * ts] = g[m];
+                }
+                h = fx::about(lp, lm, fx::to_double(c, eh, top));
             }
         } else {
             double lp[5], lm[5];

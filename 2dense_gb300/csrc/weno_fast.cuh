@@ -134,6 +134,17 @@ __device__ __forceinline__ void weno_grad(const double gd[4], const double B[3],
     g[2] = 1.0 - ((g[0] + g[1]) + (g[3] + g[4]));
 }
 
+// The gradient from a stencil's first differences alone.
+template <bool Z>
+__device__ __forceinline__ void weno_grad_of(const double gd[4], double g[5]) {
+    double d0, d1, d2, B[3];
+    betas_g(gd, d0, d1, d2, B);
+    WenoTerms t;
+    weno_terms<Z>(gd, d0, d1, d2, t);
+    const double iN = fx::rcp(t.N);
+    weno_grad<Z>(gd, B, d0, d1, d2, t, weno_num(t) * iN, iN, g);
+}
+
 // The weights' share alone of a reconstruction's stencil gradient, for weights computed from one
 // stencil (lf, through gd, B, d_k and its weno_terms t, iN = 1/N) and applied to candidates of
 // other data: AdaWENO's smooth branch reconstructs every component with the WENO-Z weights of

@@ -71,3 +71,14 @@ def test_flux_change(lines):
 def test_conversion(lines):
     """Fixed point to double is a nearest rounding at every width, up to the next power of two too."""
     assert [x[1] for x in lines if x[0] == "conversion"] == ["0"]
+
+
+@pytest.mark.parametrize("kind", range(5))
+@pytest.mark.parametrize("z", [0, 1])
+def test_gradient(lines, kind, z):
+    """The taped gradient's rms error is that of weno_grad or less, up to a quarter more (its fixed-point
+    differences know a stencil's smoothest part to 2^-55 of the largest one's, kRough bits less than
+    FP64's 2^-53 of themselves); the value is the plain sweep's to the bit; the gradient is even."""
+    (row,) = [x[3:] for x in lines if x[0] == "gradient" and x[1:3] == [str(z), str(kind)]]
+    assert float(row[0]) <= 1.25 * float(row[1])
+    assert int(row[3]) == 0 and int(row[4]) == 0

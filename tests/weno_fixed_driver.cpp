@@ -256,6 +256,65 @@ void conversion() {
     printf("conversion %d\n", bad);
 }
 
+// the gradient dW/dlf[m] of the reconstruction, written out
+template <bool Z> void exact_gradient(const double f[5], ld G[5]) {
+    const ld ss = (double)1.0e-6f, cs[3] = {0.1L, 0.6L, 0.3L};
+    ld g[4], be[3], d[3], al[3], db[3], S = 0, W = 0, st = 0;
+    for (int m = 0; m < 4; ++m) g[m] = (ld)f[m] - f[m + 1];
+    const ld A[3] = {g[0] - g[1], g[1] - g[2], g[2] - g[3]}, B[3] = {g[0] - 3 * g[1], g[1] + g[2], 3 * g[2] - g[3]};
+    const ld q[3] = {(2 * g[0] - 5 * g[1]) / 6, (-g[1] - 2 * g[2]) / 6, (g[3] - 4 * g[2]) / 6};  // about lf2
+    for (int k = 0; k < 3; ++k) { be[k] = 13 * A[k] * A[k] / 12 + B[k] * B[k] / 4; d[k] = ss + be[k]; }
+    const ld tau = fabsl(be[2] - be[0]);
+    for (int k = 0; k < 3; ++k) { al[k] = Z ? cs[k] * (1 + tau * tau / (d[k] * d[k])) : cs[k] / (d[k] * d[k]); S += al[k]; }
+    for (int k = 0; k < 3; ++k) W += al[k] * q[k] / S;
+    for (int k = 0; k < 3; ++k) {
+        const ld e = (q[k] - W) / S;
+        db[k] = Z ? -2 * e * cs[k] * tau * tau / (d[k] * d[k] * d[k]) : -2 * e * al[k] / d[k];
+        if (Z) st += 2 * e * cs[k] * tau / (d[k] * d[k]);
+    }
+    if (be[2] >= be[0]) { db[2] += st; db[0] -= st; } else { db[2] -= st; db[0] += st; }
+    const ld a[3][5] = {{1 / 3.L, -7 / 6.L, 11 / 6.L, 0, 0}, {0, -1 / 6.L, 5 / 6.L, 1 / 3.L, 0}, {0, 0, 1 / 3.L, 5 / 6.L, -1 / 6.L}};
+    const ld dA[3][5] = {{1, -2, 1, 0, 0}, {0, 1, -2, 1, 0}, {0, 0, 1, -2, 1}};
+    const ld dB[3][5] = {{1, -4, 3, 0, 0}, {0, 1, 0, -1, 0}, {0, 0, 3, -4, 1}};
+    for (int m = 0; m < 5; ++m) {
+        G[m] = 0;
+        for (int k = 0; k < 3; ++k) G[m] += al[k] / S * a[k][m] + db[k] * (13 * A[k] * dA[k][m] / 6 + B[k] * dB[k][m] / 2);
+    }
+}
+// the taped reconstruction: its gradient (weno_grad's where the stencil is rough) and weno_grad's everywhere
+// against long double, its value against the plain one, and a change of sign of the differences
+template <bool Z> void gradient(int kind) {
+    std::mt19937_64 r(61 + kind);
+    double sum = 0, sum64 = 0, worst = 0;
+    int bits = 0, even = 0;
+    const int n = 50000;
+    for (int t = 0; t < n; ++t) {
+        const Stencils s = draw(r, kind);
+        ld G[5];
+        exact_gradient<Z>(s.fp, G);
+        double g[5], g64[5], ne[4], ge[5];
+        dense::fx::u32 top = 0;
+        const dense::fx::u32 eh = dense::fx::scale_of(s.gp, top);
+        dense::fx::Gradient q, qe;
+        bits += dense::fx::correction6_taped<Z>(s.gp, eh, q) != dense::fx::correction6<Z>(s.gp, eh);
+        for (int m = 0; m < 4; ++m) ne[m] = -s.gp[m];
+        dense::fx::correction6_taped<Z>(ne, eh, qe);
+        for (int m = 0; m < 5; ++m) even += qe.g[m] != q.g[m];
+        f64::weno_grad_of<Z>(s.gp, g64);
+        dense::fx::gradient_out(q, top, g);
+        dense::fx::gradient_out(q, dense::fx::kExpMax, ge);
+        even += !std::isnan(ge[t % 5]);
+        double e = 0, e64 = 0;
+        for (int m = 0; m < 5; ++m) {
+            if (dense::fx::rough(s.gp)) g[m] = g64[m];
+            e = std::max(e, (double)fabsl(g[m] - G[m]));
+            e64 = std::max(e64, (double)fabsl(g64[m] - G[m]));
+        }
+        sum += e * e; sum64 += e64 * e64; worst = std::max(worst, e);
+    }
+    printf("gradient %d %d %.17g %.17g %.17g %d %d\n", (int)Z, kind, std::sqrt(sum / n), std::sqrt(sum64 / n), worst, bits, even);
+}
+
 int main() {
     conversion();
     roots();
@@ -274,4 +333,5 @@ int main() {
     forms<false>();
     forms<true>();
     adaptive();
+    for (int k = 0; k < 5; ++k) { gradient<false>(k); gradient<true>(k); }
 }
