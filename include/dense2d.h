@@ -166,7 +166,7 @@ int dense_stage(dense_handle_t* h, int irk, double current_time, double* dt_inou
    stages, each taken only while (*t_inout < t_end && *step_inout < total_step), advancing
    time and step on the device; no host synchronisation between steps. On return *t_inout,
    *step_inout and *dt_out hold the driver's current_time, current_step and dt. One CUDA graph
-   runs a step; for AdaWENO (105) grids of 200,000 cells or more its kernel-to-kernel edges are
+   runs a step; but for AdaWENO (105) grids of 80,000 cells or more its kernel-to-kernel edges are
    programmatic (each kernel scheduled as the one before it drains), which the environment
    variable DENSE_PDL=0 or 1 turns off or on for every grid. Results are the same either way. */
 int dense_steps(dense_handle_t* h, int nsteps, double t_end, int total_step,
