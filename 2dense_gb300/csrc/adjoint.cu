@@ -65,6 +65,7 @@ struct AdjParams {
     int gnp;          // planes per direction of what the cell kernel gathers: the tape (np), or
                       // the characteristic scheme's face sensitivities of the split fluxes (40)
     double gamma, dx, dy, inv_dx, inv_dy, cfl;
+    double g1, kg;    // gamma - 1, gamma/(gamma-1)
     int rule[4];      // ghost rule of each side (bottom, top, left, right): kRulePeriodic, ...
     // Rayleigh-Taylor's body force: each stage adds f_s (0, 0, rho, rho v) of its input, f_s =
     // dt, dt/4, (2/3 in single precision) dt (time_advance_general.f90:79,160,242); the
@@ -738,24 +739,25 @@ __device__ __forceinline__ void fetch_cell(const AdjParams& a, const double* __r
 
 // Per face of direction DIR, two threads (adjacent lanes, one per sign): the characteristic
 // reconstruction recomputed from the stage input u -- the GLF split fluxes of the stencil cells
-// (the stage's global lambda), the Roe average of the face's two cells and its eigenvectors
-// (roe_eig_fast's formulas), the sign's five split fluxes projected on the characteristic
-// fields and WENO-Z per field with its stencil gradient (weno_grad) -- and its reverse for the
-// face's hbar: the back-projection's transpose gives each field's value sensitivity, times the
-// field's stencil gradient the sensitivities of the projected values, the transposed
-// projection those of the split fluxes, written per (sign, stencil point, component) as the
-// cell kernel's gather reads them (kRecFaceSens); and the eigenvectors'
-// sensitivities -- from the projections (sum over the stencil of the projected-value
-// sensitivities times the split fluxes) and the back-projection, the two signs' shares summed
-// across the lane pair -- sent through the eigenvectors' formulas and the Roe average to the
-// primitives (rho, u, v, p) of the face's two cells (rbar: the "+" lane writes the left cell's,
-// the "-" lane the right cell's).
+// (the stage's global lambda), the Roe average of the face's two cells (roe_eig_fast's formulas),
+// the sign's split-flux differences projected on the characteristic fields (project_fast's
+// factored form) and each field's WENO-Z correction c_k with its stencil gradient -- and its
+// reverse for the face's hbar. As in the sweep, h = F(centre) + sum_k r_k c_k: the
+// back-projection's transpose gives each correction's sensitivity, times the field's gradient (less
+// one at the centre) the sensitivities of the projected values, the transposed projection those
+// of the split fluxes, written per (sign, stencil point, component) as the cell kernel's gather
+// reads them (kRecFaceSens); and the sensitivities of the Roe quantities (u_n, u_t, |u|^2/2,
+// 1/(2 a), 1/(2 hh) in the projection, and those of the back-projection; the two signs' shares
+// summed across the lane pair) go through the Roe average to the primitives (rho, u, v, p) of
+// the face's two cells (rbar: the "+" lane writes the left cell's, the "-" lane the right cell's).
 // A block of 32 x 4 threads takes 16 faces x 4 lines (xi) or 16 lines x 4 faces (eta); its
 // cells' split fluxes and primitives are staged once in shared memory (each cell's get_primary
-// and split computed once, not once per reading face), and each thread parks its projected-value
-// sensitivities there too, which keeps the field loop's live registers down.
+// and split computed once, not once per reading face), and each thread parks its fields'
+// differences, then their gradients there too: the field loop is not unrolled, so that its one
+// copy of the integer gradient stays in the instruction cache. The transposed Jacobian of the 128 x
+// 512 Rayleigh-Taylor case, where both directions' face kernels took 0.43 of 0.75 ms, takes 0.58 ms.
 template <int DIR>
-__global__ void __launch_bounds__(128, 3) k_char_face(AdjParams a, const double* __restrict__ u,
+__global__ void __launch_bounds__(128, 4) k_char_face(AdjParams a, const double* __restrict__ u,
                                                   const double* __restrict__ hb, const double* __restrict__ lamv,
                                                   const double* __restrict__ tp, const double* __restrict__ flags,
                                                   double* __restrict__ fbar) {
@@ -763,7 +765,8 @@ __global__ void __launch_bounds__(128, 3) k_char_face(AdjParams a, const double*
     constexpr int NB = DIR == 0 ? 4 : 16;  // lines of a block
     constexpr int NA = FA + 5;             // cells staged along a line: f0-3 .. f0+FA+1
     __shared__ double sC[12][NB][NA];      // F+ (0..3), F- (4..7), rho, u, v, p (8..11)
-    __shared__ double sL[20][128];         // per thread: cb[k] g_k[m] of its sign, row k*5+m
+    __shared__ double sL[24][128];         // per thread: field k's differences, then gradient, row k*5+m;
+                                           // its correction's sensitivity, then the correction, row 20+k
     const int ni = a.ni, nj = a.nj;
     const int n = DIR == 0 ? ni : nj, nline = DIR == 0 ? nj : ni;
     const int tid = threadIdx.x + 32 * threadIdx.y;
@@ -794,7 +797,7 @@ __global__ void __launch_bounds__(128, 3) k_char_face(AdjParams a, const double*
     const bool valid = f <= n && line < nline;  // the same for both lanes of a face
     const long long ts = DIR == 0 ? a.xs : a.ys;
     const long long to = DIR == 0 ? (long long)line * (ni + 1) + f : (long long)f * ni + line;
-    const double g1 = a.gamma - 1.0, kg = a.gamma / g1;
+    const double g1 = a.g1, kg = a.kg;
     // AdaWENO (flags): the branches the forward took at this face, bit 0 "+" smooth, bit 1 "-"
     int fbits = 0;
     if (flags && valid) fbits = (int)flags[(DIR == 0 ? 0 : 5 * a.xs) + to];
@@ -804,91 +807,109 @@ __global__ void __launch_bounds__(128, 3) k_char_face(AdjParams a, const double*
     auto am = [&](int m) { return fa + (sg ? 5 - m : m); };
     auto F = [&](int m, int cc) { return sC[sg * 4 + cc][bi][am(m)]; };
     // the eigen quantities' sensitivities (this lane's sign; summed across the pair below)
-    double un0b = 0, ut0b = 0, a0b = 0, h0b = 0, uu0b = 0, a0un0b = 0;
-    double A0[4] = {0, 0, 0, 0}, A1[4] = {0, 0, 0, 0}, A3[4] = {0, 0, 0, 0}, A20 = 0;  // A[k][cc]
+    double un0b = 0, ut0b = 0, a0b = 0, h0b = 0, uu0b = 0, ihb = 0, ia5b = 0;
     // the Roe average's inputs of this lane's cell (the "+" lane the left cell, the "-" lane the
     // right), exchanged across the pair: sqrt(rho) and the total enthalpy
     const int ac = fa + 2 + sg;
     const double rs = valid ? sC[8][bi][ac] : 1.0, us = valid ? sC[9][bi][ac] : 0.0;
     const double vs = valid ? sC[10][bi][ac] : 0.0, ps = valid ? sC[11][bi][ac] : 1.0;
-    const double irs = 1.0 / rs, ss = sqrt(rs), hs = fma(kg * ps, irs, 0.5 * (us * us + vs * vs));
+    const double irs = fx::rcp(rs), ss = fx::sqrt_normal(rs), hs = fma(kg * ps, irs, 0.5 * (us * us + vs * vs));
     const double ss_o = __shfl_xor_sync(0xffffffffu, ss, 1), hs_o = __shfl_xor_sync(0xffffffffu, hs, 1);
     const double us_o = __shfl_xor_sync(0xffffffffu, us, 1), vs_o = __shfl_xor_sync(0xffffffffu, vs, 1);
     const double sl = sg ? ss_o : ss, sr = sg ? ss : ss_o, hl = sg ? hs_o : hs, hr = sg ? hs : hs_o;
     const double ul = sg ? us_o : us, ur = sg ? us : us_o, vl = sg ? vs_o : vs, vr = sg ? vs : vs_o;
     double r = 0.5, u0 = 0, v0 = 0, h0 = 0, uu0 = 0, c2 = 1, ia = 1, a0 = 1;
-    double ihh = 0, un0 = 0, ut0 = 0;
+    double un0 = 0, ut0 = 0;
     if (valid) {
         double* const FB = fbar + (DIR == 0 ? 0 : a.gnp * a.xs) + to;
         double HB[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) HB[v] = hb[(DIR == 0 ? 0 : 4 * a.xs) + v * ts + to];
         if (any_char) {  // a face whose signs are both smooth never forms its Roe average
-            r = 1.0 / (sl + sr);
-            u0 = (sr * ur + sl * ul) * r; v0 = (sr * vr + sl * vl) * r; h0 = (sr * hr + sl * hl) * r;
-            uu0 = 0.5 * (u0 * u0 + v0 * v0);
+            r = fx::rcp(sl + sr);
+            const double wr = sr * r;
+            u0 = fma(wr, ur - ul, ul); v0 = fma(wr, vr - vl, vl); h0 = fma(wr, hr - hl, hl);
+            uu0 = 0.5 * fma(u0, u0, v0 * v0);
             c2 = g1 * (h0 - uu0);
-            ia = 1.0 / sqrt(c2); a0 = c2 * ia; ihh = g1 * ia * ia;
+            ia = fx::rsqrt(c2); a0 = c2 * ia;
             un0 = DIR == 0 ? u0 : v0; ut0 = DIR == 0 ? v0 : u0;
         }
         if (!smooth) {
-            const double a0un0 = a0 * un0;
-            const double hu = 0.5 * uu0 * ihh, nu = 0.5 * un0 * ia, ia5 = 0.5 * ia;
-            const double pn = 0.5 * un0 * ihh, pt = 0.5 * ut0 * ihh, ih = 0.5 * ihh;
-            const double ln0 = -pn - ia5, ln3 = -pn + ia5;
-            // M[cc][k]: the coefficient of split-flux component cc in characteristic field k
-            double M[4][4];
-            M[0][0] = hu + nu; M[3][0] = ih;
-            M[0][3] = hu - nu; M[3][3] = ih;
-            if (DIR == 0) { M[1][0] = ln0; M[2][0] = -pt; M[1][3] = ln3; M[2][3] = -pt; }
-            else          { M[1][0] = -pt; M[2][0] = ln0; M[1][3] = -pt; M[2][3] = ln3; }
-            M[0][1] = 1.0 - uu0 * ihh; M[1][1] = u0 * ihh; M[2][1] = v0 * ihh; M[3][1] = -ihh;
-            M[0][2] = -ut0; M[1][2] = DIR == 1 ? 1.0 : 0.0; M[2][2] = DIR == 0 ? 1.0 : 0.0; M[3][2] = 0.0;
-            const double hn = HB[1 + DIR], ht = HB[2 - DIR];
-            // the back-projection's transpose: each field value's sensitivity
-            const double sb = HB[0] + un0 * hn + ut0 * ht, db = a0 * hn + a0un0 * HB[3];
-            const double cb[4] = {sb - db + h0 * HB[3], sb + uu0 * HB[3], ht + ut0 * HB[3], sb + db + h0 * HB[3]};
+            const double ia5 = 0.5 * ia, ih = g1 * ia * ia5, ihh = 2.0 * ih;
+            const double hn = HB[1 + DIR], ht = HB[2 - DIR], h3 = HB[3];
+            // the differences' fields: w = f_n - u_n f_0, q = f_t - u_t f_0, z = f_3 - uu f_0 - u_n w -
+            // u_t q; l_0,3 = ih z -+ ia5 w, l_1 = f_0 - ihh z, l_2 = q
 #pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                double f[4];
+#pragma unroll
+                for (int cc = 0; cc < 4; ++cc) f[cc] = F(m, cc) - F(m + 1, cc);
+                const double wn = fma(-un0, f[0], f[1 + DIR]), qt = fma(-ut0, f[0], f[2 - DIR]);
+                const double z = fma(-ut0, qt, fma(-un0, wn, fma(-uu0, f[0], f[3]))), mm = ia5 * wn;
+                sL[m][tid] = fma(ih, z, -mm);
+                sL[5 + m][tid] = fma(-ihh, z, f[0]);
+                sL[10 + m][tid] = qt;
+                sL[15 + m][tid] = fma(ih, z, mm);
+            }
+            // the back-projection's transpose: each correction's sensitivity
+            {
+                const double sb = fma(ut0, ht, fma(un0, hn, HB[0])), db = a0 * fma(un0, h3, hn);
+                sL[20][tid] = fma(h0, h3, sb - db);
+                sL[21][tid] = fma(uu0, h3, sb);
+                sL[22][tid] = fma(ut0, h3, ht);
+                sL[23][tid] = fma(h0, h3, sb + db);
+            }
+#pragma unroll 1
             for (int k = 0; k < 4; ++k) {
-                double lf[5];
-#pragma unroll
-                for (int m = 0; m < 5; ++m)
-                    lf[m] = fma(M[0][k], F(m, 0), fma(M[1][k], F(m, 1), fma(M[2][k], F(m, 2), M[3][k] * F(m, 3))));
-                // the field's value and gradient on the integer pipes, as the taping sweeps take them
+                // the field's correction and gradient on the integer pipes
                 double gd[4], G[5];
-                first_differences(lf, gd);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) gd[m] = sL[k * 5 + m][tid];
                 fx::u32 top = 0;
                 const fx::u32 eh = fx::scale_of(gd, top);
                 fx::Gradient q;
-                const double cv = fma(fx::to_double(fx::correction6_taped<true>(gd, eh, q), eh, top), 1.0 / 6.0, lf[2]);
+                const double cv = fx::to_double(fx::correction6_taped<true>(gd, eh, q), eh, top) * (1.0 / 6.0);
                 if (fx::rough(gd)) weno_grad_of<true>(gd, G);
                 else fx::gradient_out(q, top, G);
+                const double cb = sL[20 + k][tid];
+                sL[20 + k][tid] = cv;
 #pragma unroll
-                for (int m = 0; m < 5; ++m) sL[k * 5 + m][tid] = cb[k] * G[m];
-                // the back-projection's own sensitivities, linear in the field values: with
-                // s = cv0 + cv1 + cv3 and d = cv3 - cv0, un0 takes s hn, a0 d hn, ut0 s ht + cv2 h3,
-                // h0 (cv0 + cv3) h3, a0 un0 d h3, uu0 cv1 h3
-                if (k != 2) { un0b = fma(cv, hn, un0b); ut0b = fma(cv, ht, ut0b); }
-                if (k == 0) { a0b = fma(-cv, hn, a0b); h0b = fma(cv, HB[3], h0b); a0un0b = fma(-cv, HB[3], a0un0b); }
-                if (k == 3) { a0b = fma(cv, hn, a0b); h0b = fma(cv, HB[3], h0b); a0un0b = fma(cv, HB[3], a0un0b); }
-                if (k == 1) uu0b = fma(cv, HB[3], uu0b);
-                if (k == 2) ut0b = fma(cv, HB[3], ut0b);
+                for (int m = 0; m < 5; ++m) sL[k * 5 + m][tid] = cb * (m == 2 ? G[2] - 1.0 : G[m]);
             }
-            // the split fluxes' sensitivities (the transposed projection) and the projection
-            // coefficients' (sum over the stencil of the projected values' times the split fluxes)
+            {
+                // the back-projection's own sensitivities: with s = c0 + c1 + c3 and d = c3 - c0,
+                // h_0 = s, h_n = u_n s + a d, h_t = u_t s + c2, h_3 = H (c0 + c3) + a u_n d + uu c1 + u_t c2
+                const double c0 = sL[20][tid], c1 = sL[21][tid], c2_ = sL[22][tid], c3 = sL[23][tid];
+                const double s03 = c0 + c3, d = c3 - c0, s = s03 + c1;
+                un0b = fma(s, hn, a0 * d * h3);
+                ut0b = fma(s, ht, c2_ * h3);
+                a0b = d * fma(un0, h3, hn);
+                h0b = s03 * h3;
+                uu0b = c1 * h3;
+            }
+            // the split fluxes' sensitivities (the transposed projection; the centre takes hbar itself)
+            // and the projection's own, summed over the stencil
 #pragma unroll
             for (int m = 0; m < 5; ++m) {
                 const double l0_ = sL[m][tid], l1_ = sL[5 + m][tid], l2_ = sL[10 + m][tid], l3_ = sL[15 + m][tid];
+                const double f0_ = F(m, 0), wn = fma(-un0, f0_, F(m, 1 + DIR)), qt = fma(-ut0, f0_, F(m, 2 - DIR));
+                const double z = fma(-ut0, qt, fma(-un0, wn, fma(-uu0, f0_, F(m, 3))));
+                const double sb = l0_ + l3_, mb = l3_ - l0_;
+                ihb = fma(fma(-2.0, l1_, sb), z, ihb);
+                ia5b = fma(mb, wn, ia5b);
+                const double zb = fma(ih, sb, -ihh * l1_);
+                const double wb = fma(ia5, mb, -un0 * zb), qb = fma(-ut0, zb, l2_);
+                un0b = fma(-zb, wn, fma(-wb, f0_, un0b));
+                ut0b = fma(-zb, qt, fma(-qb, f0_, ut0b));
+                uu0b = fma(-zb, f0_, uu0b);
+                double fb[4];
+                fb[0] = fma(-ut0, qb, fma(-un0, wb, fma(-uu0, zb, l1_)));
+                fb[1 + DIR] = wb;
+                fb[2 - DIR] = qb;
+                fb[3] = zb;
 #pragma unroll
-                for (int cc = 0; cc < 4; ++cc) {
-                    const double Fm = F(m, cc);
-                    FB[(long long)((sg * 5 + m) * 4 + cc) * ts] =
-                        fma(M[cc][0], l0_, fma(M[cc][1], l1_, fma(M[cc][2], l2_, M[cc][3] * l3_)));
-                    A0[cc] = fma(l0_, Fm, A0[cc]);
-                    A1[cc] = fma(l1_, Fm, A1[cc]);
-                    A3[cc] = fma(l3_, Fm, A3[cc]);
-                    if (cc == 0) A20 = fma(l2_, Fm, A20);
-                }
+                for (int cc = 0; cc < 4; ++cc)
+                    FB[(long long)((sg * 5 + m) * 4 + cc) * ts] = m == 2 ? fb[cc] + HB[cc] : fb[cc];
                 if (flags) FB[(long long)(40 + sg * 5 + m) * ts] = 0.0;  // no density share
             }
         } else {
@@ -932,10 +953,7 @@ __global__ void __launch_bounds__(128, 3) k_char_face(AdjParams a, const double*
     }
     // the two signs' shares (both lanes of a pair are valid or neither; every lane shuffles)
     auto pair_sum = [](double& v) { v += __shfl_xor_sync(0xffffffffu, v, 1); };
-    pair_sum(un0b); pair_sum(ut0b); pair_sum(a0b); pair_sum(h0b); pair_sum(uu0b); pair_sum(a0un0b);
-#pragma unroll
-    for (int cc = 0; cc < 4; ++cc) { pair_sum(A0[cc]); pair_sum(A1[cc]); pair_sum(A3[cc]); }
-    pair_sum(A20);
+    pair_sum(un0b); pair_sum(ut0b); pair_sum(a0b); pair_sum(h0b); pair_sum(uu0b); pair_sum(ihb); pair_sum(ia5b);
     if (!valid) return;
     double* const RB = a.rbar + (DIR == 0 ? 0 : 8 * a.xs) + to + (long long)(4 * sg) * ts;
     if (!any_char) {  // no Roe average at this face
@@ -943,32 +961,10 @@ __global__ void __launch_bounds__(128, 3) k_char_face(AdjParams a, const double*
         for (int v = 0; v < 4; ++v) RB[v * ts] = 0.0;
         return;
     }
-    // the eigenvector entries' sensitivities back to the Roe quantities
-    const double l00b = A0[0], l03b = A3[0];
-    const double l10b = A0[1], l13b = A3[1], l20b = A0[2], l23b = A3[2];
-    const double l30b = A0[3] + A3[3];
-    const double l01b = A1[0], l11b = A1[1], l21b = A1[2], l31b = A1[3];
-    ut0b -= A20;
-    const double hub = l00b + l03b, nub = l00b - l03b;
-    const double nrm0 = DIR == 0 ? l10b : l20b, nrm3 = DIR == 0 ? l13b : l23b;  // the ln0, ln3 entries
-    const double tg0 = DIR == 0 ? l20b : l10b, tg3 = DIR == 0 ? l23b : l13b;    // the -pt entries
-    const double pnb = -nrm0 - nrm3, ia5b = -nrm0 + nrm3, ptb = -tg0 - tg3, ihb = l30b;
-    double ihhb = 0.0, iab = 0.0, u0b = 0.0, v0b = 0.0;
-    uu0b += -ihh * l01b + 0.5 * ihh * hub;
-    ihhb += -uu0 * l01b + u0 * l11b + v0 * l21b - l31b + 0.5 * uu0 * hub + 0.5 * un0 * pnb + 0.5 * ut0 * ptb +
-            0.5 * ihb;
-    u0b += ihh * l11b;
-    v0b += ihh * l21b;
-    un0b += 0.5 * ia * nub + 0.5 * ihh * pnb + a0 * a0un0b;
-    ut0b += 0.5 * ihh * ptb;
-    iab += 0.5 * un0 * nub + 0.5 * ia5b;
-    a0b += un0 * a0un0b;
-    if (DIR == 0) { u0b += un0b; v0b += ut0b; }
-    else          { v0b += un0b; u0b += ut0b; }
-    iab += 2.0 * g1 * ia * ihhb;  // ihh = g1 ia^2
-    double c2b = ia * a0b;        // a0 = c2 ia
-    iab += c2 * a0b;
-    c2b += -0.5 * ia * ia * ia * iab;  // ia = c2^-1/2
+    // the Roe quantities' sensitivities: ih = (gamma-1)/2 ia^2, ia5 = ia/2, a = c2 ia, ia = c2^-1/2
+    const double iab = fma(g1 * ia, ihb, fma(0.5, ia5b, c2 * a0b));
+    const double c2b = fma(-0.5 * ia * ia * ia, iab, ia * a0b);
+    double u0b = DIR == 0 ? un0b : ut0b, v0b = DIR == 0 ? ut0b : un0b;
     h0b += g1 * c2b;
     uu0b += -g1 * c2b;
     u0b += u0 * uu0b;
@@ -1724,7 +1720,7 @@ int dense_adjoint_create(const dense_config_t* cfg, int checkpoint_every, dense_
     p.gnp = adapt ? 50 : charac ? 40 : p.np;
     p.charac = charac ? 1 : 0;
     p.adapt = adapt ? 1 : 0;
-    p.gamma = cfg->gamma; p.dx = cfg->dx; p.dy = cfg->dy; p.inv_dx = 1.0 / cfg->dx; p.inv_dy = 1.0 / cfg->dy;
+    p.gamma = cfg->gamma; p.g1 = cfg->gamma - 1.0; p.kg = cfg->gamma / (cfg->gamma - 1.0); p.dx = cfg->dx; p.dy = cfg->dy; p.inv_dx = 1.0 / cfg->dx; p.inv_dy = 1.0 / cfg->dy;
     p.cfl = cfg->cfl;
     for (int k = 0; k < 4; ++k) p.rule[k] = rules[k];
     // the forward solver applies the body force on the same condition (fill_params)

@@ -1752,19 +1752,20 @@ static void cw_launch(dim3 g, const Params& p, int irk, cudaStream_t s) {
 // interface (one per component: four times the warps to hide the dependent FP64 chains of a
 // sweep that is only one wave deep); same arithmetic per interface, so the results do not
 // depend on the tile. Measured on the 200 x 200 vortex: 1.925e8 -> 1.976e8 cell-updates/s for
-// the four threads; on 512 x 512 and larger grids the standard tiles gain nothing from them.
-// The adjoint's taping sweeps keep one thread per interface (no gain measured).
-constexpr int cw_small_tz(bool tape) { return tape ? 1 : 4; }
+// the four threads; on 512 x 512 and larger grids the standard tiles gain nothing from them. The
+// adjoint's taping sweeps likewise: a 122 x 175 WENO-Z adjoint 1607 -> 1387 us, 256 x 256 WENO-JS
+// 7.26 -> 7.05 ms (two threads: 1450 us and 6.94 ms).
+constexpr int kSmallTZ = 4;
 template <int SPL, int REC, bool TAPE = false>
 static void launch_cw(const Params& p, int irk, int dir, cudaStream_t s) {
     const unsigned few = 4u * sm_count();
     if (dir == 0) {
         const dim3 g = grid_xi(p, kXTX, kXTY);
-        if (g.x * g.y < few) cw_launch<0, SPL, REC, kXTX, kXSTY, TAPE, cw_small_tz(TAPE)>(grid_xi(p, kXTX, kXSTY), p, irk, s);
+        if (g.x * g.y < few) cw_launch<0, SPL, REC, kXTX, kXSTY, TAPE, kSmallTZ>(grid_xi(p, kXTX, kXSTY), p, irk, s);
         else                 cw_launch<0, SPL, REC, kXTX, kXTY, TAPE>(g, p, irk, s);
     } else {
         const dim3 g = grid_eta(p, kETX, kETY);
-        if (g.x * g.y < few) cw_launch<1, SPL, REC, kETX, kESTY, TAPE, cw_small_tz(TAPE)>(grid_eta(p, kETX, kESTY), p, irk, s);
+        if (g.x * g.y < few) cw_launch<1, SPL, REC, kETX, kESTY, TAPE, kSmallTZ>(grid_eta(p, kETX, kESTY), p, irk, s);
         else                 cw_launch<1, SPL, REC, kETX, kETY, TAPE>(g, p, irk, s);
     }
 }
@@ -2005,14 +2006,14 @@ static void allow_smem(K kernel, size_t bytes) {
 template <int SPL, int REC>
 static void allow_cw_smem() {
     allow_smem(k_flux_cw<0, SPL, REC, kXTX, kXTY>, CwTile<0, REC, kXTX, kXTY>::bytes);
-    allow_smem(k_flux_cw<0, SPL, REC, kXTX, kXSTY, false, cw_small_tz(false)>, CwTile<0, REC, kXTX, kXSTY>::bytes);
+    allow_smem(k_flux_cw<0, SPL, REC, kXTX, kXSTY, false, kSmallTZ>, CwTile<0, REC, kXTX, kXSTY>::bytes);
     allow_smem(k_flux_cw<1, SPL, REC, kETX, kETY>, CwTile<1, REC, kETX, kETY>::bytes);
-    allow_smem(k_flux_cw<1, SPL, REC, kETX, kESTY, false, cw_small_tz(false)>, CwTile<1, REC, kETX, kESTY>::bytes);
+    allow_smem(k_flux_cw<1, SPL, REC, kETX, kESTY, false, kSmallTZ>, CwTile<1, REC, kETX, kESTY>::bytes);
     // the adjoint's taping sweeps
     allow_smem(k_flux_cw<0, SPL, REC, kXTX, kXTY, true>, CwTile<0, REC, kXTX, kXTY>::bytes);
-    allow_smem(k_flux_cw<0, SPL, REC, kXTX, kXSTY, true, cw_small_tz(true)>, CwTile<0, REC, kXTX, kXSTY>::bytes);
+    allow_smem(k_flux_cw<0, SPL, REC, kXTX, kXSTY, true, kSmallTZ>, CwTile<0, REC, kXTX, kXSTY>::bytes);
     allow_smem(k_flux_cw<1, SPL, REC, kETX, kETY, true>, CwTile<1, REC, kETX, kETY>::bytes);
-    allow_smem(k_flux_cw<1, SPL, REC, kETX, kESTY, true, cw_small_tz(true)>, CwTile<1, REC, kETX, kESTY>::bytes);
+    allow_smem(k_flux_cw<1, SPL, REC, kETX, kESTY, true, kSmallTZ>, CwTile<1, REC, kETX, kESTY>::bytes);
     // the batched tile variants of batch_cw_variant
     allow_smem(kb_flux_cw<0, SPL, REC, 32, 4>, CwTile<0, REC, 32, 4>::bytes);
     allow_smem(kb_flux_cw<0, SPL, REC, 64, 2>, CwTile<0, REC, 64, 2>::bytes);
