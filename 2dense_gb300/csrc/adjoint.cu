@@ -91,6 +91,7 @@ struct AdjParams {
     const double* yleft;
     double* tpart;
     double* tacc;
+    double* wall;     // k_wall's shares (wall_at), where a side has a wall rule
 };
 // Ghost rules of the benchmarks the adjoint covers (boundary_*_general.f90): a periodic copy,
 // the recursive 4/3, -1/3 extrapolation of the two cells next to the side, the mirror of the
@@ -298,10 +299,11 @@ __device__ __forceinline__ void sw_prim_bar(const double pv[4], double gamma, co
     }
 }
 
-// Ub += (dF+/dU)^T gp + (dF-/dU)^T gm of the Steger-Warming split in both directions at one cell
-// (g[d] the sensitivities of direction d's F+ then F-): one forward pass per conserved variable.
-__device__ __forceinline__ void sw_vjp(const double U[4], double gamma, const double gpx[4], const double gmx[4],
-                                       const double gpy[4], const double gmy[4], double Ub[4]) {
+// Ub += (dF+/dU)^T gp + (dF-/dU)^T gm of the Steger-Warming split in one direction at one cell: one
+// forward pass per conserved variable.
+template <int DIR>
+__device__ __forceinline__ void sw_vjp(const double U[4], double gamma, const double gp[4], const double gm[4],
+                                       double Ub[4]) {
 #pragma unroll 1
     for (int k = 0; k < 4; ++k) {
         Dual Ud[4];
@@ -309,12 +311,9 @@ __device__ __forceinline__ void sw_vjp(const double U[4], double gamma, const do
         for (int c = 0; c < 4; ++c) Ud[c] = Dual{U[c], c == k ? 1.0 : 0.0};
         Dual fp[4], fm[4];
         double acc = 0.0;
-        sw_split_dual<0>(Ud, gamma, fp, fm);
+        sw_split_dual<DIR>(Ud, gamma, fp, fm);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc = fma(gpx[c], fp[c].d, fma(gmx[c], fm[c].d, acc));
-        sw_split_dual<1>(Ud, gamma, fp, fm);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc = fma(gpy[c], fp[c].d, fma(gmy[c], fm[c].d, acc));
+        for (int c = 0; c < 4; ++c) acc = fma(gp[c], fp[c].d, fma(gm[c], fm[c].d, acc));
         Ub[k] += acc;
     }
 }
@@ -341,11 +340,11 @@ __device__ __forceinline__ void block_argmax(double& e1, long long& i1, double& 
     }
     __shared__ double se[2][32];
     __shared__ long long si[2][32];
-    const int tid = threadIdx.x + threadIdx.y * blockDim.x;
+    const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
     if ((tid & 31) == 0) { se[0][tid >> 5] = e1; se[1][tid >> 5] = e2; si[0][tid >> 5] = i1; si[1][tid >> 5] = i2; }
     __syncthreads();
     if (tid == 0) {
-        const int nw = (blockDim.x * blockDim.y + 31) / 32;
+        const int nw = (blockDim.x * blockDim.y * blockDim.z + 31) / 32;
         for (int k = 1; k < nw; ++k) {
             if (argmax_better(se[0][k], si[0][k], e1, i1)) { e1 = se[0][k]; i1 = si[0][k]; }
             if (argmax_better(se[1][k], si[1][k], e2, i2)) { e2 = se[1][k]; i2 = si[1][k]; }
@@ -361,8 +360,8 @@ __device__ __forceinline__ void block_sum2(double& x, double& y) {
         y += __shfl_xor_sync(0xffffffffu, y, o);
     }
     __shared__ double red2[2][32];
-    const int tid = threadIdx.x + threadIdx.y * blockDim.x;
-    const int nw = (blockDim.x * blockDim.y + 31) / 32;
+    const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+    const int nw = (blockDim.x * blockDim.y * blockDim.z + 31) / 32;
     if ((tid & 31) == 0) { red2[0][tid >> 5] = x; red2[1][tid >> 5] = y; }
     __syncthreads();
     if (tid == 0) {
@@ -488,13 +487,12 @@ __device__ __forceinline__ double gather_rho_line(const double* __restrict__ T, 
     return acc;
 }
 
-// The ghost cells of a side with a wall rule that the interior cell (i, j) feeds, in direction
-// DIR (0: the left and right sides of row j, 1: the bottom and top of column i): for each such
-// ghost, its state rebuilt from the interior state by the rule, the sensitivities of its F+ and
+// The ghost cells of a side with a wall rule that an interior cell feeds, in direction DIR (0: the
+// left and right sides of a row, 1: the bottom and top of a column): for each such ghost, its state rebuilt from the interior state by the rule, the sensitivities of its F+ and
 // F- gathered from the faces whose stencils read it, the split's sensitivities in terms of the
 // ghost's U and primitives (a ghost's primitives come from the rule, not from its U), and these
 // sent back through the rule: into Ub directly, into pbar (rho, u, v, p, alpha of the cell) for
-// the caller to pull back through get_primary. A mirror ghost k copies the cell k+1 in from the
+// the cell's thread to pull back through get_primary. A mirror ghost k copies the cell k+1 in from the
 // side (normal velocity negated); an extrapolated ghost k is w1_k c1 + w2_k c2 of the two cells
 // next to the side (the recursion g = 4/3 near - 1/3 far unrolled), so both of those cells
 // rebuild all four ghosts and take their shares. GLF: a ghost's lambda sensitivity goes to the
@@ -544,148 +542,181 @@ __device__ __forceinline__ void fixed_state(const AdjParams& a, int dir, int sid
     if (qg) { qg[0] = rho; qg[1] = u; qg[2] = v; qg[3] = pr; qg[4] = sqrt(a.gamma * pr / rho); }
 }
 
+// One ghost's share for one interior cell it is built from. Per side and line there are kWallSlots
+// such pairs: an extrapolated side's cells 1 and 2 (distance from the side) with its four ghosts,
+// slot (dist - 1) 4 + k; a mirror's cells 1..4 with ghost dist - 1, slot dist - 1; a fixed
+// state's four ghosts with the cell next to the side, slot k. k_wall takes a thread for each
+// and parks its shares -- Ub (4), pbar (5), lambda's, the start time's -- in a.wall, where k_rev's
+// thread of the cell adds them in order: as a loop over the ghosts in k_rev they set the time of the
+// whole kernel on small grids and its registers on all (254 instead of 128: WALL_FIGURES).
+constexpr int kWallSlots = 8, kWallTerms = 11;
+__device__ __forceinline__ long long wall_at(const AdjParams& a, int dir, int side, int slot, int term, int line) {
+    const long long pitch = a.ni > a.nj ? a.ni : a.nj;
+    return ((long long)((dir * 2 + side) * kWallSlots + slot) * kWallTerms + term) * pitch + line;
+}
+// the rule of a side at a line (the double Mach reflection's bottom resolved)
+__device__ __forceinline__ int rule_at(const AdjParams& a, int dir, int side, int line) {
+    const int rule = a.rule[dir == 0 ? 2 + side : side];
+    if (rule == kRuleDMRBottom) return ((double)(line + 1) - 0.5) * a.dx >= 1.0 / 6.0 ? kRuleReflect : kRuleFixed;
+    return rule;
+}
 template <int DIR, int SPL, int REC>
-__device__ __forceinline__ void wall_terms(const AdjParams& a, const double* __restrict__ u,
-                                           const double* __restrict__ tape, const double* __restrict__ hb, int i,
-                                           int j, const Prim& q, const double U[4], double lam_g, double t,
-                                           double Ub[4], double pbar[5], double& lb, double& tl) {
-    const int n = DIR == 0 ? a.ni : a.nj, x = DIR == 0 ? i : j;
+__device__ __forceinline__ void wall_ghost(const AdjParams& a, const double* __restrict__ u,
+                                           const double* __restrict__ T, const double* __restrict__ H, int side,
+                                           int slot, int line, double lam_g, double t) {
+    const int rule = rule_at(a, DIR, side, line);
+    if (rule == kRulePeriodic || (slot >= 4 && rule != kRuleExtrap)) return;
+    const int n = DIR == 0 ? a.ni : a.nj;
     const long long ts = DIR == 0 ? a.xs : a.ys;
-    const double* T = DIR == 0 ? tape : tape + a.gnp * a.xs;
-    const double* H = DIR == 0 ? hb : hb + 4 * a.xs;
-    const long long base = DIR == 0 ? (long long)j * (a.ni + 1) : i;
+    const long long base = DIR == 0 ? (long long)line * (a.ni + 1) : line;
     const long long stride = DIR == 0 ? 1 : a.ni;
-    constexpr double we[2][4] = {{4.0 / 3.0, 13.0 / 9.0, 40.0 / 27.0, 121.0 / 81.0},
-                                 {-1.0 / 3.0, -4.0 / 9.0, -13.0 / 27.0, -40.0 / 81.0}};
-#pragma unroll 1
-    for (int side = 0; side < 2; ++side) {
-        int rule = a.rule[DIR == 0 ? 2 + side : side];
-        if (rule == kRulePeriodic) continue;
-        const int line = DIR == 0 ? j : i;
-        if (rule == kRuleDMRBottom) rule = ((double)(i + 1) - 0.5) * a.dx >= 1.0 / 6.0 ? kRuleReflect : kRuleFixed;
-        const int dist = side == 0 ? x + 1 : n - x;  // 1 = next to the side
-        if (rule == kRuleFixed || rule == kRuleSSLInflow) {
-            // a fixed ghost state depends on no cell; only GLF's global lambda enters its
-            // split, dF+-/dlambda = +-U/2, whose sensitivity the cell next to the side takes for
-            // the line's four ghosts. The shear layer's inflow moves with the step's start time:
-            // the same cell takes its ghosts' time sensitivity, (dL/dghost)^T w . dghost/dt
-            // with only v moving (dU/dt = (0, 0, rho, rho v) v', dprim/dt = (0, 0, v', 0, 0)),
-            // and, for the characteristic schemes, the boundary face's Roe share of ghost 0.
-            const bool moving = rule == kRuleSSLInflow;
-            if (dist != 1 || (SPL != 1 && !moving)) continue;
-            double Ug[4], qg[5];
-            fixed_state(a, DIR, side, line, t, Ug, qg);
-            double dv = 0.0;
-            if (moving) {
-                double r_, u_, v_, p_;
-                ssl_inflow(a, line, t, r_, u_, v_, p_, dv);
-            }
-#pragma unroll 1
-            for (int k = 0; k < 4; ++k) {
-                double gp[4] = {0, 0, 0, 0}, gm[4] = {0, 0, 0, 0};
-                gather_line<REC>(T, H, ts, base, stride, side == 0 ? -1 - k : n + k, n, false, gp, gm);
-                if (SPL == 1) {
-                    double s = 0.0;
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) s = fma(gp[c] - gm[c], Ug[c], s);
-                    lb += 0.5 * s;
-                }
-                if (!moving) continue;
-                if (SPL == 2) {
-                    const double pv[4] = {qg[0], qg[1], qg[2], qg[4]};
-                    double pr4[4] = {0, 0, 0, 0};
-                    sw_prim_bar<DIR>(pv, a.gamma, gp, gm, pr4);
-                    tl = fma(pr4[2], dv, tl);
-                } else {
-                    // U of the ghost and its primitives (rho, u, v, p, alpha)
-                    const double g[9] = {Ug[0], Ug[1], Ug[2], Ug[3], qg[0], qg[1], qg[2], qg[3], qg[4]};
-                    double Ubg[4] = {0, 0, 0, 0}, unb, pb, ab;
-                    llf_bar<DIR, SPL == 1>(g, g[5 + DIR], g[7], g[8], gp, gm, lam_g, Ubg, unb, pb, ab);
-                    // the normal velocity (u on the left side) does not move; v does
-                    tl = fma(Ubg[2] * qg[0] + Ubg[3] * (qg[0] * qg[2]), dv, tl);
-                    if (DIR == 1) tl = fma(unb, dv, tl);
-                }
-                if (a.charac && k == 0) {
-                    const double* RB = a.rbar + (DIR == 0 ? 0 : 8 * a.xs) + base + (long long)(side == 0 ? 0 : n) * stride;
-                    tl = fma(RB[(side == 0 ? 2 : 6) * ts], dv, tl);
-                }
-            }
-            continue;
+    auto off = [&](int xx) { return DIR == 0 ? (long long)line * a.ni + xx : (long long)xx * a.ni + line; };
+    const int k = rule == kRuleExtrap ? slot & 3 : slot;                    // the ghost's layer
+    const int dist = rule == kRuleExtrap ? 1 + (slot >> 2) : rule == kRuleReflect ? slot + 1 : 1;
+    if (dist > n) return;
+    double Ub[4] = {0, 0, 0, 0}, pbar[5] = {0, 0, 0, 0, 0}, lb = 0.0, tl = 0.0;
+    double gp[4] = {0, 0, 0, 0}, gm[4] = {0, 0, 0, 0};
+    gather_line<REC>(T, H, ts, base, stride, side == 0 ? -1 - k : n + k, n, false, gp, gm);
+    if (rule == kRuleFixed || rule == kRuleSSLInflow) {
+        // a fixed ghost state depends on no cell; only GLF's global lambda enters its
+        // split, dF+-/dlambda = +-U/2, whose sensitivity the cell next to the side takes for
+        // the line's four ghosts. The shear layer's inflow moves with the step's start time:
+        // the same cell takes its ghosts' time sensitivity, (dL/dghost)^T w . dghost/dt
+        // with only v moving (dU/dt = (0, 0, rho, rho v) v', dprim/dt = (0, 0, v', 0, 0)),
+        // and, for the characteristic schemes, the boundary face's Roe share of ghost 0.
+        const bool moving = rule == kRuleSSLInflow;
+        double Ug[4], qg[5], dv = 0.0;
+        fixed_state(a, DIR, side, line, t, Ug, qg);
+        if (moving) {
+            double r_, u_, v_, p_;
+            ssl_inflow(a, line, t, r_, u_, v_, p_, dv);
         }
-        if (dist > (rule == kRuleReflect ? 4 : 2)) continue;
-        // extrapolation: conserved variables and primitives (rho, u, v, p, alpha) of the two
-        // cells next to the side
-        double c1[9], c2[9];
-        if (rule == kRuleExtrap) {
+        if (SPL == 1) {
+            double s = 0.0;
 #pragma unroll
-            for (int d = 0; d < 2; ++d) {
-                const int xx = side == 0 ? d : n - 1 - d;
-                const long long o = DIR == 0 ? (long long)j * a.ni + xx : (long long)xx * a.ni + i;
-                double* c = d == 0 ? c1 : c2;
-#pragma unroll
-                for (int v = 0; v < 4; ++v) c[v] = u[v * a.plane + o];
-                const Prim qq = prim_of(c, a.gamma);
-                c[4] = c[0]; c[5] = qq.u; c[6] = qq.v; c[7] = qq.p; c[8] = qq.a;
-            }
+            for (int c = 0; c < 4; ++c) s = fma(gp[c] - gm[c], Ug[c], s);
+            lb = 0.5 * s;
         }
-#pragma unroll 1
-        for (int k = 0; k < 4; ++k) {
-            double w;
-            if (rule == kRuleReflect) {
-                if (dist != k + 1) continue;
-                w = 1.0;
-            } else {
-                w = we[dist - 1][k];
-            }
-            double g[9];  // the ghost's U (0..3) and primitives (4..8)
-            if (rule == kRuleReflect) {
-#pragma unroll
-                for (int v = 0; v < 4; ++v) g[v] = U[v];
-                g[4] = U[0]; g[5] = q.u; g[6] = q.v; g[7] = q.p; g[8] = q.a;
-                g[1 + DIR] = -g[1 + DIR];
-                g[5 + DIR] = -g[5 + DIR];
-            } else {
-#pragma unroll
-                for (int v = 0; v < 9; ++v) {
-                    double na = c1[v], fa = c2[v], gv = 0.0;
-                    for (int l = 0; l <= k; ++l) {
-                        gv = fma(na, 4.0 / 3.0, -(fa * (1.0 / 3.0)));
-                        fa = na;
-                        na = gv;
-                    }
-                    g[v] = gv;
-                }
-            }
-            double gp[4] = {0, 0, 0, 0}, gm[4] = {0, 0, 0, 0};
-            gather_line<REC>(T, H, ts, base, stride, side == 0 ? -1 - k : n + k, n, false, gp, gm);
-            double Ubg[4] = {0, 0, 0, 0}, prb[5] = {0, 0, 0, 0, 0};
+        if (moving) {
             if (SPL == 2) {
-                const double pv[4] = {g[4], g[5], g[6], g[8]};
+                const double pv[4] = {qg[0], qg[1], qg[2], qg[4]};
                 double pr4[4] = {0, 0, 0, 0};
                 sw_prim_bar<DIR>(pv, a.gamma, gp, gm, pr4);
-                prb[0] = pr4[0]; prb[1] = pr4[1]; prb[2] = pr4[2]; prb[4] = pr4[3];
+                tl = pr4[2] * dv;
             } else {
-                double unb, pb, ab;
-                const double lamb = llf_bar<DIR, SPL == 1>(g, g[5 + DIR], g[7], g[8], gp, gm, lam_g, Ubg, unb, pb, ab);
-                prb[1 + DIR] = unb;
-                prb[3] = pb;
-                prb[4] = ab;
-                if (SPL == 1 && (rule == kRuleReflect || dist == 1)) lb += lamb;
+                // U of the ghost and its primitives (rho, u, v, p, alpha)
+                const double g[9] = {Ug[0], Ug[1], Ug[2], Ug[3], qg[0], qg[1], qg[2], qg[3], qg[4]};
+                double Ubg[4] = {0, 0, 0, 0}, unb, pb, ab;
+                llf_bar<DIR, SPL == 1>(g, g[5 + DIR], g[7], g[8], gp, gm, lam_g, Ubg, unb, pb, ab);
+                // the normal velocity (u on the left side) does not move; v does
+                tl = (Ubg[2] * qg[0] + Ubg[3] * (qg[0] * qg[2])) * dv;
+                if (DIR == 1) tl = fma(unb, dv, tl);
             }
-            if (a.adapt)  // the ghost's density in the surrogate stencils that read it
-                prb[0] += gather_rho_line(T, ts, base, stride, side == 0 ? -1 - k : n + k, n, false);
             if (a.charac && k == 0) {
-                // the ghost next to the side is a Roe cell of the boundary face: the left cell of
-                // face 0, the right cell of face n
                 const double* RB = a.rbar + (DIR == 0 ? 0 : 8 * a.xs) + base + (long long)(side == 0 ? 0 : n) * stride;
-#pragma unroll
-                for (int v = 0; v < 4; ++v) prb[v] += RB[(side == 0 ? v : 4 + v) * ts];
+                tl = fma(RB[(side == 0 ? 2 : 6) * ts], dv, tl);
             }
-            const double sn = rule == kRuleReflect ? -1.0 : 1.0;
+        }
+    } else {
+        double w = 1.0, g[9];  // the cell's weight in the ghost; the ghost's U (0..3) and primitives (4..8)
+        auto state = [&](int xx, double c[9]) {
+            const long long o = off(xx);
 #pragma unroll
-            for (int v = 0; v < 4; ++v) Ub[v] += (v == 1 + DIR ? sn * w : w) * Ubg[v];
+            for (int v = 0; v < 4; ++v) c[v] = u[v * a.plane + o];
+            const Prim qq = prim_of(c, a.gamma);
+            c[4] = c[0]; c[5] = qq.u; c[6] = qq.v; c[7] = qq.p; c[8] = qq.a;
+        };
+        if (rule == kRuleReflect) {
+            state(side == 0 ? k : n - 1 - k, g);
+            g[1 + DIR] = -g[1 + DIR];
+            g[5 + DIR] = -g[5 + DIR];
+        } else {
+            constexpr double we[2][4] = {{4.0 / 3.0, 13.0 / 9.0, 40.0 / 27.0, 121.0 / 81.0},
+                                         {-1.0 / 3.0, -4.0 / 9.0, -13.0 / 27.0, -40.0 / 81.0}};
+            w = we[dist - 1][k];
+            double c1[9], c2[9];
+            state(side == 0 ? 0 : n - 1, c1);
+            state(side == 0 ? 1 : n - 2, c2);
 #pragma unroll
-            for (int v = 0; v < 5; ++v) pbar[v] += (v == 1 + DIR ? sn * w : w) * prb[v];
+            for (int v = 0; v < 9; ++v) {
+                double na = c1[v], fa = c2[v], gv = 0.0;
+                for (int l = 0; l <= k; ++l) {
+                    gv = fma(na, 4.0 / 3.0, -(fa * (1.0 / 3.0)));
+                    fa = na;
+                    na = gv;
+                }
+                g[v] = gv;
+            }
+        }
+        double Ubg[4] = {0, 0, 0, 0}, prb[5] = {0, 0, 0, 0, 0};
+        if (SPL == 2) {
+            const double pv[4] = {g[4], g[5], g[6], g[8]};
+            double pr4[4] = {0, 0, 0, 0};
+            sw_prim_bar<DIR>(pv, a.gamma, gp, gm, pr4);
+            prb[0] = pr4[0]; prb[1] = pr4[1]; prb[2] = pr4[2]; prb[4] = pr4[3];
+        } else {
+            double unb, pb, ab;
+            const double lamb = llf_bar<DIR, SPL == 1>(g, g[5 + DIR], g[7], g[8], gp, gm, lam_g, Ubg, unb, pb, ab);
+            prb[1 + DIR] = unb;
+            prb[3] = pb;
+            prb[4] = ab;
+            if (SPL == 1 && (rule == kRuleReflect || dist == 1)) lb = lamb;
+        }
+        if (a.adapt)  // the ghost's density in the surrogate stencils that read it
+            prb[0] += gather_rho_line(T, ts, base, stride, side == 0 ? -1 - k : n + k, n, false);
+        if (a.charac && k == 0) {
+            // the ghost next to the side is a Roe cell of the boundary face: the left cell of
+            // face 0, the right cell of face n
+            const double* RB = a.rbar + (DIR == 0 ? 0 : 8 * a.xs) + base + (long long)(side == 0 ? 0 : n) * stride;
+#pragma unroll
+            for (int v = 0; v < 4; ++v) prb[v] += RB[(side == 0 ? v : 4 + v) * ts];
+        }
+        const double sn = rule == kRuleReflect ? -1.0 : 1.0;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) Ub[v] = (v == 1 + DIR ? sn * w : w) * Ubg[v];
+#pragma unroll
+        for (int v = 0; v < 5; ++v) pbar[v] = (v == 1 + DIR ? sn * w : w) * prb[v];
+    }
+#pragma unroll
+    for (int v = 0; v < 4; ++v) a.wall[wall_at(a, DIR, side, slot, v, line)] = Ub[v];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) a.wall[wall_at(a, DIR, side, slot, 4 + v, line)] = pbar[v];
+    a.wall[wall_at(a, DIR, side, slot, 9, line)] = lb;
+    a.wall[wall_at(a, DIR, side, slot, 10, line)] = tl;
+}
+// blockIdx.y the slot, blockIdx.z the side (left, right, bottom, top), a thread per line
+template <int SPL, int REC>
+__global__ void __launch_bounds__(128) k_wall(AdjParams a, const double* __restrict__ u,
+                                              const double* __restrict__ tape, const double* __restrict__ hb,
+                                              const double* __restrict__ lamv, const double* __restrict__ tp) {
+    const int line = blockIdx.x * blockDim.x + threadIdx.x, side = blockIdx.z & 1, slot = blockIdx.y;
+    const double t = tp ? *tp : 0.0;  // the step's start time (the moving shock's ghosts)
+    if (blockIdx.z < 2) {
+        if (line < a.nj) wall_ghost<0, SPL, REC>(a, u, tape, hb, side, slot, line, SPL == 1 ? lamv[0] : 0.0, t);
+    } else if (line < a.ni) {
+        wall_ghost<1, SPL, REC>(a, u, tape + a.gnp * a.xs, hb + 4 * a.xs, side, slot, line, SPL == 1 ? lamv[1] : 0.0, t);
+    }
+}
+// The parked shares of the cell at position x of a line.
+template <int DIR>
+__device__ __forceinline__ void wall_terms(const AdjParams& a, int line, int x, double Ub[4], double pbar[5],
+                                           double& lb, double& tl) {
+    const int n = DIR == 0 ? a.ni : a.nj;
+#pragma unroll 1
+    for (int side = 0; side < 2; ++side) {
+        const int rule = rule_at(a, DIR, side, line), dist = side == 0 ? x + 1 : n - x;  // 1 = next to the side
+        int s0 = 0, ns = 0;
+        if (rule == kRuleExtrap && dist <= 2) { s0 = (dist - 1) * 4; ns = 4; }
+        else if (rule == kRuleReflect && dist <= 4) { s0 = dist - 1; ns = 1; }
+        else if ((rule == kRuleFixed || rule == kRuleSSLInflow) && dist == 1) ns = 4;
+#pragma unroll 1
+        for (int q = s0; q < s0 + ns; ++q) {
+#pragma unroll
+            for (int v = 0; v < 4; ++v) Ub[v] += a.wall[wall_at(a, DIR, side, q, v, line)];
+#pragma unroll
+            for (int v = 0; v < 5; ++v) pbar[v] += a.wall[wall_at(a, DIR, side, q, 4 + v, line)];
+            lb += a.wall[wall_at(a, DIR, side, q, 9, line)];
+            tl += a.wall[wall_at(a, DIR, side, q, 10, line)];
         }
     }
 }
@@ -981,78 +1012,92 @@ __global__ void __launch_bounds__(128, 4) k_char_face(AdjParams a, const double*
     RB[3 * ts] = kgir * hbar;
 }
 
+// One direction's share of Ub = (dL/du)^T w at a cell; lb: GLF's lambda sensitivity, tl: the start
+// time's.
+template <int DIR, int REC, int SPL, bool WALLS>
+__device__ __forceinline__ void rev_direction(const AdjParams& a, const double* __restrict__ tape,
+                                              const double* __restrict__ hb, int i, int j, const double U[4],
+                                              const Prim& q, double lam_g, double Ub[4], double& lb, double& tl) {
+    constexpr bool GLF = SPL == 1;
+    const int ni = a.ni, n = DIR == 0 ? ni : a.nj, x = DIR == 0 ? i : j;
+    const bool periodic = a.rule[DIR == 0 ? 2 : 0] == kRulePeriodic;
+    const long long ts = DIR == 0 ? a.xs : a.ys, stride = DIR == 0 ? 1 : ni;
+    const long long base = DIR == 0 ? (long long)j * (ni + 1) : i;
+    const double* T = tape + (DIR == 0 ? 0 : a.gnp * a.xs);
+    double gp[4] = {0, 0, 0, 0}, gm[4] = {0, 0, 0, 0};
+    gather_line<REC>(T, hb + (DIR == 0 ? 0 : 4 * a.xs), ts, base, stride, x, n, periodic, gp, gm);
+    if (SPL != 2) lb = llf_vjp<DIR, GLF>(U, q, a.gamma, gp, gm, lam_g, Ub);
+    else          sw_vjp<DIR>(U, a.gamma, gp, gm, Ub);
+    double pbar[5] = {0, 0, 0, 0, 0};
+    if (a.charac) {
+        // the Roe averages of the faces this cell is a side of: the left cell of face x+1 and
+        // the right cell of face x (and, on periodic lines, the right cell of face n from cell 0 and
+        // the left cell of face 0 from cell n-1, their images)
+        const double* RB = a.rbar + (DIR == 0 ? 0 : 8 * a.xs) + base;
+        auto add = [&](int f, int q0) {
+#pragma unroll
+            for (int v = 0; v < 4; ++v) pbar[v] += RB[(q0 + v) * ts + f * stride];
+        };
+        add(x + 1, 0);
+        add(x, 4);
+        if (periodic) {
+            if (x == n - 1) add(0, 0);
+            if (x == 0) add(n, 4);
+        }
+    }
+    if (a.adapt) Ub[0] += gather_rho_line(T, ts, base, stride, x, n, periodic);  // (rho = U[0])
+    if (WALLS && !periodic) wall_terms<DIR>(a, DIR == 0 ? j : i, x, Ub, pbar, lb, tl);
+    if (a.charac || (WALLS && !periodic))
+        prim_pullback_all(U, q, a.gamma, pbar[0], pbar[1], pbar[2], pbar[3], pbar[4], Ub);
+}
+
 // Cell kernel: Ub = (dL/du)^T w at the cell from the stage's tape and hbar, then the reverse of
 // RK stage STAGE (3, 2, 1; 0 = Ub alone; a kernel argument, uniform over the grid). Stage 1
 // also reduces the wave-speed maxima of its state u0 (the time step's input) per block, with
-// their cells. WALLS: the grid has wall sides (wall_terms). SPL: 0 LLF, 1 GLF, 2 SW. GLF:
+// their cells. WALLS: the grid has wall sides (k_wall). SPL: 0 LLF, 1 GLF, 2 SW. GLF:
 // lamv holds the stage's global lambda of both directions; the sensitivities of lambda are summed
-// per block into lpart.
+// per block into lpart. Two threads share a cell (threadIdx.z), one a direction -- the gather of a
+// direction's 40 taped entries and its split's transpose are one long chain of loads and FP64
+// operations, and a thread a cell leaves most of the GPU idle on the adjoint's grids --, and the
+// first adds the second's share and finishes the cell (REV_FIGURES).
 template <int REC, int SPL, bool WALLS>
-__global__ void __launch_bounds__(128) k_rev(AdjParams a, const double* __restrict__ u,
+__global__ void __launch_bounds__(256) k_rev(AdjParams a, const double* __restrict__ u,
                                              const double* __restrict__ w, const double* __restrict__ tape,
                                              const double* __restrict__ hb, double* __restrict__ acc,
                                              double* __restrict__ out, const double* __restrict__ dtp,
-                                             const double* __restrict__ tp, double* __restrict__ mpart,
+                                             double* __restrict__ mpart,
                                              const double* __restrict__ lamv, double* __restrict__ lpart,
                                              int STAGE) {
+    __shared__ double other[4][128];
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int ni = a.ni, nj = a.nj;
+    const int ni = a.ni, nj = a.nj, cell = threadIdx.x + blockDim.x * threadIdx.y;
+    const bool inside = i < ni && j < nj;
     double e1 = -1.0, e2 = -1.0;
     long long i1 = LLONG_MAX, i2 = LLONG_MAX;
     double lbx = 0.0, lby = 0.0;
     double bsum = 0.0, Ub_bf0 = 0.0, Ub_bf2 = 0.0;  // the body force's terms (a.bodyforce)
     double tsl = 0.0;                                 // the inflow ghosts' time sensitivity (a.ssl)
-    if (i < ni && j < nj) {
-        const long long o = (long long)j * ni + i;
-        double U[4], Ub[4] = {0.0, 0.0, 0.0, 0.0};
+    const long long o = (long long)j * ni + i;
+    double U[4], Ub[4] = {0.0, 0.0, 0.0, 0.0};
+    Prim q;
+    if (inside) {
 #pragma unroll
         for (int v = 0; v < 4; ++v) U[v] = u[v * a.plane + o];
+        q = prim_of(U, a.gamma);
         constexpr bool GLF = SPL == 1;
-        const Prim q = prim_of(U, a.gamma);
-        double gpx[4] = {0, 0, 0, 0}, gmx[4] = {0, 0, 0, 0}, gpy[4] = {0, 0, 0, 0}, gmy[4] = {0, 0, 0, 0};
-        const bool px = a.rule[2] == kRulePeriodic, py = a.rule[0] == kRulePeriodic;
-        gather_line<REC>(tape, hb, a.xs, (long long)j * (ni + 1), 1, i, ni, px, gpx, gmx);
-        // LF splittings pull each direction back before gathering the next (fewer live
-        // registers); Steger-Warming seeds each variable once for both directions
-        if (SPL != 2) lbx = llf_vjp<0, GLF>(U, q, a.gamma, gpx, gmx, GLF ? lamv[0] : 0.0, Ub);
-        gather_line<REC>(tape + a.gnp * a.xs, hb + 4 * a.xs, a.ys, i, ni, j, nj, py, gpy, gmy);
-        if (SPL != 2) lby = llf_vjp<1, GLF>(U, q, a.gamma, gpy, gmy, GLF ? lamv[1] : 0.0, Ub);
-        else          sw_vjp(U, a.gamma, gpx, gmx, gpy, gmy, Ub);
-        if (a.charac) {
-            // the Roe averages of the faces this cell is a side of: the left cell of face x+1 and
-            // the right cell of face x in each direction (and, on periodic lines, the right cell
-            // of face n from cell 0 and the left cell of face 0 from cell n-1, their images)
-            double rb[4] = {0.0, 0.0, 0.0, 0.0};
+        if (threadIdx.z == 0)
+            rev_direction<0, REC, SPL, WALLS>(a, tape, hb, i, j, U, q, GLF ? lamv[0] : 0.0, Ub, lbx, tsl);
+        else
+            rev_direction<1, REC, SPL, WALLS>(a, tape, hb, i, j, U, q, GLF ? lamv[1] : 0.0, Ub, lby, tsl);
+        if (threadIdx.z == 1) {
 #pragma unroll
-            for (int D = 0; D < 2; ++D) {
-                const int n = D == 0 ? ni : nj, x = D == 0 ? i : j;
-                const long long ts = D == 0 ? a.xs : a.ys;
-                const double* RB = a.rbar + (D == 0 ? 0 : 8 * a.xs);
-                auto face = [&](int f) { return D == 0 ? (long long)j * (ni + 1) + f : (long long)f * ni + i; };
-                auto add = [&](int f, int q0) {
+            for (int v = 0; v < 4; ++v) other[v][cell] = Ub[v];
+        }
+    }
+    __syncthreads();
+    if (inside && threadIdx.z == 0) {
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) rb[v] += RB[(q0 + v) * ts + face(f)];
-                };
-                add(x + 1, 0);
-                add(x, 4);
-                if (D == 0 ? px : py) {
-                    if (x == n - 1) add(0, 0);
-                    if (x == 0) add(n, 4);
-                }
-            }
-            prim_pullback_all(U, q, a.gamma, rb[0], rb[1], rb[2], rb[3], 0.0, Ub);
-        }
-        if (a.adapt)  // the surrogate stencils' density sensitivities (rho = U[0])
-            Ub[0] += gather_rho_line(tape, a.xs, (long long)j * (ni + 1), 1, i, ni, px) +
-                     gather_rho_line(tape + a.gnp * a.xs, a.ys, i, ni, j, nj, py);
-        if (WALLS && (!px || !py)) {  // the ghost cells of wall sides that this cell feeds
-            // (a separate instantiation: the periodic kernels keep their registers)
-            double pbar[5] = {0, 0, 0, 0, 0};
-            const double t = tp ? *tp : 0.0;  // the step's start time (the moving shock's ghosts)
-            if (!px) wall_terms<0, SPL, REC>(a, u, tape, hb, i, j, q, U, GLF ? lamv[0] : 0.0, t, Ub, pbar, lbx, tsl);
-            if (!py) wall_terms<1, SPL, REC>(a, u, tape, hb, i, j, q, U, GLF ? lamv[1] : 0.0, t, Ub, pbar, lby, tsl);
-            prim_pullback_all(U, q, a.gamma, pbar[0], pbar[1], pbar[2], pbar[3], pbar[4], Ub);
-        }
+        for (int v = 0; v < 4; ++v) Ub[v] += other[v][cell];
         const double dt = STAGE == 0 ? 0.0 : *dtp;
         if (STAGE != 0 && a.bodyforce) {
             // the stage's body force f_s (0, 0, rho, rho v) of its input u: (df/du)^T w sends
@@ -1091,7 +1136,7 @@ __global__ void __launch_bounds__(128) k_rev(AdjParams a, const double* __restri
     if (STAGE == 1 && mpart) {
         // block argmax, ties to the lowest cell index
         block_argmax(e1, i1, e2, i2);
-        if (threadIdx.x == 0 && threadIdx.y == 0) {
+        if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
             double* mp = mpart + 4 * (blockIdx.y * gridDim.x + blockIdx.x);
             mp[0] = e1; mp[1] = (double)i1; mp[2] = e2; mp[3] = (double)i2;
         }
@@ -1099,7 +1144,7 @@ __global__ void __launch_bounds__(128) k_rev(AdjParams a, const double* __restri
     if (SPL == 1) {
         __syncthreads();  // the argmax reduction's shared arrays are read before the next sum
         block_sum2(lbx, lby);
-        if (threadIdx.x == 0 && threadIdx.y == 0) {
+        if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
             double* lp = lpart + 2 * (blockIdx.y * gridDim.x + blockIdx.x);
             lp[0] = lbx;
             lp[1] = lby;
@@ -1109,7 +1154,7 @@ __global__ void __launch_bounds__(128) k_rev(AdjParams a, const double* __restri
         __syncthreads();  // the shared arrays of the reductions above are free again
         block_sum2(bsum, tsl);
         const int blk = (STAGE - 1) * (gridDim.x * gridDim.y) + blockIdx.y * gridDim.x + blockIdx.x;
-        if (threadIdx.x == 0 && threadIdx.y == 0) {
+        if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
             if (a.bodyforce) a.bpart[blk] = bsum;
             if (a.ssl) a.tpart[blk] = tsl;
         }
@@ -1427,15 +1472,19 @@ template <int REC, int SPL, bool WALLS>
 void launch_rev_w(dense_adjoint* a, int stage, const double* u, const double* tape, const double* w, double* out,
                   const double* dtp, const double* tp, cudaStream_t s) {
     using namespace dense::adj;
-    const dim3 bc(kCX, kCY);
+    const dim3 bc(kCX, kCY, 2);
     double* const lv = a->lamv;
     double* const lp = a->lpart;
     const double* hb = a->hb;
+    if (WALLS) {
+        const int lines = a->ap.ni > a->ap.nj ? a->ap.ni : a->ap.nj;
+        k_wall<SPL, REC><<<dim3((lines + 127) / 128, kWallSlots, 4), 128, 0, s>>>(a->ap, u, tape, hb, lv, tp);
+        a->launches += 1;
+    }
     if (stage == 0)
-        k_rev<REC, SPL, WALLS><<<a->gc, bc, 0, s>>>(a->ap, u, w, tape, hb, nullptr, out, nullptr, tp, nullptr,
-                                                    lv, lp, 0);
+        k_rev<REC, SPL, WALLS><<<a->gc, bc, 0, s>>>(a->ap, u, w, tape, hb, nullptr, out, nullptr, nullptr, lv, lp, 0);
     else
-        k_rev<REC, SPL, WALLS><<<a->gc, bc, 0, s>>>(a->ap, u, w, tape, hb, a->acc, out, dtp, tp,
+        k_rev<REC, SPL, WALLS><<<a->gc, bc, 0, s>>>(a->ap, u, w, tape, hb, a->acc, out, dtp,
                                                     stage == 1 ? a->mpart : nullptr, lv, lp, stage);
 }
 template <int REC, int SPL>
@@ -1613,7 +1662,7 @@ void dense_adjoint_destroy(dense_adjoint_t* a) {
     if (a->h) cudaStreamSynchronize(a->h->stream);
     double* bufs[] = {a->ckpt, a->dts, a->rec, a->tape, a->g, a->g1, a->g2, a->acc, a->hb, a->part, a->mpart,
                       a->lamv, a->lmp, a->lpart, a->seg_dts, a->ap.bpart, a->fbar, a->ap.rbar,
-                      a->ap.tpart, a->ap.tacc};
+                      a->ap.tpart, a->ap.tacc, a->ap.wall};
     for (double* b : bufs) if (b) cudaFree(b);
     if (a->argmax) cudaFree(a->argmax);
     if (a->seg_argmax) cudaFree(a->seg_argmax);
@@ -1743,6 +1792,7 @@ int dense_adjoint_create(const dense_config_t* cfg, int checkpoint_every, dense_
         {&a->rec, (size_t)3 * a->k * a->state}, {&a->tape, (size_t)3 * a->k * a->tape_stage},
         {&a->lamv, 4}, {&a->lmp, (size_t)4 * a->nm}, {&a->lpart, (size_t)2 * a->nm}, {&a->seg_dts, (size_t)2 * a->k},
         {&p.bpart, (size_t)3 * a->nm}, {&p.tpart, (size_t)3 * a->nm}, {&p.tacc, 1},
+        {&p.wall, (size_t)4 * dense::adj::kWallSlots * dense::adj::kWallTerms * (size_t)(cfg->ni > cfg->nj ? cfg->ni : cfg->nj)},
     };
     for (auto& b : bufs) {
         cudaError_t e = cudaMalloc((void**)b.p, b.n * sizeof(double));
