@@ -548,7 +548,8 @@ __device__ __forceinline__ void fixed_state(const AdjParams& a, int dir, int sid
 // state's four ghosts with the cell next to the side, slot k. k_wall takes a thread for each
 // and parks its shares -- Ub (4), pbar (5), lambda's, the start time's -- in a.wall, where k_rev's
 // thread of the cell adds them in order: as a loop over the ghosts in k_rev they set the time of the
-// whole kernel on small grids and its registers on all (254 instead of 128: WALL_FIGURES).
+// whole kernel on small grids and its registers on all (254 instead of 128; the 128 x 512 characteristic
+// case's kernel 118 us, now 55 and 11 for the ghosts).
 constexpr int kWallSlots = 8, kWallTerms = 11;
 __device__ __forceinline__ long long wall_at(const AdjParams& a, int dir, int side, int slot, int term, int line) {
     const long long pitch = a.ni > a.nj ? a.ni : a.nj;
@@ -788,20 +789,22 @@ __device__ __forceinline__ void fetch_cell(const AdjParams& a, const double* __r
 // copy of the integer gradient stays in the instruction cache. The transposed Jacobian of the 128 x
 // 512 Rayleigh-Taylor case, where both directions' face kernels took 0.43 of 0.75 ms, takes 0.58 ms.
 template <int DIR>
-__global__ void __launch_bounds__(128, 4) k_char_face(AdjParams a, const double* __restrict__ u,
-                                                  const double* __restrict__ hb, const double* __restrict__ lamv,
-                                                  const double* __restrict__ tp, const double* __restrict__ flags,
-                                                  double* __restrict__ fbar) {
+__device__ __forceinline__ void char_face_block(const AdjParams& a, const double* __restrict__ u,
+                                                const double* __restrict__ hb, const double* __restrict__ lamv,
+                                                const double* __restrict__ tp, const double* __restrict__ flags,
+                                                double* __restrict__ fbar, int bx, int by) {
     constexpr int FA = DIR == 0 ? 16 : 4;  // faces of a block along the direction
     constexpr int NB = DIR == 0 ? 4 : 16;  // lines of a block
     constexpr int NA = FA + 5;             // cells staged along a line: f0-3 .. f0+FA+1
-    __shared__ double sC[12][NB][NA];      // F+ (0..3), F- (4..7), rho, u, v, p (8..11)
-    __shared__ double sL[24][128];         // per thread: field k's differences, then gradient, row k*5+m;
+    extern __shared__ double sm[];         // (one allocation for both directions)
+    double(*const sL)[128] = (double(*)[128])sm;
+    double(*const sC)[NB][NA] = (double(*)[NB][NA])(sm + 24 * 128);
+    // sC[12]: F+ (0..3), F- (4..7), rho, u, v, p (8..11); sL[24]: per thread: field k's differences, then gradient, row k*5+m;
                                            // its correction's sensitivity, then the correction, row 20+k
     const int ni = a.ni, nj = a.nj;
     const int n = DIR == 0 ? ni : nj, nline = DIR == 0 ? nj : ni;
     const int tid = threadIdx.x + 32 * threadIdx.y;
-    const int f0 = (DIR == 0 ? blockIdx.x : blockIdx.y) * FA, l0 = (DIR == 0 ? blockIdx.y : blockIdx.x) * NB;
+    const int f0 = (DIR == 0 ? bx : by) * FA, l0 = (DIR == 0 ? by : bx) * NB;
     const double lam = lamv[DIR];
     {
         const double t = tp ? *tp : 0.0;
@@ -1012,6 +1015,22 @@ __global__ void __launch_bounds__(128, 4) k_char_face(AdjParams a, const double*
     RB[3 * ts] = kgir * hbar;
 }
 
+// Both directions in one launch, whose blocks fill the GPU together where one direction's would not
+// (the 161 x 106 AdaWENO adjoint, nine steps, 8.02 -> 7.00 ms): the first nx x ny blocks are xi's.
+constexpr size_t kCharFaceSmem = sizeof(double) * (24 * 128 + 12 * 144);  // 4 x 21 or 16 x 9 cells
+__global__ void __launch_bounds__(128, 4) k_char_face(AdjParams a, const double* __restrict__ u,
+                                                  const double* __restrict__ hb, const double* __restrict__ lamv,
+                                                  const double* __restrict__ tp, const double* __restrict__ flags,
+                                                  double* __restrict__ fbar, int nx, int ny, int mx) {
+    int b = blockIdx.x;
+    if (b < nx * ny) {
+        char_face_block<0>(a, u, hb, lamv, tp, flags, fbar, b % nx, b / nx);
+    } else {
+        b -= nx * ny;
+        char_face_block<1>(a, u, hb, lamv, tp, flags, fbar, b % mx, b / mx);
+    }
+}
+
 // One direction's share of Ub = (dL/du)^T w at a cell; lb: GLF's lambda sensitivity, tl: the start
 // time's.
 template <int DIR, int REC, int SPL, bool WALLS>
@@ -1059,7 +1078,8 @@ __device__ __forceinline__ void rev_direction(const AdjParams& a, const double* 
 // per block into lpart. Two threads share a cell (threadIdx.z), one a direction -- the gather of a
 // direction's 40 taped entries and its split's transpose are one long chain of loads and FP64
 // operations, and a thread a cell leaves most of the GPU idle on the adjoint's grids --, and the
-// first adds the second's share and finishes the cell (REV_FIGURES).
+// first adds the second's share and finishes the cell (Steger-Warming on 141 x 47 cells with its walls,
+// 171 us a stage before: five steps' adjoint 3965 -> 2861 us with the ghosts' kernel).
 template <int REC, int SPL, bool WALLS>
 __global__ void __launch_bounds__(256) k_rev(AdjParams a, const double* __restrict__ u,
                                              const double* __restrict__ w, const double* __restrict__ tape,
@@ -1523,9 +1543,9 @@ void vjp(dense_adjoint* a, int stage, const double* u, const double* tape, const
     k_hbar<<<a->gh, dim3(kHX, kHY), 0, s>>>(a->ap, w, tape, a->hb, part);
     if (charac) {
         const double* flags = a->ap.adapt ? tape : nullptr;  // the branches taken, first plane a direction
-        k_char_face<0><<<a->gfx, dim3(kCX, kCY), 0, s>>>(a->ap, u, a->hb, a->lamv, tp, flags, a->fbar);
-        k_char_face<1><<<a->gfy, dim3(kCX, kCY), 0, s>>>(a->ap, u, a->hb, a->lamv, tp, flags, a->fbar);
-        a->launches += 2;
+        k_char_face<<<a->gfx.x * a->gfx.y + a->gfy.x * a->gfy.y, dim3(kCX, kCY), kCharFaceSmem, s>>>(
+            a->ap, u, a->hb, a->lamv, tp, flags, a->fbar, (int)a->gfx.x, (int)a->gfx.y, (int)a->gfy.x);
+        a->launches += 1;
         launch_rev<dense::adj::kRecFaceSens, 1>(a, stage, u, a->fbar, w, out, dtp, tp, s);  // the faces' own sensitivities
     } else if (glf) launch_rev_recon<1>(a, stage, u, tape, w, out, dtp, tp, s);
     else if (a->cfg.splitting == DENSE_SPLIT_SW) launch_rev_recon<2>(a, stage, u, tape, w, out, dtp, tp, s);
