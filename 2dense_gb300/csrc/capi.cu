@@ -184,8 +184,8 @@ int ensure_side(dense_handle* h) {
 // 64 x 64 3-4 % faster, 400 x 400 8.6 %, 512 x 512 4.2 %, 1024 x 1024 1.3 %; characteristic
 // Rayleigh-Taylor 128 x 512 19 %, 256 x 1024 1.9 %, 512 x 2048 0.2 %; Steger-Warming 481 x 479 0.8 %;
 // AdaWENO's double Mach reflection 240 x 60 5.7 %, 480 x 120 1.6 %, but 640 x 160 0.4 % slower,
-// 960 x 240 1.0 % and 1920 x 480 0.9 %: its sweeps' blocks are large and stay long, and the next
-// kernel's early blocks take their places. So: everywhere but on AdaWENO grids of 80,000 cells or
+// 960 x 240 1.0 % and 1920 x 480 0.9 % (in blocks of 128 threads 640 x 160 8 %, 1920 x 480 1.3 %): its
+// sweeps' blocks stay long, and the next kernel's early blocks take their places. So: everywhere but on AdaWENO grids of 80,000 cells or
 // more; DENSE_PDL=0 / 1 in the environment forces it off / on. (An explicit early trigger in every
 // kernel is slower on small grids: 200 x 200 vortex 920 against 886 us.)
 bool use_programmatic_edges(const dense_handle* h) {
@@ -194,7 +194,7 @@ bool use_programmatic_edges(const dense_handle* h) {
         return v && (v[0] == '0' || v[0] == '1') ? v[0] - '0' : -1;
     }();
     if (env >= 0) return env == 1;
-    return h->prm.splitting != DENSE_SPLIT_SC || (long long)h->prm.ni * h->prm.nj < 80000;
+    return h->prm.splitting != DENSE_SPLIT_SC || (long long)h->prm.ni * h->prm.nj < dense::kAdaptiveSmall;
 }
 cudaError_t programmatic_edges(cudaGraph_t g) {
     size_t ne = 0;

@@ -664,7 +664,8 @@ __global__ void k_flux_noop(Params p, int irk) {
 // whole block then works through the queue on full warps.
 // What bounds it: the FP64 pipe. The surrogate's weights and the smooth branch run on the integer
 // pipes (weno_fixed.cuh), which leaves some 55 FP64 instructions an interface of 150 and took the
-// 1920 x 480 double Mach reflection's sweeps from 0.282 and 0.305 ms to 0.149 and 0.172.
+// 1920 x 480 double Mach reflection's sweeps from 0.282 and 0.305 ms to 0.149 and 0.172 (0.139 and 0.141
+// with tiles of 128 threads).
 // Dynamic shared memory of one characteristic sweep block, in doubles: the tile's split fluxes
 // sF[8][NL][NC] and primitives sQ[4][NL][NC]; per-cell sqrt(rho) sS (104, fast); the split fluxes'
 // forward differences along the sweep sDF[8][NL][NC] (fast); and one region R that AdaWENO uses
@@ -1462,16 +1463,16 @@ __device__ __forceinline__ void bc_block(const Params& p, int bx) {
 // ---------------------------------------------------------------------------------------------
 // Kernels of one block (instance) of the solver: block coordinates are the launch's own.
 // Resident blocks the register allocation of a characteristic sweep is sized for. AdaWENO's
-// blocks stall on the barriers of their work queue, which a third block per SM hides (80
-// registers, a few bytes spilled; sweeps of the 1920 x 480 double Mach reflection, xi and eta:
-// 0.149 and 0.172 ms at three blocks; before its weights' last trimming 0.159 and 0.180 at three,
-// 0.180 and 0.203 at two, 0.162 and 0.188 at four). The 104
+// blocks stall on the barriers of their work queue, which 768 resident threads per SM hide (80
+// registers, a few bytes spilled; sweeps of the 1920 x 480 double Mach reflection in blocks of 256, xi
+// and eta: 0.159 and 0.180 ms at 768, 0.180 and 0.203 at 512, 0.162 and 0.188 at 1024; steps in blocks
+// of 128: 3.97 ms at 768, 4.00 at 640). The 104
 // sweeps' four inlined integer
 // reconstructions would take 160 registers; at 1024 resident threads (64 registers) the sweeps of
 // the 256 x 1024 Rayleigh-Taylor case took 0.127 (xi) and 0.111 ms (eta), at 768 0.131 and 0.113,
 // unbounded 0.141 and 0.158 (now 0.106 and 0.098, the roots on the integer pipes too; 0.340 and
 // 0.293 with the reconstructions in FP64).
-constexpr int char_min_blocks(bool adapt, int nt) { return adapt ? 3 : 1024 / nt; }
+constexpr int char_min_blocks(bool adapt, int nt) { return adapt ? 768 / nt : 1024 / nt; }
 template <int DIR, int SPL, int REC, int TX, int TY, bool TAPE = false, int TZ = 1>
 __global__ void __launch_bounds__(TX* TY* TZ) k_flux_cw(Params p, int irk) {
     grid_dependency_wait();
@@ -1700,26 +1701,40 @@ kb_persist(const Params* tab, PersistLaunch L, int xi_variant, int eta_variant) 
 
 // ---------------------------------------------------------------------------------------------
 // Launchers
-// Component-wise sweeps. xi tile: 32 interfaces x 4 rows (32 x 2 on small grids): a tile
-// stages (32 + 5)/32 = 1.16 cells per interface whatever its height. eta tile: 8 columns x 32
-// interfaces (8 x 8 on small grids): the halo runs along the sweep, so a tall narrow tile stages
-// (32 + 5)/32 = 1.16 cells per interface where 32 x 8 staged 1.63 and 32 x 4 2.25 (each staged
-// cell costs its split fluxes and eight indicator terms); 8-wide rows still read whole 64-byte
-// segments, and the smem rows of a warp (4 rows x 8 columns) stay free of bank conflicts.
-constexpr int kXTX = 32, kXTY = 4, kXSTY = 2;   // xi tile; small-grid height
-constexpr int kETX = 8, kETY = 32, kESTY = 8;   // eta tile; small-grid height
-// characteristic sweeps: eta tiles of 4 columns x 64 interfaces, AdaWENO xi tiles of one row of
-// 256 threads (251 interfaces, 256 cells; long lines along the sweep stage fewer halo cells per
-// interface: 1.02 in xi and 1.08 in eta against 1.16 and 1.63 for 32 x 4 and 32 x 8; measured on
-// the 1920 x 480 double Mach reflection, these shapes took the sweeps from 0.430 / 0.427 to
-// 0.385 / 0.374 ms, the eta tile below to 0.355 ms)
-constexpr int kCETX = 4, kCETY = 64;
-constexpr int kCXTX = 256, kCXTY = 1;
-// AdaWENO eta tiles: 2 columns of 128 threads (123 interfaces, 128 cells each): every thread
-// stages one cell, and 123-interface columns cover 481 interfaces in 4 tiles with 2 % idle
-// lanes against 6 % for 64-interface columns. (The 104 eta sweep, at 102 registers a thread,
-// ran 5 % slower on such tiles on the 256 x 1024 Rayleigh-Taylor case and keeps 4 x 64.)
-constexpr int kAETX = 2, kAETY = 128;
+// Component-wise sweeps. xi tile: 64 interfaces x 2 rows (32 x 2 on small grids), which stages
+// (64 + 5)/64 = 1.08 cells per interface. eta tile: 4 columns x 32 interfaces (8 x 8 on small
+// grids): the halo runs along the sweep, so a tall narrow tile stages (32 + 5)/32 = 1.16 cells per
+// interface (each staged cell costs its split fluxes); 4-wide rows still read whole 32-byte
+// sectors. Blocks of 128 threads: the last wave ends sooner, and a block waits less for its
+// slowest warp. Sweeps (xi, eta) against tiles of 32 x 4 and 8 x 32: 2048 x 2048 LLF + WENO-JS 0.682 and
+// 0.668 -> 0.675 and 0.657 ms, 1024 x 1024 GLF + upwind 0.157 and 0.131 -> 0.143 and 0.131, 481 x 479
+// Steger-Warming + WENO-Z 0.069 and 0.071 -> 0.067 and 0.064. Steps, the last: 4.26 -> 4.08 ms (xi 128 x 1:
+// 4.01, but 5 % slower on a 512 x 512 vortex; 96 x 1: 4.21; eta 4 x 16: 4.36; 8 x 64: 4.75).
+constexpr int kXTX = 64, kXTY = 2, kXSTX = 32, kXSTY = 2;  // xi tile; on small grids
+constexpr int kETX = 4, kETY = 32, kESTX = 8, kESTY = 8;   // eta tile; on small grids
+// 104 sweeps: 32 interfaces x 4 rows, 4 columns x 32 interfaces. Steps of the Rayleigh-Taylor case
+// against eta tiles of 4 x 64: 128 x 512 2.44 -> 2.19 ms, 256 x 1024 3.20 -> 3.15, 512 x 2048 4.52 -> 4.44
+// (xi 64 x 1: 2.73, 3.13 and 4.36; eta 8 x 32: 2.15, 3.19 and 4.53).
+constexpr int kCXTX = 32, kCXTY = 4;
+constexpr int kCETX = 4, kCETY = 32;
+// AdaWENO sweeps: blocks of 128 threads, 64 interfaces x 2 rows in xi and 8 columns x 16 interfaces
+// in eta. A block waits at its barriers for the characteristic items of its own interfaces, so
+// small blocks lose less to an uneven queue, and 16-interface columns fill 481 interfaces to 97 %.
+// Time of the steps of double Mach reflections, against blocks of 256 (below): 640 x 160 2.33 ->
+// 2.15 ms, 960 x 240 3.67 -> 3.41, 1280 x 320 2.41 -> 2.06, 1920 x 480 4.48 -> 3.96; with xi 128 x 1
+// 3.97 for the last, with eta 4 x 32 4.12, 16 x 8 4.04, 8 x 8 4.11, 8 x 32 4.22.
+constexpr int kAXTX = 64, kAXTY = 2;
+constexpr int kAETX = 8, kAETY = 16;
+// Grids too small to fill the GPU with those (under 80,000 cells) finish with their longest block,
+// and take one row of 256 threads (251 interfaces, 256 cells) in xi, 2 columns of 128 (123
+// interfaces each) in eta: every thread stages one cell. 240 x 60 2.04 against 2.24 ms, 480 x 120 1.62
+// against 1.63.
+constexpr int kASXTX = 256, kASXTY = 1;
+constexpr int kASETX = 2, kASETY = 128;
+static inline bool adaptive_small(const Params& p) {
+    // (branch counts are per warp of the small-grid shapes, on every grid)
+    return (long long)p.ni * p.nj < kAdaptiveSmall || p.count_branches;
+}
 
 static inline dim3 grid_xi(const Params& p, int tx, int ty) {
     return dim3((p.ni + 1 + tx - 1) / tx, (p.nj + ty - 1) / ty);
@@ -1746,28 +1761,35 @@ static void cw_launch(dim3 g, const Params& p, int irk, cudaStream_t s) {
     k_flux_cw<DIR, SPL, REC, TX, TY, TAPE, TZ><<<g, dim3(TX, TY, TZ), CwTile<DIR, REC, TX, TY>::bytes, s>>>(p, irk);
 }
 
-// On small grids the standard tiles give a sweep only one or two blocks per SM, and the SMs that
-// get one more block than the others set the launch's time. Below four blocks per SM the sweep
-// runs with shorter tiles, which multiplies the block count, and with four threads per
-// interface (one per component: four times the warps to hide the dependent FP64 chains of a
-// sweep that is only one wave deep); same arithmetic per interface, so the results do not
-// depend on the tile. Measured on the 200 x 200 vortex: 1.925e8 -> 1.976e8 cell-updates/s for
-// the four threads; on 512 x 512 and larger grids the standard tiles gain nothing from them. The
-// adjoint's taping sweeps likewise: a 122 x 175 WENO-Z adjoint 1607 -> 1387 us, 256 x 256 WENO-JS
-// 7.26 -> 7.05 ms (two threads: 1450 us and 6.94 ms).
+// On small grids the standard tiles give a sweep only a few blocks per SM, and the SMs that get one
+// more block than the others set the launch's time. There the sweeps run with four threads per
+// interface (one per component: four times the warps to hide the dependent chains of a sweep that
+// is only one wave deep) on smaller tiles; same arithmetic per interface, so the results do not
+// depend on the tile. The line lies at 850 cells per SM, for Steger-Warming's split, of which the
+// smaller tiles do more, at 440: steps (small against standard tiles) of LLF + WENO-JS vortices 262 x 262
+// 1.28 and 1.44 ms, 320 x 320 1.69 and 1.77, 350 x 350 1.87 and 1.93, 380 x 380 2.15 and 2.11;
+// Steger-Warming 260 x 260 1.87 and 1.85, 300 x 300 2.30 and 2.12. Both sweeps of a stage switch
+// together: they run side by side, and one of each kind took 1.48 ms at 256 x 256 (1.23 and 1.34). The
+// adjoint's taping sweeps likewise: 122 x 175 WENO-Z adjoint 1607 -> 1387 us with four threads (two:
+// 1450), 320 x 320 WENO-JS 5.16 -> 5.08 ms, 400 x 400 7.33 and 7.36.
 constexpr int kSmallTZ = 4;
 template <int SPL, int REC, bool TAPE = false>
 static void launch_cw(const Params& p, int irk, int dir, cudaStream_t s) {
-    const unsigned few = 4u * sm_count();
+    const bool small = (long long)p.ni * p.nj < (SPL ? 440LL : 850LL) * sm_count();
     if (dir == 0) {
-        const dim3 g = grid_xi(p, kXTX, kXTY);
-        if (g.x * g.y < few) cw_launch<0, SPL, REC, kXTX, kXSTY, TAPE, kSmallTZ>(grid_xi(p, kXTX, kXSTY), p, irk, s);
-        else                 cw_launch<0, SPL, REC, kXTX, kXTY, TAPE>(g, p, irk, s);
+        if (small) cw_launch<0, SPL, REC, kXSTX, kXSTY, TAPE, kSmallTZ>(grid_xi(p, kXSTX, kXSTY), p, irk, s);
+        else       cw_launch<0, SPL, REC, kXTX, kXTY, TAPE>(grid_xi(p, kXTX, kXTY), p, irk, s);
     } else {
-        const dim3 g = grid_eta(p, kETX, kETY);
-        if (g.x * g.y < few) cw_launch<1, SPL, REC, kETX, kESTY, TAPE, kSmallTZ>(grid_eta(p, kETX, kESTY), p, irk, s);
-        else                 cw_launch<1, SPL, REC, kETX, kETY, TAPE>(g, p, irk, s);
+        if (small) cw_launch<1, SPL, REC, kESTX, kESTY, TAPE, kSmallTZ>(grid_eta(p, kESTX, kESTY), p, irk, s);
+        else       cw_launch<1, SPL, REC, kETX, kETY, TAPE>(grid_eta(p, kETX, kETY), p, irk, s);
     }
+}
+
+template <int DIR, bool ADAPT, int TX, int TY>
+static void launch_char(const Params& p, int irk, cudaStream_t s) {
+    using L = CharTile<DIR, ADAPT, TX, TY>;
+    const dim3 g = DIR == 0 ? grid_xi(p, L::KW, TY) : grid_eta(p, TX, L::KW);
+    k_flux_char<DIR, ADAPT, TX, TY><<<g, dim3(TX, TY), L::bytes, s>>>(p, irk);
 }
 
 static bool recon_known(int r) {
@@ -1786,12 +1808,11 @@ static void launch_flux(const Params& p, int irk, int dir, void* stream) {
         break;
     }
     case DENSE_SPLIT_CH:
-        if (dir == 0) k_flux_char<0, false, kXTX, kXTY><<<grid_xi(p, kXTX, kXTY), dim3(kXTX, kXTY), CharTile<0, false, kXTX, kXTY>::bytes, s>>>(p, irk);
-        else          k_flux_char<1, false, kCETX, kCETY><<<grid_eta(p, kCETX, CharTile<1, false, kCETX, kCETY>::KW), dim3(kCETX, kCETY), CharTile<1, false, kCETX, kCETY>::bytes, s>>>(p, irk);
+        dir == 0 ? launch_char<0, false, kCXTX, kCXTY>(p, irk, s) : launch_char<1, false, kCETX, kCETY>(p, irk, s);
         break;
     case DENSE_SPLIT_SC:
-        if (dir == 0) k_flux_char<0, true, kCXTX, kCXTY><<<grid_xi(p, CharTile<0, true, kCXTX, kCXTY>::KW, kCXTY), dim3(kCXTX, kCXTY), CharTile<0, true, kCXTX, kCXTY>::bytes, s>>>(p, irk);
-        else          k_flux_char<1, true, kAETX, kAETY><<<grid_eta(p, kAETX, CharTile<1, true, kAETX, kAETY>::KW), dim3(kAETX, kAETY), CharTile<1, true, kAETX, kAETY>::bytes, s>>>(p, irk);
+        if (adaptive_small(p)) dir == 0 ? launch_char<0, true, kASXTX, kASXTY>(p, irk, s) : launch_char<1, true, kASETX, kASETY>(p, irk, s);
+        else                   dir == 0 ? launch_char<0, true, kAXTX, kAXTY>(p, irk, s) : launch_char<1, true, kAETX, kAETY>(p, irk, s);
         break;
     default:
         break;
@@ -1901,11 +1922,11 @@ static void batch_flux(const BatchLaunch& b, int irk, int dir, void* stream) {
         break;  // unknown reconstruction: rejected when the batch is created
     }
     case DENSE_SPLIT_CH:
-        if (dir == 0) kb_flux_char<0, false, kXTX, kXTY><<<b.nb_xi, dim3(kXTX, kXTY), CharTile<0, false, kXTX, kXTY>::bytes, s>>>(b.tab, as_map(b.map_xi), irk);
+        if (dir == 0) kb_flux_char<0, false, kCXTX, kCXTY><<<b.nb_xi, dim3(kCXTX, kCXTY), CharTile<0, false, kCXTX, kCXTY>::bytes, s>>>(b.tab, as_map(b.map_xi), irk);
         else          kb_flux_char<1, false, kCETX, kCETY><<<b.nb_eta, dim3(kCETX, kCETY), CharTile<1, false, kCETX, kCETY>::bytes, s>>>(b.tab, as_map(b.map_eta), irk);
         break;
     case DENSE_SPLIT_SC:
-        if (dir == 0) kb_flux_char<0, true, kCXTX, kCXTY><<<b.nb_xi, dim3(kCXTX, kCXTY), CharTile<0, true, kCXTX, kCXTY>::bytes, s>>>(b.tab, as_map(b.map_xi), irk);
+        if (dir == 0) kb_flux_char<0, true, kAXTX, kAXTY><<<b.nb_xi, dim3(kAXTX, kAXTY), CharTile<0, true, kAXTX, kAXTY>::bytes, s>>>(b.tab, as_map(b.map_xi), irk);
         else          kb_flux_char<1, true, kAETX, kAETY><<<b.nb_eta, dim3(kAETX, kAETY), CharTile<1, true, kAETX, kAETY>::bytes, s>>>(b.tab, as_map(b.map_eta), irk);
         break;
     default:
@@ -2006,14 +2027,14 @@ static void allow_smem(K kernel, size_t bytes) {
 template <int SPL, int REC>
 static void allow_cw_smem() {
     allow_smem(k_flux_cw<0, SPL, REC, kXTX, kXTY>, CwTile<0, REC, kXTX, kXTY>::bytes);
-    allow_smem(k_flux_cw<0, SPL, REC, kXTX, kXSTY, false, kSmallTZ>, CwTile<0, REC, kXTX, kXSTY>::bytes);
+    allow_smem(k_flux_cw<0, SPL, REC, kXSTX, kXSTY, false, kSmallTZ>, CwTile<0, REC, kXSTX, kXSTY>::bytes);
     allow_smem(k_flux_cw<1, SPL, REC, kETX, kETY>, CwTile<1, REC, kETX, kETY>::bytes);
-    allow_smem(k_flux_cw<1, SPL, REC, kETX, kESTY, false, kSmallTZ>, CwTile<1, REC, kETX, kESTY>::bytes);
+    allow_smem(k_flux_cw<1, SPL, REC, kESTX, kESTY, false, kSmallTZ>, CwTile<1, REC, kESTX, kESTY>::bytes);
     // the adjoint's taping sweeps
     allow_smem(k_flux_cw<0, SPL, REC, kXTX, kXTY, true>, CwTile<0, REC, kXTX, kXTY>::bytes);
-    allow_smem(k_flux_cw<0, SPL, REC, kXTX, kXSTY, true, kSmallTZ>, CwTile<0, REC, kXTX, kXSTY>::bytes);
+    allow_smem(k_flux_cw<0, SPL, REC, kXSTX, kXSTY, true, kSmallTZ>, CwTile<0, REC, kXSTX, kXSTY>::bytes);
     allow_smem(k_flux_cw<1, SPL, REC, kETX, kETY, true>, CwTile<1, REC, kETX, kETY>::bytes);
-    allow_smem(k_flux_cw<1, SPL, REC, kETX, kESTY, true, kSmallTZ>, CwTile<1, REC, kETX, kESTY>::bytes);
+    allow_smem(k_flux_cw<1, SPL, REC, kESTX, kESTY, true, kSmallTZ>, CwTile<1, REC, kESTX, kESTY>::bytes);
     // the batched tile variants of batch_cw_variant
     allow_smem(kb_flux_cw<0, SPL, REC, 32, 4>, CwTile<0, REC, 32, 4>::bytes);
     allow_smem(kb_flux_cw<0, SPL, REC, 64, 2>, CwTile<0, REC, 64, 2>::bytes);
@@ -2032,13 +2053,15 @@ static bool allow_tile_smem() {
     allow_cw_smem<1, 253>();
     allow_cw_smem<0, 255>();
     allow_cw_smem<1, 255>();
-    allow_smem(k_flux_char<0, false, kXTX, kXTY>, CharTile<0, false, kXTX, kXTY>::bytes);
+    allow_smem(k_flux_char<0, false, kCXTX, kCXTY>, CharTile<0, false, kCXTX, kCXTY>::bytes);
     allow_smem(k_flux_char<1, false, kCETX, kCETY>, CharTile<1, false, kCETX, kCETY>::bytes);
-    allow_smem(k_flux_char<0, true, kCXTX, kCXTY>, CharTile<0, true, kCXTX, kCXTY>::bytes);
+    allow_smem(k_flux_char<0, true, kASXTX, kASXTY>, CharTile<0, true, kASXTX, kASXTY>::bytes);
+    allow_smem(k_flux_char<1, true, kASETX, kASETY>, CharTile<1, true, kASETX, kASETY>::bytes);
+    allow_smem(k_flux_char<0, true, kAXTX, kAXTY>, CharTile<0, true, kAXTX, kAXTY>::bytes);
     allow_smem(k_flux_char<1, true, kAETX, kAETY>, CharTile<1, true, kAETX, kAETY>::bytes);
-    allow_smem(kb_flux_char<0, false, kXTX, kXTY>, CharTile<0, false, kXTX, kXTY>::bytes);
+    allow_smem(kb_flux_char<0, false, kCXTX, kCXTY>, CharTile<0, false, kCXTX, kCXTY>::bytes);
     allow_smem(kb_flux_char<1, false, kCETX, kCETY>, CharTile<1, false, kCETX, kCETY>::bytes);
-    allow_smem(kb_flux_char<0, true, kCXTX, kCXTY>, CharTile<0, true, kCXTX, kCXTY>::bytes);
+    allow_smem(kb_flux_char<0, true, kAXTX, kAXTY>, CharTile<0, true, kAXTX, kAXTY>::bytes);
     allow_smem(kb_flux_char<1, true, kAETX, kAETY>, CharTile<1, true, kAETX, kAETY>::bytes);
     return true;
 }
@@ -2073,12 +2096,11 @@ const BatchKernelTable* batch_kernels_fast() {
 // Tile shapes of the batched sweeps (the shapes instantiated above).
 void batch_tile_shape(int splitting, int dir, int variant, int* tx, int* ty) {
     if (splitting == DENSE_SPLIT_CH || splitting == DENSE_SPLIT_SC) {
-        // xi: 32 x 4 for 104, one row of 251 interfaces (256 threads) for AdaWENO; eta: 4 x 64
-        // for 104, 2 columns of 123 interfaces (256 threads) for AdaWENO
+        // xi: 32 x 4 for 104, 64 x 2 for AdaWENO; eta: 4 x 32 for 104, 8 x 16 for AdaWENO
         const bool sc = splitting == DENSE_SPLIT_SC;
-        *tx = dir == 0 ? (sc ? VNS::CharTile<0, true, VNS::kCXTX, VNS::kCXTY>::KW : VNS::kXTX)
+        *tx = dir == 0 ? (sc ? VNS::CharTile<0, true, VNS::kAXTX, VNS::kAXTY>::KW : VNS::kCXTX)
                        : (sc ? VNS::kAETX : VNS::kCETX);
-        *ty = dir == 0 ? (sc ? VNS::kCXTY : VNS::kXTY)
+        *ty = dir == 0 ? (sc ? VNS::kAXTY : VNS::kCXTY)
                        : (sc ? VNS::CharTile<1, true, VNS::kAETX, VNS::kAETY>::KW
                              : VNS::CharTile<1, false, VNS::kCETX, VNS::kCETY>::KW);
         return;
