@@ -20,13 +20,15 @@
 // checkpoint, the flux sweeps run in their taping form (flux_tape of the kernel table), which
 // writes, per face, the gradient g[m] = dW/dlf[m] of each of its 8 reconstructions and the
 // fluxes h -- 352 bytes per face and direction, read back once. The vector-Jacobian product
-// v -> (dL/du)^T v of a stage is then two light kernels:
+// v -> (dL/du)^T v of a stage is then light:
 //   k_hbar (one thread per face, both directions): hbar_f = (v_right - v_left)/dx, and the
 //     face's share h_f . hbar_f of v . L(u) (summation by parts), summed per block;
-//   k_rev (one thread per cell): for every face whose stencils read the cell or one of its
-//     periodic images, hbar_f g[m] accumulated in a fixed order into the sensitivities of the
-//     cell's F+ and F-; the transposed Jacobian of F+- at the cell (both directions); the
-//     reverse of the RK stage;
+//   k_char_face (104 and 105, one launch for both directions): the characteristic faces' gradients;
+//   k_wall (grids with walls): the sensitivities of the ghosts' split fluxes, per ghost;
+//   k_rev (two threads per cell, one per direction): for every face whose stencils read the cell or
+//     one of its periodic images, hbar_f g[m] accumulated in a fixed order into the sensitivities
+//     of the cell's F+ and F-; the transposed Jacobian of F+- at the cell; the reverse of the RK
+//     stage;
 // and once per step k_dt (one block): the time step's sensitivity sum_s c_s v_s . L(u_{s-1}),
 // sent through dt(max wave speeds) to the cells where the maxima are attained.
 // GLF (flux_splitting_GLF.f90:13-70) splits with the stage's global lambda = max over the cells

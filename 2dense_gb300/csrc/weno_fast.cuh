@@ -1,6 +1,7 @@
-// weno_fast.cuh -- the WENO-JS5 / WENO-Z5 reconstruction terms of the fast kernels and their
-// stencil gradient, shared by the sweeps (kernels.cu) and the discrete adjoint's face-level
-// reverse (adjoint.cu). Included inside each file's own namespace (both see dense::fx).
+// weno_fast.cuh -- the WENO-JS5 / WENO-Z5 reconstruction terms in FP64 and their stencil gradient:
+// for the taping sweeps' stencils that the integer form (weno_fixed.cuh) leaves to FP64, AdaWENO's
+// indicator (kernels.cu) and the discrete adjoint's face-level reverse (adjoint.cu). Included inside
+// each file's own namespace (both see dense::fx).
 #pragma once
 
 // weno module constants (source/inv_scheme/weno_mod.f90:3-14,37)
@@ -10,7 +11,7 @@ constexpr double a320 = 1.0 / 3.0, a321 = 5.0 / 6.0, a322 = -1.0 / 6.0;
 constexpr double c30 = 0.1, c31 = 0.6, c32 = 0.3;
 constexpr double kSS = (double)1.0e-6f;       // ss = 1.0e-6, a default-real literal (:37)
 
-// The fast WENO reconstructions work from a stencil's centre value lf[2] and its first
+// The reconstructions work from a stencil's centre value lf[2] and its first
 // differences g_m = lf[m] - lf[m+1] (m = 0..3): the indicators' second differences A_k =
 // g_k - g_{k+1} and first-order combinations B_0 = g_0 - 3 g_1, B_1 = g_1 + g_2, B_2 = 3 g_2 - g_3,
 // and the candidates relative to the centre, q_0 - lf2 = g_0/3 - 5 g_1/6, q_1 - lf2 = -g_1/6 -
@@ -59,20 +60,6 @@ __device__ __forceinline__ void weno_terms(const double g[4], double d0, double 
 __device__ __forceinline__ double weno_num(const WenoTerms& t) {
     return fma(t.v[2], t.r[2], fma(t.v[1], t.r[1], t.v[0] * t.r[0]));
 }
-// h = lf2 + sum_k v_k r_k / N with iN = 1/N. Every operation is an explicit FMA or a product
-// feeding one, so no kernel contracts it differently from another (the plain and taping sweeps
-// agree bit for bit).
-__device__ __forceinline__ double weno_value(const WenoTerms& t, double iN, double lf2) {
-    return fma(weno_num(t), iN, lf2);
-}
-// WENO reconstruction from its centre value, first differences and d_k.
-template <bool Z>
-__device__ __forceinline__ double weno_from_d(double lf2, const double g[4], double d0, double d1, double d2) {
-    WenoTerms t;
-    weno_terms<Z>(g, d0, d1, d2, t);
-    return weno_value(t, fx::rcp(t.N), lf2);
-}
-
 // Gradient of the WENO reconstruction with respect to its stencil, g[m] = dW/dlf[m], for the
 // discrete adjoint's tape. W = sum_k w_k q_k with w_k = a_k / sum(a): dW/dq_k = w_k and
 // dW/da_k = (q_k - W)/sum(a); a_k depends on lf through beta_k (JS: a_k = c_k/d_k^2, so

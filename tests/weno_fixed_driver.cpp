@@ -18,7 +18,9 @@ static double rcp(double d) { return 1.0 / d; }
 template <bool Z> double recon(double lf2, const double g[4]) {
     double d0, d1, d2, B[3];
     betas_g(g, d0, d1, d2, B);
-    return weno_from_d<Z>(lf2, g, d0, d1, d2);
+    WenoTerms t;
+    weno_terms<Z>(g, d0, d1, d2, t);
+    return fma(weno_num(t), fx::rcp(t.N), lf2);
 }
 }  // namespace f64
 
