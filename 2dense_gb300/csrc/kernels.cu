@@ -1476,7 +1476,7 @@ constexpr int char_min_blocks(bool adapt, int nt) { return adapt ? 768 / nt : 10
 template <int DIR, int SPL, int REC, int TX, int TY, bool TAPE = false, int TZ = 1>
 __global__ void __launch_bounds__(TX* TY* TZ) k_flux_cw(Params p, int irk) {
     grid_dependency_wait();
-    flux_cw_block<DIR, SPL, REC, TX, TY, TAPE, TZ>(p, irk, blockIdx.x, blockIdx.y);
+    flux_cw_block<DIR, SPL, REC, TX, TY, TAPE, TZ>(p, irk, blockIdx.x, blockIdx.y + gridDim.y * blockIdx.z);
 }
 template <int DIR, bool ADAPT, int TX, int TY>
 __global__ void __launch_bounds__(TX* TY, char_min_blocks(ADAPT, TX* TY)) k_flux_char(Params p, int irk) {
@@ -1758,6 +1758,8 @@ static int sm_count() {
 // A component-wise sweep on its tile's dynamic shared memory.
 template <int DIR, int SPL, int REC, int TX, int TY, bool TAPE = false, int TZ = 1>
 static void cw_launch(dim3 g, const Params& p, int irk, cudaStream_t s) {
+    const unsigned gz = (g.y + 65534u) / 65535u;  // (a grid's y is 65,535 blocks at most)
+    g = dim3(g.x, (g.y + gz - 1) / gz, gz);
     k_flux_cw<DIR, SPL, REC, TX, TY, TAPE, TZ><<<g, dim3(TX, TY, TZ), CwTile<DIR, REC, TX, TY>::bytes, s>>>(p, irk);
 }
 

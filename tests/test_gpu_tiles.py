@@ -16,6 +16,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("split,recon,sizes", [
     (101, 253, [(359, 359), (360, 360), (383, 351), (321, 415)]),
     (102, 255, [(383, 352), (320, 407)]),
+    (101, 253, [(16, 131075)]),  # more rows of tiles than a grid's y holds
     (103, 255, [(258, 258), (260, 258), (319, 287)]),
 ])
 def test_component_wise_tiles(dense, split, recon, sizes):
