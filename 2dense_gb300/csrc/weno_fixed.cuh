@@ -17,11 +17,8 @@
 //   6 (h - lf_2) = -(g_1 + 2 g_2) + 2 w_0 (A_0 - A_1) + w_2 (A_1 - A_2).
 // The representation:
 //  * the first differences become fixed-point integers of one exponent for the stencils of a face
-//    value, below 2^58: their sums and differences are exact. The exponent is the largest
-//    difference's, but at most kCap above that of the smoothest substencil (of sqrt(ss), where that
-//    is more): past a jump of 2^kCap times the rest, the weights leave 2^-3kCap of the rest to the
-//    substencils that contain it, whatever it is, so it may as well be clipped, and the rest keeps
-//    57 - kCap bits or more beside any jump;
+//    value, that of the largest one, below 2^58: their sums and differences are exact (a large
+//    difference cannot be clipped: two clipped ones would look alike to WENO-Z's tau);
 //  * the indicators 3 d_k = 12 ss + 13 A_k^2 + 3 B_k^2 and everything made of them are positive
 //    floating-point numbers of a 64-bit mantissa and an integer exponent, whose products need
 //    no normalising between them; the weights' common denominators are those of weno_terms;
@@ -46,19 +43,20 @@ constexpr u32 kExpMask = 0x7ff00000u;
 constexpr u32 kExpMin = 200u << 20;   // differences below 2^-882 count as zero
 constexpr u32 kExpSS = 1014u << 20;   // of sqrt(4 ss) = 2^-9
 constexpr u32 kExpMax = 2000u << 20;  // NaN, infinity, or so large that the result is NaN too
-constexpr u32 kCap = 15u;
 DENSE_FX u32 exponent(double g) { return hi32(bits(g)) & kExpMask; }
+// The largest exponent of a stencil's differences.
+DENSE_FX u32 exponent_of(const double g[4]) {
+    return umax(umax(exponent(g[0]), exponent(g[1])), umax(exponent(g[2]), exponent(g[3])));
+}
 // The fixed-point exponent E, in place, of a stencil's differences; top: at least the largest one's.
 DENSE_FX u32 scale_of(const double g[4], u32& top) {
-    const u32 e1 = exponent(g[1]), e2 = exponent(g[2]);
-    const u32 m0 = umax(exponent(g[0]), e1), m1 = umax(e1, e2), m2 = umax(e2, exponent(g[3]));
-    const u32 most = umax(m0, m2), least = umin(umin(m0, m1), m2);
+    const u32 most = exponent_of(g);
     top = umax(top, most);
-    return umax(umin(most, umax(least, kExpSS) + (kCap << 20)), kExpMin);
+    return umax(most, kExpMin);
 }
 
-// A double as a fixed-point integer in units of 2^(E - 1080) (E in place in eh): below 2^58,
-// truncated; a larger one clipped to E.
+// A double as a fixed-point integer in units of 2^(E - 1080) (E in place in eh, at least the
+// double's): below 2^58, truncated. (A larger one comes out clipped.)
 DENSE_FX i64 to_fixed(double g, u32 eh) {
     const u64 b = bits(g);
     const u32 h = hi32(b);
@@ -362,15 +360,11 @@ DENSE_FX bool surrogate(const double g[4], double theta_c, u64& f0, u64& f2) {
     return smooth && top < kExpMax;
 }
 // 6 (h - lf_2) of another stencil by a surrogate's weights, in units of 2^(E - 1080), E at least
-// the exponent of its differences (the weights are not its own: nothing is clipped).
+// the exponent of its differences.
 DENSE_FX i64 correction6_by(const double g[4], u32 eh, u64 f0, u64 f2) {
     const i64 G1 = to_fixed(g[1], eh), G2 = to_fixed(g[2], eh);
     const i64 A0 = to_fixed(g[0], eh) - G1, A1 = G1 - G2, A2 = G2 - to_fixed(g[3], eh);
     return scaled(f0, (A0 - A1) * 4) + scaled(f2, (A1 - A2) * 4) - G1 - 2 * G2;
-}
-// The largest exponent of a stencil's differences.
-DENSE_FX u32 exponent_of(const double g[4]) {
-    return umax(umax(exponent(g[0]), exponent(g[1])), umax(exponent(g[2]), exponent(g[3])));
 }
 
 // dt/dx and dt/dy as fixed-point factors of one exponent, below 2^62 (in units of 2^-shift), and
