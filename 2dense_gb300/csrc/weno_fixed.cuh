@@ -8,8 +8,10 @@
 // to the split fluxes of other warps. The component-wise xi sweep of a 2048 x 2048 LLF stage went
 // from 2.414 to 0.684 ms (JS) and from 2.773 to 0.778 ms (Z), the eta sweep from 2.301 to 0.663 and
 // from 2.657 to 0.772 ms; what bounds them now is the integer ALU (72 % busy, 340 instructions a
-// reconstruction before its last trimming). Nothing is computed in fewer bits than before: the
-// words carry 57 to 64 significant bits where a double carries 53.
+// reconstruction before its last trimming). The words carry 57 to
+// 64 significant bits where a double carries 53, but counted from a stencil's largest difference; on
+// the small side of a jump, where that says too little, FP64 takes over (enough, weno_value.cuh: 1 to
+// 2 % of the time of a step, the test above all).
 //
 // The value. With g_m = lf_m - lf_(m+1), A_k = g_k - g_(k+1), B_0 = A_0 - 2 g_1, B_1 = g_1 + g_2,
 // B_2 = A_2 + 2 g_2 and d_k = 4 (ss + beta_k) = 4 ss + 13/3 A_k^2 + B_k^2 (weno_fast.cuh), the
@@ -29,7 +31,7 @@
 //    sign of the result and nothing else: mirror-symmetric flows stay so bit for bit.
 // A NaN or infinity among the differences gives NaN. Against long double over random smooth,
 // discontinuous and rough stencils the error's rms is 0.57 to 0.86 of the FP64 form's, its maximum
-// 0.58 to 1.0.
+// 0.58 to 1.0; relative to the small side of a jump, where FP64 takes over, 0.6 to 1.0 and 0.6 to 1.1.
 //
 // The functions compile for the host too, where the tests compare them with long double.
 #pragma once
@@ -47,6 +49,15 @@ DENSE_FX u32 exponent(double g) { return hi32(bits(g)) & kExpMask; }
 // The largest exponent of a stencil's differences.
 DENSE_FX u32 exponent_of(const double g[4]) {
     return umax(umax(exponent(g[0]), exponent(g[1])), umax(exponent(g[2]), exponent(g[3])));
+}
+// The largest exponent of its smoothest substencil's two.
+DENSE_FX u32 smoothest_of(const double g[4]) {
+    const u32 e1 = exponent(g[1]), e2 = exponent(g[2]);
+    return umin(umin(umax(exponent(g[0]), e1), umax(e1, e2)), umax(e2, exponent(g[3])));
+}
+// The exponent of what the rounding of a sum of two reconstructions is relative to (enough).
+DENSE_FX u32 size_of(double lp, const double gp[4], double lm, const double gm[4]) {
+    return umax(umax(exponent(lp), exponent(lm)), umax(smoothest_of(gp), smoothest_of(gm)) + (1u << 20));
 }
 // The fixed-point exponent E, in place, of a stencil's differences; top: at least the largest one's.
 DENSE_FX u32 scale_of(const double g[4], u32& top) {
@@ -304,21 +315,45 @@ DENSE_FX void gradient_out(const Gradient& q, u32 top, double g[5]) {
     for (int m = 0; m < 5; ++m) g[m] = to_double(q.g[m], 1025u << 20, top) * (1.0 / 6.0);
 }
 
+// Whether lp is the smaller one in magnitude (of two opposite ones, the positive).
+DENSE_FX bool smaller(double lp, double lm) {
+    const u64 ap = bits(lp) << 1, am = bits(lm) << 1;          // (an FP64 absolute value would take that pipe)
+    return ap < am || (ap == am && (i64)bits(lp) >= 0);
+}
 // lp + lm + c/6, c on the smaller one first: the two FP64 roundings are no larger than those of two
 // values and their sum, and the same in either order.
 DENSE_FX double about(double lp, double lm, double c) {
-    const u64 ap = bits(lp) << 1, am = bits(lm) << 1;          // (an FP64 absolute value would take that pipe)
-    const bool first = ap < am || (ap == am && (i64)bits(lp) >= 0);  // of two opposite ones, the positive
+    const bool first = smaller(lp, lm);
     return fma(c, 1.0 / 6.0, first ? lp : lm) + (first ? lm : lp);
+}
+// Whether about(lp, lm, c) is to be computed in FP64 instead: the exponent, in place, that c has to reach
+// for the integer form, 0 where any will do. c is of the unit eh, top the largest exponent of the
+// differences, size that of what the value's rounding is relative to: lp, lm and twice the smoothest
+// substencil (smoothest_of, of either stencil). Past the value's own rounding the integer form is good
+// to a few of its units, which are 2^-57 of the largest difference, FP64 to 2^-53 of the values and
+// of the corrections, which are no smaller than the smoothest substencils' differences but by
+// chance. So where the largest difference lies binades above all of these -- on the small side
+// of a jump, of either stencil -- FP64 is more exact. (Above 2^72 its products would overflow;
+// from kExpMax on the result is NaN.)
+constexpr u32 kExpFP64 = 1095u << 20;
+DENSE_FX u32 enough(u32 eh, u32 top, u32 size) {
+    u32 n = eh > size && top != 0 && top <= kExpFP64 ? eh : 0u;
+#ifdef __CUDA_ARCH__
+    asm volatile("" : "+r"(n));  // formed here, not after the corrections with its inputs kept in registers
+#endif
+    return n;
 }
 // The sum of two reconstructions about lp and lm, whose corrections share their exponent and the
 // conversion back. gm: the second's differences with the opposite sign, as a sweep has them (a
-// correction is odd in its differences, to the bit; negating doubles would take the FP64 pipe).
+// correction is odd in its differences, to the bit; negating doubles would take the FP64 pipe). fp64:
+// takes whether it is to be computed in FP64 instead.
 template <bool Z>
-DENSE_FX double pair(double lp, const double gp[4], double lm, const double gm[4]) {
+DENSE_FX double pair(double lp, const double gp[4], double lm, const double gm[4], bool* fp64 = nullptr) {
     u32 top = 0;
     const u32 ep = scale_of(gp, top), eh = umax(ep, scale_of(gm, top));
+    const u32 need = fp64 ? enough(eh, top, size_of(lp, gp, lm, gm)) : 0u;
     const double c = to_double(correction6<Z>(gp, eh) - correction6<Z>(gm, eh), eh, top);
+    if (fp64) *fp64 = exponent(c) < need;
     return about(lp, lm, c);
 }
 // Whether a stencil's largest difference is more than 2^kRough times its smoothest substencil's (or

@@ -1,0 +1,47 @@
+"""The fast sweeps on the small side of a jump: a gas 1e8 times as thin beside a dense one at the same
+temperature (and so of the same wave speeds), whose faces two and three cells from the jump have it in
+their stencils. The right-hand side there, fast against strict, relative to the thin side: each face flux
+is some fifty roundings of that size, so 1e-13."""
+import importlib
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+THIN = 1e-8
+
+
+def state(c, axis):
+    """Dense in the first half along the axis, thin in the second; smooth variations of a few percent."""
+    X, Y = np.meshgrid(np.arange(c.ni + 8) - 4 + 0.5, np.arange(c.nj + 8) - 4 + 0.5, indexing="ij")
+    k = 2 * np.pi / np.array([c.ni, c.nj])
+    rho = 1 + 0.05 * np.sin(k[0] * X) * np.cos(k[1] * Y)
+    u, v = 0.4 + 0.1 * np.cos(k[0] * X + k[1] * Y), -0.3 + 0.1 * np.sin(2 * k[0] * X - k[1] * Y)
+    p = 1 + 0.04 * np.cos(k[0] * X - k[1] * Y)
+    thin = np.where((X if axis == 0 else Y) % (c.ni if axis == 0 else c.nj) < (c.ni if axis == 0 else c.nj) // 2, 1.0, THIN)
+    rho, p = rho * thin, p * thin
+    cons = np.zeros(rho.shape + (4,), order="F")
+    cons[..., 0], cons[..., 1], cons[..., 2] = rho, rho * u, rho * v
+    cons[..., 3] = p / (c.gamma - 1.0) + 0.5 * rho * (u * u + v * v)
+    return cons
+
+
+@pytest.mark.parametrize("n", [40, 400])  # the small grids' tiles and the others
+@pytest.mark.parametrize("axis", [0, 1])
+@pytest.mark.parametrize("split,recon", [(101, 253), (101, 255), (102, 255), (103, 253), (103, 255)])
+def test_thin_side(dense, split, recon, axis, n):
+    ops = importlib.import_module("2dense_gb300.torch_ops")
+    L, c = [], None
+    for strict in (1, 0):
+        c = dense.init_general(dense.config_default(ni=n, nj=n + 8, benchmark=11, splitting=split, recon=recon,
+                                                    cfl=0.5, strict=strict))[0]
+        u = ops.padded_state(state(c, axis))
+        L.append(torch.ops.dense2d.rhs(u, ops.config_tensor(c)).cpu().numpy())
+    m = n if axis == 0 else n + 8
+    rows = [m // 2 + 1, m // 2 + 2, m // 2 + 3, m - 4, m - 3, m - 2]
+    strict, fast = (np.take(x, rows, axis=2 if axis == 0 else 1) for x in L)
+    size = THIN * 3.0 / min(c.dx, c.dy)  # a thin-side flux over the cell's size
+    assert np.abs(strict).max() < 100 * size  # (the dense side is not in these)
+    assert np.abs(fast - strict).max() <= 1e-13 * size

@@ -1,4 +1,5 @@
-"""The reconstructions beside jumps (csrc/weno_fixed.cuh), compiled for the host, against long double."""
+"""The reconstructions beside jumps (csrc/weno_fixed.cuh, csrc/weno_value.cuh), compiled for the host,
+against long double."""
 import os
 import subprocess
 
@@ -23,3 +24,22 @@ def test_between_two_jumps(lines, z):
     ((worst, smooth),) = [x[2:] for x in lines if x[0] == "between" and x[1] == str(z)]
     assert float(worst) <= 16 * 2.0 ** -53
     assert int(smooth) == 0
+
+
+@pytest.mark.parametrize("decades", [-3, 0, 1, 2, 4, 6, 10, 14])
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("z", [0, 1])
+def test_small_side(lines, z, kind, decades):
+    """A face's value on the small side of a jump, relative to that side: as exact as in FP64 (the rms
+    over the same 20,000 stencils, whose scatter is 1 %; the worst of them to a factor of two)."""
+    ((rms, rms64, worst, worst64),) = [[float(v) for v in x[4:]] for x in lines
+                                       if x[0] == "sided" and x[1:4] == [str(z), str(kind), str(decades)]]
+    assert rms <= 1.02 * rms64
+    assert worst <= 2.0 * worst64
+
+
+@pytest.mark.parametrize("z", [0, 1])
+def test_forms(lines, z):
+    """Odd, the same in either order, and a flat stencil's centre, in both arithmetics."""
+    (row,) = [[int(v) for v in x[2:]] for x in lines if x[0] == "forms" and x[1] == str(z)]
+    assert row[:3] == [0, 0, 0] and row[3] > 10000
