@@ -487,7 +487,7 @@ struct CwTile {
 template <int DIR, int SPL, int REC, int TX, int TY, bool TAPE = false, int TZ = 1>
 __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, int by) {
     static_assert(TZ == 1 || TZ == 2 || TZ == 4, "TZ divides the four components");
-    static_assert(TX * TY * TZ % 32 == 0, "whole warps");
+    static_assert(TX * TY * TZ % 32 == 0 && TX * TY <= 16384, "whole warps, items of 16 bits");
     if (!p.sc->active) return;
     using L = CwTile<DIR, REC, TX, TY>;
     constexpr int NL = L::NL, NC = L::NC, NCELL = L::NCELL;
@@ -597,7 +597,7 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
                 // slots 0 "+" and 5 "-"; they are even in the differences)
                 fx::u32 top = 0;
                 const fx::u32 ep = fx::scale_of(gp, top), eh = fx::umax(ep, fx::scale_of(gm, top));
-                const fx::u32 need = fx::enough(eh, top, fx::size_of(lp, gp, lm, gm));
+                const fx::u32 need = fx::enough(top, fx::size_of(lp, gp, lm, gm));
                 fx::i64 c = 0;
 #pragma unroll 1
                 for (int s = 0; s < 2; ++s) {
@@ -644,28 +644,34 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
         if constexpr (TAPE) tape_at[(tape_planes(REC) - 4 + v) * ts] = h;
     }
     if constexpr (kStageG)
-        if (__any_sync(0xffffffffu, redo != 0)) {
-            // A warp's values left to FP64 (a handful of faces beside a jump, several components of
-            // each), two lanes a value, one a sign: each lane's in turn, they kept their block from
-            // ending (481 x 479 Steger-Warming xi sweep, 5 % of the warps: 0.067 -> 0.086 ms).
+        if (__syncthreads_or((int)redo)) {
+            // The block's values left to FP64 (a handful of faces beside a jump, several components
+            // of each), queued and then taken by the block's first warps, two lanes a value, one a sign.
+            // Each lane's in turn, they kept the block from ending (481 x 479 Steger-Warming xi
+            // sweep, 5 % of the warps: 0.067 -> 0.086 ms; so 0.068); each warp's by itself, they
+            // took the FP64 pipe for a few lanes (steps of 240 x 240 Steger-Warming 1.78 ms; so 1.70).
             constexpr bool Z = REC == DENSE_RECON_WENOZ5;
+            constexpr int NT = TX * TY * TZ;
+            __shared__ unsigned short items[4 * TX * TY];
+            __shared__ int count;
             const int lane = lt & 31, s = lane & 1;
-            unsigned m[4 / TZ];
-            int n = 0;
+            if (lt == 0) count = 0;
+            __syncthreads();
 #pragma unroll
             for (int vz = 0; vz < 4 / TZ; ++vz) {
-                m[vz] = __ballot_sync(0xffffffffu, redo >> vz & 1u);
-                n += __popc(m[vz]);
+                const unsigned m = __ballot_sync(0xffffffffu, redo >> vz & 1u);
+                if (!m) continue;
+                int base = 0;
+                if (lane == 0) base = atomicAdd(&count, __popc(m));
+                base = __shfl_sync(0xffffffffu, base, 0);
+                if (redo >> vz & 1u) items[base + __popc(m & ((1u << lane) - 1u))] = (unsigned short)((lt % (TX * TY)) * 4 + tz + vz * TZ);
             }
+            __syncthreads();
+            const int n = count;
 #pragma unroll 1
-            for (int q0 = 0; q0 < n; q0 += 16) {
-                int q = min(q0 + (lane >> 1), n - 1), vz = 0;
-                unsigned of = m[0];
-#pragma unroll
-                for (int k = 1; k < 4 / TZ; ++k)
-                    if (vz == k - 1 && q >= __popc(of)) { q -= __popc(of); of = m[k]; vz = k; }
-                const int other = (lt & ~31) + (int)__fns(of, 0, q + 1), v = tz + vz * TZ;
-                const int ox = other % TX, oy = (other / TX) % TY, ot = DIR == 0 ? ox : oy;
+            for (int q0 = (lt >> 5) * 16; q0 < n; q0 += NT / 2) {
+                const int it = items[min(q0 + (lane >> 1), n - 1)], v = it & 3, other = it >> 2;
+                const int ox = other % TX, oy = other / TX, ot = DIR == 0 ? ox : oy;
                 auto ato = [&](int k) { return DIR == 0 ? at(oy, k) : at(k, ox); };
                 double g[4];
 #pragma unroll
@@ -1521,8 +1527,10 @@ __device__ __forceinline__ void bc_block(const Params& p, int bx) {
 // unbounded 0.141 and 0.158 (now 0.106 and 0.098, the roots on the integer pipes too; 0.340 and
 // 0.293 with the reconstructions in FP64).
 constexpr int char_min_blocks(bool adapt, int nt) { return adapt ? 768 / nt : 1024 / nt; }
+// The four-thread tiles: five resident blocks (48 registers), which grids of a few blocks an SM need to
+// run as one wave (200 x 200 vortex, ten steps 0.927 -> 0.897 ms).
 template <int DIR, int SPL, int REC, int TX, int TY, bool TAPE = false, int TZ = 1>
-__global__ void __launch_bounds__(TX* TY* TZ) k_flux_cw(Params p, int irk) {
+__global__ void __launch_bounds__(TX* TY* TZ, TZ == 4 && !TAPE ? 5 : 0) k_flux_cw(Params p, int irk) {
     grid_dependency_wait();
     flux_cw_block<DIR, SPL, REC, TX, TY, TAPE, TZ>(p, irk, blockIdx.x, blockIdx.y + gridDim.y * blockIdx.z);
 }

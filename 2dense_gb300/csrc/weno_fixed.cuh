@@ -327,17 +327,17 @@ DENSE_FX double about(double lp, double lm, double c) {
     return fma(c, 1.0 / 6.0, first ? lp : lm) + (first ? lm : lp);
 }
 // Whether about(lp, lm, c) is to be computed in FP64 instead: the exponent, in place, that c has to reach
-// for the integer form, 0 where any will do. c is of the unit eh, top the largest exponent of the
-// differences, size that of what the value's rounding is relative to: lp, lm and twice the smoothest
-// substencil (smoothest_of, of either stencil). Past the value's own rounding the integer form is good
-// to a few of its units, which are 2^-57 of the largest difference, FP64 to 2^-53 of the values and
-// of the corrections, which are no smaller than the smoothest substencils' differences but by
-// chance. So where the largest difference lies binades above all of these -- on the small side
-// of a jump, of either stencil -- FP64 is more exact. (Above 2^72 its products would overflow;
-// from kExpMax on the result is NaN.)
+// for the integer form, 0 where any will do. top is the largest exponent of the differences, size
+// that of what the value's rounding is relative to: lp, lm and twice the smoothest substencil
+// (size_of). Past the value's own rounding the integer form is good to a few of its units, which are
+// 2^-57 of the largest difference, FP64 to 2^-53 of the values and of the corrections, which are
+// no smaller than the smoothest substencils' differences but by chance. So where the largest
+// difference is of a higher binade than all of these -- on the small side of a jump, of either
+// stencil -- FP64 is more exact. (Above 2^72 its products would overflow; from kExpMax on the
+// result is NaN.)
 constexpr u32 kExpFP64 = 1095u << 20;
-DENSE_FX u32 enough(u32 eh, u32 top, u32 size) {
-    u32 n = eh > size && top != 0 && top <= kExpFP64 ? eh : 0u;
+DENSE_FX u32 enough(u32 top, u32 size) {
+    u32 n = top > size && top <= kExpFP64 ? top : 0u;
 #ifdef __CUDA_ARCH__
     asm volatile("" : "+r"(n));  // formed here, not after the corrections with its inputs kept in registers
 #endif
@@ -351,7 +351,7 @@ template <bool Z>
 DENSE_FX double pair(double lp, const double gp[4], double lm, const double gm[4], bool* fp64 = nullptr) {
     u32 top = 0;
     const u32 ep = scale_of(gp, top), eh = umax(ep, scale_of(gm, top));
-    const u32 need = fp64 ? enough(eh, top, size_of(lp, gp, lm, gm)) : 0u;
+    const u32 need = fp64 ? enough(top, size_of(lp, gp, lm, gm)) : 0u;
     const double c = to_double(correction6<Z>(gp, eh) - correction6<Z>(gm, eh), eh, top);
     if (fp64) *fp64 = exponent(c) < need;
     return about(lp, lm, c);
