@@ -347,86 +347,7 @@ __device__ __forceinline__ void char_weno(const Eig& e, const double F[5][4], do
         h[q] = e.R[0][q] * cv[0] + e.R[1][q] * cv[1] + e.R[2][q] * cv[2] + e.R[3][q] * cv[3];
 }
 
-// FAST characteristic machinery. The Roe state of the two cells next to an interface from
-// their sqrt(rho) and total enthalpy H = gamma/(gamma-1) p/rho + |u|^2/2 (staged once per cell),
-// with one reciprocal for the three weighted means and one inverse square root giving both
-// alpha0 and 1/alpha0; 1/hh0 = (gamma-1)/alpha0^2. With n the normal and t the tangential momentum
-// component, the projection on the left eigenvectors of get_l_r_vec_xi/_eta
-// (scheme_weno5th_SC.f90:277-328, 607-658) is
-//   w = f_n - u_n0 f_0,  q = f_t - u_t0 f_0,  z = f_3 - uu0 f_0 - u_n0 w - u_t0 q,
-//   l_0 = z/(2 hh0) - w/(2 a0),  l_1 = f_0 - z/hh0,  l_2 = q,  l_3 = z/(2 hh0) + w/(2 a0)
-// (9 operations where the rows' products take 13), and the back-projection
-//   h_0 = c0 + c1 + c3,  h_n = u_n0 h_0 + a0 (c3 - c0),  h_t = u_t0 h_0 + c2,
-//   h_3 = H0 (c0 + c3) + a0 u_n0 (c3 - c0) + uu0 c1 + u_t0 c2.
-struct EigFast {
-    double un0, ut0, a0, h0, uu0;
-    double ia5, ih, ihh;  // 1/(2 a0), 1/(2 hh0), 1/hh0
-};
-
-template <int DIR>
-__device__ __forceinline__ bool roe_eig_fast(double g1, double sl, double sr, double ul, double ur,
-                                             double vl, double vr, double hl, double hr, EigFast& e) {
-    const double w = sr * fx::rcp(sl + sr);
-    const double u0 = fma(w, ur - ul, ul);
-    const double v0 = fma(w, vr - vl, vl);
-    e.h0 = fma(w, hr - hl, hl);
-    e.uu0 = 0.5 * fma(u0, u0, v0 * v0);
-    const double c2 = g1 * (e.h0 - e.uu0);
-    const double ia = fx::rsqrt(c2);
-    e.a0 = c2 * ia;
-    e.ia5 = 0.5 * ia;
-    e.ih = g1 * ia * e.ia5;
-    e.ihh = 2.0 * e.ih;
-    e.un0 = DIR == 0 ? u0 : v0;
-    e.ut0 = DIR == 0 ? v0 : u0;
-    return c2 > 0.0;
-}
-
-// Characteristic fields of a flux (or flux difference) f.
-template <int DIR>
-__device__ __forceinline__ void project_fast(const EigFast& e, const double f[4], double l[4]) {
-    const double w = fma(-e.un0, f[0], f[1 + DIR]), q = fma(-e.ut0, f[0], f[2 - DIR]);
-    const double z = fma(-e.ut0, q, fma(-e.un0, w, fma(-e.uu0, f[0], f[3])));
-    const double m = e.ia5 * w;
-    l[0] = fma(e.ih, z, -m);
-    l[1] = fma(-e.ihh, z, f[0]);
-    l[2] = q;
-    l[3] = fma(e.ih, z, m);
-}
-
-// Characteristic-wise WENO-Z. The projection is linear, so a field's first differences are the
-// projected differences of the split flux; and the projected centre value, projected back, is the
-// centre flux itself, so that only the reconstructions' corrections pass through the fields:
-//   h = F+(centre) + F-(centre) + sum_k r_k (c_k+ + c_k-),
-// one back-projection for both signs and none of the centres' projections. c[k] takes 6 c_k (added,
-// the "-" stencil's differences read in mirrored order with the opposite sign: neg).
-template <int DIR>
-__device__ __forceinline__ void char_corrections(const EigFast& e, const double dF[4][4], bool neg, double c[4]) {
-    double g[4][4];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        double l[4];
-        project_fast<DIR>(e, dF[m], l);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) g[k][m] = l[k];
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        // a correction is odd in its differences, to the bit
-        c[k] += fx::from_bits(fx::bits(fx::correction<true>(g[k])) ^ (neg ? 0x8000000000000000ull : 0ull));
-    }
-}
-template <int DIR>
-__device__ __forceinline__ void back_project_fast(const EigFast& e, const double c[4], const double centre[4],
-                                                  double h[4]) {
-    const double s = c[0] + c[3], d = c[3] - c[0], h0 = s + c[1], ad = e.a0 * d;
-    const double hn = fma(e.un0, h0, ad), ht = fma(e.ut0, h0, c[2]);
-    const double h3 = fma(e.h0, s, fma(e.un0, ad, fma(e.uu0, c[1], e.ut0 * c[2])));
-    h[0] = fma(1.0 / 6.0, h0, centre[0]);
-    h[1 + DIR] = fma(1.0 / 6.0, hn, centre[1 + DIR]);
-    h[2 - DIR] = fma(1.0 / 6.0, ht, centre[2 - DIR]);
-    h[3] = fma(1.0 / 6.0, h3, centre[3]);
-}
+#include "char_fast.cuh"
 
 // ---------------------------------------------------------------------------------------------
 // Index helpers
@@ -480,6 +401,17 @@ struct CwTile {
     static constexpr bool kStageG = FAST && REC != DENSE_RECON_UPWIND5;
     static constexpr size_t bytes = sizeof(double) * (size_t)NCELL * (kStageG ? 16 : 8);
 };
+
+// The position of the (n + 1)-th set bit of m, which has more than n.
+__device__ __forceinline__ int nth_bit(unsigned m, int n) {
+    int at = 0;
+#pragma unroll
+    for (int w = 16; w; w >>= 1) {
+        const int c = __popc(m >> at & ((1u << w) - 1u));
+        if (n >= c) { n -= c; at += w; }
+    }
+    return at;
+}
 
 // TZ threads share an interface (threadIdx.z): they stage the tile's cells together and each
 // reconstructs the components tz, tz + TZ, ...; the arithmetic of every component is the same
@@ -748,6 +680,64 @@ struct CharTile {
     static constexpr size_t bytes = sizeof(double) * (size_t)(kR + kRSize);
 };
 
+#if FAST
+// The corrections of a warp's stencils, one a lane (active: the lane has one), added to c[k]. where: the
+// offset in sDF of a stencil's first difference, twice over, and its sign (step: the next difference's
+// offset; the "-" stencil's are read in mirrored order with the opposite sign). The fields left to
+// FP64 are few, but several of one stencil, and its lane's in turn would keep the block from its
+// barriers (sweeps of the 480 x 120 double Mach reflection: xi 0.024 -> 0.030 ms); the warp takes them
+// together, a lane a field, its Roe state by shuffles.
+template <int DIR, int NCELL>
+__device__ __forceinline__ void warp_corrections(const Params& p, const EigFast& e, const double* sDF, int where, int step,
+                                                 double f0, double ft, bool active, double c[4]) {
+    auto diff = [&](int w, int m, double d[4]) {
+        const int o = (w >> 1) + (w & 1 ? -m : m) * step;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) d[v] = sDF[chk(p, o + v * NCELL, 8 * NCELL)];
+    };
+    double cs[4];
+    unsigned redo = char_fields<DIR>(e, [&](int m, double d[4]) { diff(where, m, d); }, f0, ft, cs);
+    if (!active) redo = 0;
+    if (__any_sync(0xffffffffu, redo != 0)) {
+        asm volatile("" ::: "memory");  // the differences are read again, not kept
+        const int lane = (threadIdx.x + blockDim.x * threadIdx.y) & 31;
+        unsigned of[4];
+        int n = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            of[k] = __ballot_sync(0xffffffffu, redo >> k & 1u);
+            n += __popc(of[k]);
+        }
+#pragma unroll 1
+        for (int n0 = 0; n0 < n; n0 += 32) {
+            int q = min(n0 + lane, n - 1), k = 0;
+            unsigned from = of[0];
+#pragma unroll
+            for (int l = 1; l < 4; ++l)
+                if (k == l - 1 && q >= __popc(from)) { q -= __popc(from); from = of[l]; k = l; }
+            const int src = nth_bit(from, q);
+            auto get = [&](double x) { return __shfl_sync(0xffffffffu, x, src); };
+            EigFast o;
+            o.un0 = get(e.un0); o.ut0 = get(e.ut0); o.uu0 = get(e.uu0);
+            o.ia5 = get(e.ia5); o.ih = get(e.ih); o.ihh = get(e.ihh);
+            const int w = __shfl_sync(0xffffffffu, where, src);
+            const double v = char_field_fp64<DIR>(o, [&](int m, double d[4]) { diff(w, m, d); }, k);
+            int at = -n0;
+#pragma unroll
+            for (int l = 0; l < 4; ++l) {
+                const int mine = at + __popc(of[l] & ((1u << lane) - 1u));
+                const double r = __shfl_sync(0xffffffffu, v, mine & 31);
+                if ((redo >> l & 1u) && mine >= 0 && mine < 32) cs[l] = r;
+                at += __popc(of[l]);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)  // a correction is odd in its differences, to the bit
+        c[k] += fx::from_bits(fx::bits(cs[k]) ^ (where & 1 ? 0x8000000000000000ull : 0ull));
+}
+#endif
+
 template <int DIR, bool ADAPT, int TX, int TY>
 __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx, int by) {
     if (!p.sc->active) return;
@@ -918,31 +908,29 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
 
     if constexpr (!ADAPT) {
         // 104: every interface takes the characteristic branch for both signs
-        if (!valid) return;
         EigT e;
-        eig_at(tx, ty, e);
         double hsum[4];
 #if FAST
+        // (whole warps go on: the threads past the last interface or line take that of the tile's first)
+        const int ox = valid ? tx : 0, oy = valid ? ty : 0;
+        if (!__any_sync(0xffffffffu, valid)) return;
+        eig_at(ox, oy, e);
         // "+": centre F+(t+2), differences F+(t+m) - F+(t+m+1) = DF+(t+m); "-": centre
         // F-(t+3), differences F-(t+5-m) - F-(t+4-m) = -DF-(t+4-m)
-        const int t = DIR == 0 ? tx : ty;
+        const int t = DIR == 0 ? ox : oy;
         double c6[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 1
-        for (int s = 0; s < 2; ++s) {
-            double dF[4][4];
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const int o = atk(s == 0 ? t + m : t + 4 - m, tx, ty);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) dF[m][c] = sDF[(4 * s + c) * NCELL + o];
-            }
-            char_corrections<DIR>(e, dF, s != 0, c6);
-        }
+        for (int s = 0; s < 2; ++s)
+            warp_corrections<DIR, NCELL>(p, e, sDF, (4 * s * NCELL + atk(t + 4 * s, ox, oy)) * 2 + s, DIR == 0 ? 1 : NC,
+                                         SF(4 * s, t + 2 + s, ox, oy), SF(4 * s + 2 - DIR, t + 2 + s, ox, oy), valid, c6);
+        if (!valid) return;
         double centre[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) centre[c] = SF(c, t + 2, tx, ty) + SF(4 + c, t + 3, tx, ty);
         back_project_fast<DIR>(e, c6, centre, hsum);
 #else
+        if (!valid) return;
+        eig_at(tx, ty, e);
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
             double h[4];
@@ -1069,32 +1057,32 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
         }
 #endif
         __syncthreads();
-        // phase 2b: the block works through the characteristic items (SC.f90:126-163)
+        // phase 2b: the block works through the characteristic items (SC.f90:126-163), whole warps at a
+        // time: the lanes past the last item take that one
         const int nq = qn;
-        for (int it = tid; it < nq; it += NT) {
-            const int item = queue[it], owner = item >> 1, s = item & 1;
+        for (int it0 = tid & ~31; it0 < nq; it0 += NT) {
+            const int it = it0 + (tid & 31);
+            const int item = queue[min(it, nq - 1)], owner = item >> 1, s = item & 1;
             const int ox = owner % TX, oy = owner / TX;
             EigT e;
             eig_at(ox, oy, e);
             double h[4];
 #if FAST
             const int t0 = DIR == 0 ? ox : oy;
-            double dF[4][4], centre[4], c6[4] = {0.0, 0.0, 0.0, 0.0};
+            double centre[4], c6[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                centre[c] = SF(4 * s + c, t0 + 2 + s, ox, oy);
-#pragma unroll
-                for (int m = 0; m < 4; ++m) dF[m][c] = sDF[(4 * s + c) * NCELL + atk(s == 0 ? t0 + m : t0 + 4 - m, ox, oy)];
-            }
-            char_corrections<DIR>(e, dF, s != 0, c6);
+            for (int c = 0; c < 4; ++c) centre[c] = SF(4 * s + c, t0 + 2 + s, ox, oy);
+            warp_corrections<DIR, NCELL>(p, e, sDF, (4 * s * NCELL + atk(t0 + 4 * s, ox, oy)) * 2 + s, DIR == 0 ? 1 : NC,
+                                         centre[0], centre[2 - DIR], it < nq, c6);
             back_project_fast<DIR>(e, c6, centre, h);
 #else
             double F[5][4];
             stencil(ox, oy, s, F);
             char_weno(e, F, h);
 #endif
+            if (it < nq)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) hbuf(s, c, owner) = h[c];
+                for (int c = 0; c < 4; ++c) hbuf(s, c, owner) = h[c];
         }
         __syncthreads();
         // phase 2c: h = h+ + h- (sum_field, field_op.f90:1-21)

@@ -43,3 +43,14 @@ def test_forms(lines, z):
     """Odd, the same in either order, and a flat stencil's centre, in both arithmetics."""
     (row,) = [[int(v) for v in x[2:]] for x in lines if x[0] == "forms" and x[1] == str(z)]
     assert row[:3] == [0, 0, 0] and row[3] > 10000
+
+
+@pytest.mark.parametrize("ratio", ["0.1", "2", "8", "100", "10000", "1e+08"])
+def test_characteristic_fluxes(lines, ratio):
+    """The characteristic schemes' fluxes beside jumps, each relative to its own small side: no less exact
+    than an FP64 reconstruction of the fields' values (the worst to a factor of two)."""
+    rows = [[float(v) for v in x[3:]] for x in lines if x[0] == "fields" and x[1] == ratio]
+    assert len(rows) == 4
+    for rms, rms64, worst, worst64 in rows:
+        assert rms <= 1.02 * rms64
+        assert worst <= 2.0 * worst64

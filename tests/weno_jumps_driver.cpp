@@ -12,13 +12,14 @@
 namespace fx = dense::fx;
 #include "../2dense_gb300/csrc/weno_fast.cuh"
 #include "../2dense_gb300/csrc/weno_value.cuh"
+#include "../2dense_gb300/csrc/char_fast.cuh"
 
 typedef long double ld;
 
 static double draw(std::mt19937_64& r) { return std::uniform_real_distribution<double>(-1, 1)(r); }
 
 // what a reconstruction adds to its centre value, from the first differences
-template <bool Z> ld correction(const double g[4]) {
+template <bool Z, typename T> ld correction_of(const T g[4]) {
     const ld ss = (double)1.0e-6f, cs[3] = {1, 6, 3};
     const ld A[3] = {(ld)g[0] - g[1], (ld)g[1] - g[2], (ld)g[2] - g[3]};
     const ld B[3] = {g[0] - 3 * (ld)g[1], (ld)g[1] + g[2], 3 * (ld)g[2] - g[3]};
@@ -33,6 +34,8 @@ template <bool Z> ld correction(const double g[4]) {
     }
     return num / den;
 }
+
+template <bool Z> ld correction(const double g[4]) { return correction_of<Z>(g); }
 
 // two jumps, one at each end of the stencil, a power of two apart, the middle smooth: the error in
 // units of the largest value, and what AdaWENO's switch (delta 1/2) takes for smooth
@@ -124,7 +127,91 @@ template <bool Z> void value_forms() {
     printf("forms %d %d %d %d %d\n", (int)Z, odd, swap, flat, fp64s);
 }
 
+// A face's four fluxes of the characteristic schemes beside a jump of about `ratio` times the level in
+// density, pressure and velocities (the tangential one zero on the small side now and then), with the
+// Roe state as given: char_fields and char_field_fp64 as the sweeps put them together, and an FP64
+// reconstruction of the fields' values, centre included. Errors relative to each flux's centre values and itself.
+void fields(double ratio) {
+    std::mt19937_64 r((unsigned)(500 + 10 * std::log10(ratio)));
+    const double g = 1.4;
+    Errors err[4];
+    for (int t = 0; t < 10000; ++t) {
+        const int j = 1 + (int)(r() % 5);
+        const bool left = r() & 1;
+        const double jr = 1 + ratio * (0.5 + std::fabs(draw(r))), jp = 1 + ratio * (0.5 + 3 * std::fabs(draw(r)));
+        const double amp = std::pow(10.0, -3 + 2 * draw(r)), p0 = 0.1 + std::fabs(draw(r)), u0 = 2 * draw(r);
+        const double v0 = r() % 3 ? draw(r) : 0.0, du = 2 * draw(r), dv = r() % 3 ? 2 * draw(r) : 0.0;
+        double F[2][6][4], cell[6][4], lam = 0;
+        for (int m = 0; m < 6; ++m) {
+            const bool big = left ? m < j : m >= j;
+            const double x = m - 2.5;
+            cell[m][0] = (1 + amp * (0.1 * draw(r) + 0.1 * x)) * (big ? jr : 1);
+            cell[m][1] = u0 + amp * (0.1 * draw(r) + 0.2 * x) + (big ? du : 0);
+            cell[m][2] = (v0 != 0 ? v0 + amp * (0.1 * draw(r) - 0.1 * x) : 0.0) + (big ? dv : 0);
+            cell[m][3] = p0 * (1 + amp * (0.1 * draw(r) + 0.1 * x)) * (big ? jp : 1);
+            lam = std::max(lam, std::fabs(cell[m][1]) + std::sqrt(g * cell[m][3] / cell[m][0]));
+        }
+        lam *= 1 + 0.5 * std::fabs(draw(r));
+        for (int m = 0; m < 6; ++m) {
+            const double *c = cell[m], E = c[3] / (g - 1) + 0.5 * c[0] * (c[1] * c[1] + c[2] * c[2]);
+            const double U[4] = {c[0], c[0] * c[1], c[0] * c[2], E};
+            const double f[4] = {U[1], U[1] * c[1] + c[3], U[1] * c[2], c[1] * (E + c[3])};
+            for (int k = 0; k < 4; ++k) { F[0][m][k] = 0.5 * (f[k] + lam * U[k]); F[1][m][k] = 0.5 * (f[k] - lam * U[k]); }
+        }
+        EigFast e;
+        const double *L = cell[2], *R = cell[3];
+        auto H = [&](const double* c) { return g / (g - 1) * c[3] / c[0] + 0.5 * (c[1] * c[1] + c[2] * c[2]); };
+        roe_eig_fast<0>(g - 1, std::sqrt(L[0]), std::sqrt(R[0]), L[1], R[1], L[2], R[2], H(L), H(R), e);
+        ld cq[4] = {0, 0, 0, 0}, zq[4] = {0, 0, 0, 0};
+        double c6[4] = {0, 0, 0, 0}, w6[4] = {0, 0, 0, 0}, centre[4] = {0, 0, 0, 0}, size[4] = {0, 0, 0, 0};
+        for (int s = 0; s < 2; ++s) {
+            double d[4][4], gk[4][4], lc[4], cs[4];
+            for (int m = 0; m < 4; ++m)
+                for (int c = 0; c < 4; ++c) d[m][c] = F[s][s ? 5 - m : m][c] - F[s][s ? 4 - m : m + 1][c];
+            auto dF = [&](int m, double f[4]) { for (int c = 0; c < 4; ++c) f[c] = d[m][c]; };
+            const double* C = F[s][s ? 3 : 2];
+            const unsigned redo = char_fields<0>(e, dF, C[0], C[2], cs);
+            for (int k = 0; k < 4; ++k) c6[k] += redo >> k & 1 ? char_field_fp64<0>(e, dF, k) : cs[k];
+            for (int m = 0; m < 4; ++m) {
+                double l[4];
+                project_fast<0>(e, d[m], l);
+                for (int k = 0; k < 4; ++k) gk[k][m] = l[k];
+            }
+            project_fast<0>(e, C, lc);
+            for (int k = 0; k < 4; ++k) {
+                w6[k] += 6 * (lc[k] + correction_fp64<true>(gk[k]));
+                // the exact differences' exact fields
+                ld gq[4];
+                for (int m = 0; m < 4; ++m) {
+                    const double *a = F[s][s ? 5 - m : m], *b = F[s][s ? 4 - m : m + 1];
+                    const ld f0 = (ld)a[0] - b[0], w = ((ld)a[1] - b[1]) - e.un0 * f0, qt = ((ld)a[2] - b[2]) - e.ut0 * f0;
+                    const ld z = ((ld)a[3] - b[3]) - e.uu0 * f0 - e.un0 * w - e.ut0 * qt;
+                    gq[m] = k == 0 ? e.ih * z - e.ia5 * w : k == 1 ? f0 - e.ihh * z : k == 2 ? qt : e.ih * z + e.ia5 * w;
+                }
+                cq[k] += correction_of<true>(gq);
+                zq[k] += C[k];
+                centre[k] += C[k];
+                size[k] = std::max(size[k], std::fabs(C[k]));
+            }
+        }
+        const ld s = cq[0] + cq[1] + cq[3], dd = cq[3] - cq[0];
+        const ld want[4] = {zq[0] + s, zq[1] + e.un0 * s + e.a0 * dd, zq[2] + e.ut0 * s + cq[2],
+                            zq[3] + e.h0 * (cq[0] + cq[3]) + e.a0 * e.un0 * dd + e.uu0 * cq[1] + e.ut0 * cq[2]};
+        double h[4], h64[4];
+        const double zero[4] = {0, 0, 0, 0};
+        back_project_fast<0>(e, c6, centre, h);
+        back_project_fast<0>(e, w6, zero, h64);
+        for (int k = 0; k < 4; ++k) {
+            // (a transverse flux beside a larger normal one is not held to its own smallness)
+            const double sz = std::max(size[k] + (double)fabsl(want[k]), k == 2 ? 1e-3 * size[1] : 0.0);
+            err[k].add((double)fabsl(h[k] - want[k]) / sz, (double)fabsl(h64[k] - want[k]) / sz);
+        }
+    }
+    for (int k = 0; k < 4; ++k) { printf("fields %g %d ", ratio, k); err[k].print(); }
+}
+
 int main() {
+    for (double ratio : {0.1, 2.0, 8.0, 100.0, 1e4, 1e8}) fields(ratio);
     for (int kind = 0; kind < 2; ++kind)
         for (int decades : {-3, 0, 1, 2, 4, 6, 10, 14}) { sided<false>(kind, decades); sided<true>(kind, decades); }
     value_forms<false>();
