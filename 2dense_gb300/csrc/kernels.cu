@@ -950,6 +950,8 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
         bool smooth[2] = {true, true};
 #if FAST
         fx::u64 f0[2], f2[2];
+        const bool far = fx::far_weights(p.theta_c);
+        unsigned redo = 0;  // the components of the smooth branch left to FP64 (small deltas only)
 #else
         double wsur[2][3];
 #endif
@@ -966,6 +968,7 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
                 const bool sm = fx::surrogate(g, p.theta_c, a, b);
                 if (s == 0) { smooth[0] = sm; f0[0] = a; f2[0] = b; }
                 else        { smooth[1] = sm; f0[1] = a; f2[1] = b; }
+                if (far && sm && fx::rough(g)) redo = 15u;
                 if (p.theta) theta_out(s, theta_of(g));
             }
 #else
@@ -1023,8 +1026,34 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
                     const fx::u32 ep = smooth[0] ? fx::exponent_of(gp) : 0u, em = smooth[1] ? fx::exponent_of(gm) : 0u;
                     const fx::u32 top = fx::umax(ep, em), eh = fx::umax(top, fx::kExpMin);
                     const fx::i64 kp = fx::correction6_by(gp, eh, f0[0], f2[0]), km = fx::correction6_by(gm, eh, f0[1], f2[1]);
-                    const double h = fx::about(smooth[0] ? SF(c, t + 2, tx, ty) : 0.0, smooth[1] ? SF(4 + c, t + 3, tx, ty) : 0.0,
-                                               fx::to_double((smooth[0] ? kp : 0) - (smooth[1] ? km : 0), eh, top));
+                    const double lp = smooth[0] ? SF(c, t + 2, tx, ty) : 0.0, lm = smooth[1] ? SF(4 + c, t + 3, tx, ty) : 0.0;
+                    const double c6 = fx::to_double((smooth[0] ? kp : 0) - (smooth[1] ? km : 0), eh, top);
+                    if (far && fx::coarse_by(top, lp, lm, c6)) redo |= 1u << c;
+                    const double h = fx::about(lp, lm, c6);
+                    if (both) store_one(c, h);
+                    else hbuf(smooth[0] ? 0 : 1, c, tid) = h;
+                }
+#pragma unroll 1
+                for (; redo; redo &= redo - 1) {
+                    const int c = __ffs((int)redo) - 1;
+                    double l[2] = {0.0, 0.0}, cs = 0.0;
+#pragma unroll 1
+                    for (int s = 0; s < 2; ++s) {
+                        if (!(s == 0 ? smooth[0] : smooth[1])) continue;
+                        double g[4], u[3];
+#pragma unroll
+                        for (int m = 0; m < 4; ++m) {  // the surrogate's differences, as they were staged
+                            const int o = atk(s == 0 ? t + m : t + 4 - m, tx, ty);
+                            g[m] = (sQ[o] - sQ[o + (DIR == 0 ? 1 : NC)]) + sDF[(4 * s + 1 + DIR) * NCELL + o];
+                        }
+                        weights_fp64<true>(g, u);
+#pragma unroll
+                        for (int m = 0; m < 4; ++m) g[m] = sDF[(4 * s + c) * NCELL + atk(s == 0 ? t + m : t + 4 - m, tx, ty)];
+                        const double k = correction_by_fp64(g, u);
+                        cs += s == 0 ? k : -k;
+                        (s == 0 ? l[0] : l[1]) = SF(4 * s + c, t + 2 + s, tx, ty);
+                    }
+                    const double h = about_fp64(l[0], l[1], cs);
                     if (both) store_one(c, h);
                     else hbuf(smooth[0] ? 0 : 1, c, tid) = h;
                 }

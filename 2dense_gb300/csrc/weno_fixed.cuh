@@ -402,6 +402,18 @@ DENSE_FX i64 correction6_by(const double g[4], u32 eh, u64 f0, u64 f2) {
     return scaled(f0, (A0 - A1) * 4) + scaled(f2, (A1 - A2) * 4) - G1 - 2 * G2;
 }
 
+// Whether the smooth branch may meet weights far from the linear ones: down to delta = 0.01 a smooth
+// surrogate's are within a factor of 11 (sum alpha - 1 <= 10) and its differences alike, so that a jump
+// of a component counts in its value, and the integer form's rms error is 0.6 to 0.75 of FP64's beside
+// jumps of any size. theta_c = k/(1 + k), k = sqrt(delta/(1 - delta)).
+DENSE_FX bool far_weights(double theta_c) { return theta_c < 0.0913; }
+// Where it may: whether about(lp, lm, c6) of such corrections is to be computed in FP64 instead (enough; the
+// sum's rounding is relative to a few binades more than it, and a surrogate that is rough is never left
+// to integers).
+DENSE_FX bool coarse_by(u32 top, double lp, double lm, double c6) {
+    return exponent(c6) + (3u << 20) < enough(top, umax(exponent(lp), exponent(lm)));
+}
+
 // dt/dx and dt/dy as fixed-point factors of one exponent, below 2^62 (in units of 2^-shift), and
 // dt's sign; shift kNoShift where one is not finite.
 constexpr int kNoShift = 1 << 20;

@@ -54,3 +54,14 @@ def test_characteristic_fluxes(lines, ratio):
     for rms, rms64, worst, worst64 in rows:
         assert rms <= 1.02 * rms64
         assert worst <= 2.0 * worst64
+
+
+@pytest.mark.parametrize("decades", [-3, 0, 2, 6, 10])
+@pytest.mark.parametrize("delta", ["0", "0.001", "0.01", "0.5", "0.9"])
+def test_borrowed_weights(lines, delta, decades):
+    """AdaWENO's smooth branch, a component beside a jump with a smooth surrogate's weights (or, delta 0,
+    with any surrogate's): no less exact than in FP64, as test_small_side."""
+    ((rms, rms64, worst, worst64),) = [[float(v) for v in x[3:]] for x in lines
+                                       if x[0] == "borrowed" and x[1:3] == [delta, str(decades)]]
+    assert rms <= 1.02 * rms64
+    assert worst <= 2.0 * worst64

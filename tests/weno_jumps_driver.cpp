@@ -37,6 +37,17 @@ template <bool Z, typename T> ld correction_of(const T g[4]) {
 
 template <bool Z> ld correction(const double g[4]) { return correction_of<Z>(g); }
 
+// the weights over the linear ones, from the first differences
+static void weights_of(const double g[4], ld w[3]) {
+    const ld ss = (double)1.0e-6f, cs[3] = {0.1L, 0.6L, 0.3L};
+    const ld A[3] = {(ld)g[0] - g[1], (ld)g[1] - g[2], (ld)g[2] - g[3]};
+    const ld B[3] = {g[0] - 3 * (ld)g[1], (ld)g[1] + g[2], 3 * (ld)g[2] - g[3]};
+    ld d[3], sum = 0;
+    for (int k = 0; k < 3; ++k) d[k] = ss + 13 * A[k] * A[k] / 12 + B[k] * B[k] / 4;
+    for (int k = 0; k < 3; ++k) sum += w[k] = cs[k] * (1 + (d[2] - d[0]) / d[k] * ((d[2] - d[0]) / d[k]));
+    for (int k = 0; k < 3; ++k) w[k] /= sum;
+}
+
 // two jumps, one at each end of the stencil, a power of two apart, the middle smooth: the error in
 // units of the largest value, and what AdaWENO's switch (delta 1/2) takes for smooth
 template <bool Z> void between() {
@@ -210,7 +221,56 @@ void fields(double ratio) {
     for (int k = 0; k < 4; ++k) { printf("fields %g %d ", ratio, k); err[k].print(); }
 }
 
+// AdaWENO's smooth branch: a component beside a jump of 10^decades times its level, reconstructed with
+// the weights of a surrogate that is smooth for the given delta, relative to the centre values and
+// corrections; FP64's from the same weights. few: surrogates with a jump among them (delta 0: always smooth)
+void borrowed(double delta, int decades) {
+    std::mt19937_64 r((unsigned)(900 + 10 * decades + (int)(100 * delta)));
+    const double k = std::sqrt(delta / (1.0 - delta)), theta_c = k / (1.0 + k);
+    Errors err;
+    for (int t = 0; t < 200000 && err.n < 20000; ++t) {
+        const double level = std::pow(10.0, 3 * draw(r)), amp = std::pow(10.0, -2 + 2 * draw(r)), half = r() & 1 ? 0.0 : 1.0;
+        double gs[2][4], g[2][4];
+        ld c[2];
+        double c64[2];
+        fx::u64 f0[2], f2[2];
+        bool ok = true, rough = false;
+        for (int s = 0; s < 2; ++s) {
+            const double a = draw(r), b = 0.3 * draw(r), js = std::pow(10.0, 3 * draw(r)) * draw(r);
+            const int j = (int)(r() % 4), i = (int)(r() % 4);
+            for (int m = 0; m < 4; ++m) {
+                gs[s][m] = 0.1 * (a + b * (m - 1.5)) + (delta == 0.0 && m == i && r() & 1 ? js : 0.0);
+                g[s][m] = level * (amp * (a + draw(r) * 0.3) + (m == j ? std::pow(10.0, decades) * (1 + 0.5 * draw(r)) : 0.0));
+            }
+            ok = fx::surrogate(gs[s], theta_c, f0[s], f2[s]) && ok;
+            rough = fx::rough(gs[s]) || rough;
+        }
+        if (!ok) continue;
+        const double lp = half * level * (1 + 0.3 * draw(r)), lm = -0.7 * half * level * (1 + 0.3 * draw(r));
+        for (int s = 0; s < 2; ++s) {
+            ld w[3];
+            double u[3];
+            weights_of(gs[s], w);
+            c[s] = (w[0] * (2 * (ld)g[s][0] - 5 * (ld)g[s][1]) + w[1] * (-(ld)g[s][1] - 2 * (ld)g[s][2]) +
+                    w[2] * ((ld)g[s][3] - 4 * (ld)g[s][2])) / 6;
+            weights_fp64<true>(gs[s], u);
+            c64[s] = correction_by_fp64(g[s], u);
+        }
+        const fx::u32 top = fx::umax(fx::exponent_of(g[0]), fx::exponent_of(g[1])), eh = fx::umax(top, fx::kExpMin);
+        const double c6 = fx::to_double(fx::correction6_by(g[0], eh, f0[0], f2[0]) + fx::correction6_by(g[1], eh, f0[1], f2[1]), eh, top);
+        double h = fx::about(lp, lm, c6);
+        if (fx::far_weights(theta_c) && (rough || fx::coarse_by(top, lp, lm, c6))) h = about_fp64(lp, lm, c64[0] + c64[1]);
+        const ld want = c[0] + c[1] + lp + lm;
+        const double size = std::max(std::fabs(lp), std::fabs(lm)) + (double)(fabsl(c[0]) + fabsl(c[1]));
+        err.add((double)fabsl(h - want) / size, (double)fabsl((lp + c64[0]) + (lm + c64[1]) - want) / size);
+    }
+    printf("borrowed %g %d ", delta, decades);
+    err.print();
+}
+
 int main() {
+    for (double delta : {0.0, 0.001, 0.01, 0.5, 0.9})
+        for (int decades : {-3, 0, 2, 6, 10}) borrowed(delta, decades);
     for (double ratio : {0.1, 2.0, 8.0, 100.0, 1e4, 1e8}) fields(ratio);
     for (int kind = 0; kind < 2; ++kind)
         for (int decades : {-3, 0, 1, 2, 4, 6, 10, 14}) { sided<false>(kind, decades); sided<true>(kind, decades); }
