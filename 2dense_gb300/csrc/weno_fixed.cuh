@@ -414,36 +414,64 @@ DENSE_FX bool coarse_by(u32 top, double lp, double lm, double c6) {
     return exponent(c6) + (3u << 20) < enough(top, umax(exponent(lp), exponent(lm)));
 }
 
-// dt/dx and dt/dy as fixed-point factors of one exponent, below 2^62 (in units of 2^-shift), and
-// dt's sign; shift kNoShift where one is not finite.
-constexpr int kNoShift = 1 << 20;
+// dt/dx and dt/dy, each m 2^(e - 1086) with the top bit of m set, 0 for a zero rate, and dt's sign; e kNoRate
+// where one is not finite.
+constexpr int kNoRate = 1 << 20;
+struct Rate {
+    u64 m;
+    int e;
+};
 struct Rates {
-    u64 x, y;
-    int shift;
+    Rate x, y;
     u32 sign;  // 0 or the sign bit of an upper word
 };
-DENSE_FX Rates rates_of(double dtdx, double dtdy) {
-    const u64 bx = bits(dtdx), by = bits(dtdy), top = 0x2000000000000000ull;
-    const u32 ex = (hi32(bx) >> 20) & 0x7ffu, ey = (hi32(by) >> 20) & 0x7ffu, e = umax(ex, ey);
-    Rates r;
-    r.x = shr(((bx << 9) & (top - 1)) | top, e - ex);
-    r.y = shr(((by << 9) & (top - 1)) | top, e - ey);
-    r.shift = e == 0x7ffu ? kNoShift : 61 + 1023 - (int)e;
-    r.sign = hi32(bx) & 0x80000000u;
+DENSE_FX Rate rate_of(u64 b) {
+    const int e = (int)((b >> 52) & 0x7ff);
+    Rate r;
+    r.m = e ? (b << 11) | 0x8000000000000000ull : 0;
+    r.e = e == 0x7ff ? kNoRate : e;
     return r;
 }
-// dt/dx (xr - xl) + dt/dy (yr - yl): the differences exact in fixed point, their products with the rates
-// and the sum truncated below 2^-57 of the largest flux times the larger rate, rounded once.
-DENSE_FX double flux_change(double xl, double xr, double yl, double yr, const Rates& r) {
-    const u32 top = umax(umax(exponent(xl), exponent(xr)), umax(exponent(yl), exponent(yr)));
-    const u32 eh = umax(top, kExpMin);
-    const i64 X = to_fixed(xr, eh) - to_fixed(xl, eh), Y = to_fixed(yr, eh) - to_fixed(yl, eh);  // below 2^59
-    const i64 t = scaled(r.x, X * 8) + scaled(r.y, Y * 8);     // 2^(shift - 61) of the sum, below 2^61
-    const int e = (int)(eh >> 20) + 61 - r.shift;
-    double d = to_double(t, (u32)imax(e, 64) << 20, top);
-    if (e < 64) d = 0.0;                                       // below 2^-950: also where a rate is 0
-    if (r.shift == kNoShift) d = from_bits(0x7ff8000000000000ull);
-    return from_bits(bits(d) ^ ((u64)r.sign << 32));
+DENSE_FX Rates rates_of(double dtdx, double dtdy) {
+    Rates r;
+    r.x = rate_of(bits(dtdx));
+    r.y = rate_of(bits(dtdy));
+    r.sign = hi32(bits(dtdx)) & 0x80000000u;
+    return r;
+}
+// A rate times the difference of two fluxes: sign (all ones or zero) and m 2^(e - 1080), m below 2^63 and not below
+// 2^61 (or 0). The fluxes are fixed-point integers of their own exponent, 2^-57 of the larger one, so
+// that their difference is exact unless one of them is 2^5 times the other, and good to 2^-57 then.
+struct Change {
+    u64 m, sign;
+    int e;
+};
+DENSE_FX Change change_of(double l, double r, const Rate& q, u32& top) {
+    const u32 t = umax(exponent(l), exponent(r)), eh = umax(t, 64u << 20);
+    top = umax(top, t);
+    const i64 d = to_fixed(r, eh) - to_fixed(l, eh);  // below 2^59
+    const u64 a = abs64(d);
+    const int n = clz64(a) & 63;
+    Change c;
+    c.m = mulhi(a << n, q.m) >> 1;
+    c.sign = (u64)(d >> 63);
+    c.e = c.m ? (int)(eh >> 20) - n + q.e - 1021 : -10000;
+    return c;
+}
+// dt/dx (xr - xl) + dt/dy (yr - yl): each direction's difference exact or good to 2^-57 of itself, its
+// product with the rate truncated below 2^-60, the smaller product to the larger one's unit, their sum
+// rounded once. Below 2^-950 the result is 0; NaN for what is not finite.
+DENSE_FX double flux_change(double xl, double xr, double yl, double yr, const Rates& q) {
+    u32 top = 0;
+    const Change x = change_of(xl, xr, q.x, top), y = change_of(yl, yr, q.y, top);
+    const int e = imax(x.e, y.e);
+    const u64 a = shr(x.m, (u32)(e - x.e) + 1), b = shr(y.m, (u32)(e - y.e) + 1);
+    const i64 t = (i64)((a ^ x.sign) - x.sign) + (i64)((b ^ y.sign) - y.sign);   // below 2^63
+    double d = to_double(t, (u32)imin(imax(e + 1, 64), 2040) << 20, 0);
+    if (e + 1 < 64) d = 0.0;
+    if (e + 1 > 2040) d = d * from_bits((u64)(1023 + imin(e + 1 - 2040, 1000)) << 52);  // (towards infinity)
+    if (top >= 0x7ff00000u || umax((u32)q.x.e, (u32)q.y.e) == (u32)kNoRate) d = from_bits(0x7ff8000000000000ull);
+    return from_bits(bits(d) ^ ((u64)q.sign << 32));
 }
 
 }  // namespace fx

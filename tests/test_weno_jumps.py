@@ -65,3 +65,15 @@ def test_borrowed_weights(lines, delta, decades):
                                        if x[0] == "borrowed" and x[1:3] == [delta, str(decades)]]
     assert rms <= 1.02 * rms64
     assert worst <= 2.0 * worst64
+
+
+@pytest.mark.parametrize("kind", range(4))
+def test_flux_change(lines, kind):
+    """The update's dt/dx dh_xi + dt/dy dh_eta, whatever lies between the directions' fluxes, differences
+    and rates: no less exact than in FP64 relative to the larger product (two roundings there, one
+    here), odd, and towards infinity where the result leaves the doubles' range."""
+    ((odd, *errors),) = [x[2:] for x in lines if x[0] == "change" and x[1] == str(kind)]
+    rms, rms64, worst, worst64 = map(float, errors)
+    assert int(odd) == 0
+    assert rms <= 1.02 * rms64
+    assert worst <= 2.0 * worst64

@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <limits>
 #include <random>
 
 #include "../2dense_gb300/csrc/weno_fixed.cuh"
@@ -268,7 +269,41 @@ void borrowed(double delta, int decades) {
     err.print();
 }
 
+// the update's flux change with the directions' fluxes and differences orders apart, relative to the larger
+// product; FP64's beside it. kind 0: both; 1: large eta fluxes that cancel; 2: large xi fluxes that
+// cancel; 3: dt/dx and dt/dy up to 1e9 apart
+void change(int kind) {
+    std::mt19937_64 r(131 + kind);
+    Errors err;
+    int odd = 0;
+    for (int t = 0; t < 50000; ++t) {
+        double h[4];
+        for (int d = 0; d < 2; ++d) {
+            const double size = std::pow(10.0, 12 * draw(r)), small = std::pow(10.0, -12 * std::fabs(draw(r))), base = draw(r);
+            for (int k = 0; k < 2; ++k) h[2 * d + k] = size * (base + small * draw(r));
+        }
+        if (kind == 1) { h[2] = h[3] = 1e3 * std::fabs(h[2]); }
+        if (kind == 2) { h[0] = h[1] = 1e3 * std::fabs(h[0]); }
+        const double dtdx = std::pow(10.0, -3 + 3 * draw(r)), dtdy = dtdx * std::pow(10.0, kind == 3 ? 9 * draw(r) : draw(r));
+        const fx::Rates q = fx::rates_of(dtdx, dtdy);
+        const ld x = (ld)dtdx * ((ld)h[1] - h[0]), y = (ld)dtdy * ((ld)h[3] - h[2]);
+        const double size = (double)std::max(fabsl(x), fabsl(y)), got = fx::flux_change(h[0], h[1], h[2], h[3], q);
+        odd += fx::flux_change(h[1], h[0], h[3], h[2], q) != -got || fx::flux_change(-h[0], -h[1], -h[2], -h[3], q) != -got;
+        if (size == 0.0) continue;
+        err.add((double)fabsl(got - (x + y)) / size, (double)fabsl(fma(dtdx, h[1] - h[0], dtdy * (h[3] - h[2])) - (x + y)) / size);
+    }
+    // the ends of the range
+    const double inf = std::numeric_limits<double>::infinity();
+    odd += fx::flux_change(-4e307, 4e307, 0.0, 0.0, fx::rates_of(1.0, 1.0)) != 8e307;
+    odd += fx::flux_change(-1e200, 1e200, 0.0, 0.0, fx::rates_of(1e200, 1.0)) != inf;
+    odd += fx::flux_change(1e200, -1e200, 0.0, 0.0, fx::rates_of(1e200, 1.0)) != -inf;
+    odd += fx::flux_change(1.0, 2.0, 5.0, 5.0, fx::rates_of(0x1p-600, 1.0)) != 0x1p-600;
+    printf("change %d %d ", kind, odd);
+    err.print();
+}
+
 int main() {
+    for (int kind = 0; kind < 4; ++kind) change(kind);
     for (double delta : {0.0, 0.001, 0.01, 0.5, 0.9})
         for (int decades : {-3, 0, 2, 6, 10}) borrowed(delta, decades);
     for (double ratio : {0.1, 2.0, 8.0, 100.0, 1e4, 1e8}) fields(ratio);
