@@ -356,17 +356,15 @@ DENSE_FX double pair(double lp, const double gp[4], double lm, const double gm[4
     if (fp64) *fp64 = exponent(c) < need;
     return about(lp, lm, c);
 }
-// Whether a stencil's largest difference is more than 2^kRough times its smoothest substencil's (or
-// sqrt(ss)): the gradient's terms are relative to the latter, and its fixed-point differences then
-// know it less well than FP64 does, so such stencils (a few percent beside extrema and jumps) take
-// weno_grad's gradient. Against long double, JS and Z, the rms error is 0.65 to 1.0 of weno_grad's in
-// smooth and rough stencils and up to 1.1 beside single jumps; at 2^3 it would be 1.5 there.
-constexpr u32 kRough = 2u;
-DENSE_FX bool rough(const double g[4]) {
-    const u32 e1 = exponent(g[1]), e2 = exponent(g[2]);
-    const u32 m0 = umax(exponent(g[0]), e1), m1 = umax(e1, e2), m2 = umax(e2, exponent(g[3]));
-    return umax(m0, m2) > umax(umin(umin(m0, m1), m2), kExpSS) + (kRough << 20);
-}
+// Whether the unit eh of a stencil's differences lies more than kRough binades above its smoothest substencil
+// (or sqrt(ss)), by a difference of its own or of the stencil it shares the unit with: the gradient's
+// terms are relative to the smoothest substencil, and the fixed-point differences then know it less
+// well than FP64 does. Such stencils, beside extrema and jumps, take weno_grad's gradient. Against long
+// double, JS and Z, the rms error is 0.67 to 1.0 of weno_grad's; at 2 binades it would be 1.1 beside
+// jumps, and told by a stencil's own differences alone 9 to 11 where the partner has the jump.
+constexpr u32 kRough = 1u;
+DENSE_FX bool rough(const double g[4], u32 eh) { return eh > umax(smoothest_of(g), kExpSS) + (kRough << 20); }
+DENSE_FX bool rough(const double g[4]) { return rough(g, exponent_of(g)); }
 // 6 (h - lf_2) of one reconstruction.
 template <bool Z>
 DENSE_FX double correction(const double g[4]) {

@@ -77,3 +77,15 @@ def test_flux_change(lines, kind):
     assert int(odd) == 0
     assert rms <= 1.02 * rms64
     assert worst <= 2.0 * worst64
+
+
+@pytest.mark.parametrize("decades", [-2, -1, 0, 1, 4])
+@pytest.mark.parametrize("kind", range(4))
+@pytest.mark.parametrize("z", [0, 1])
+def test_taped_gradient(lines, z, kind, decades):
+    """The taped gradient on the exponent two stencils share: smooth ones, a jump in its own stencil, one
+    in its partner, and rough ones, no less exact than weno_grad's (the worst to a factor of two)."""
+    ((rms, rms64, worst, worst64),) = [[float(v) for v in x[4:]] for x in lines
+                                       if x[0] == "taped" and x[1:4] == [str(z), str(kind), str(decades)]]
+    assert rms <= 1.02 * rms64
+    assert worst <= 2.0 * worst64

@@ -302,7 +302,70 @@ void change(int kind) {
     err.print();
 }
 
+// dW/dlf[m] from the first differences, written out (the five sum to one)
+template <bool Z> void gradient_of(const double g[4], ld G[5]) {
+    const ld ss = (double)1.0e-6f, cs[3] = {0.1L, 0.6L, 0.3L};
+    const ld A[3] = {(ld)g[0] - g[1], (ld)g[1] - g[2], (ld)g[2] - g[3]};
+    const ld B[3] = {g[0] - 3 * (ld)g[1], (ld)g[1] + g[2], 3 * (ld)g[2] - g[3]};
+    const ld q[3] = {(2 * (ld)g[0] - 5 * (ld)g[1]) / 6, (-(ld)g[1] - 2 * (ld)g[2]) / 6, ((ld)g[3] - 4 * (ld)g[2]) / 6};
+    const ld a[3][5] = {{1 / 3.L, -7 / 6.L, 11 / 6.L, 0, 0}, {0, -1 / 6.L, 5 / 6.L, 1 / 3.L, 0}, {0, 0, 1 / 3.L, 5 / 6.L, -1 / 6.L}};
+    const ld dA[3][5] = {{1, -2, 1, 0, 0}, {0, 1, -2, 1, 0}, {0, 0, 1, -2, 1}};
+    const ld dB[3][5] = {{1, -4, 3, 0, 0}, {0, 1, 0, -1, 0}, {0, 0, 3, -4, 1}};
+    ld be[3], d[3], al[3], db[3], S = 0, W = 0, st = 0;
+    for (int k = 0; k < 3; ++k) { be[k] = 13 * A[k] * A[k] / 12 + B[k] * B[k] / 4; d[k] = ss + be[k]; }
+    const ld tau = fabsl(be[2] - be[0]);
+    for (int k = 0; k < 3; ++k) { al[k] = Z ? cs[k] * (1 + tau * tau / (d[k] * d[k])) : cs[k] / (d[k] * d[k]); S += al[k]; }
+    for (int k = 0; k < 3; ++k) W += al[k] * q[k] / S;
+    for (int k = 0; k < 3; ++k) {
+        const ld e = (q[k] - W) / S;
+        db[k] = Z ? -2 * e * cs[k] * tau * tau / (d[k] * d[k] * d[k]) : -2 * e * al[k] / d[k];
+        if (Z) st += 2 * e * cs[k] * tau / (d[k] * d[k]);
+    }
+    if (be[2] >= be[0]) { db[2] += st; db[0] -= st; } else { db[2] -= st; db[0] += st; }
+    for (int m = 0; m < 5; ++m) {
+        G[m] = 0;
+        for (int k = 0; k < 3; ++k) G[m] += al[k] / S * a[k][m] + db[k] * (13 * A[k] * dA[k][m] / 6 + B[k] * dB[k][m] / 2);
+    }
+}
+// the taped gradient of a stencil as the component-wise sweeps form it, on the exponent it shares with its
+// partner, beside weno_grad's. kind 0: both smooth; 1: a jump of 10^decades times the level in this one;
+// 2: in the partner; 3: both rough
+template <bool Z> void taped(int kind, int decades) {
+    std::mt19937_64 r(171 + 10 * kind + decades);
+    Errors err;
+    for (int t = 0; t < 20000; ++t) {
+        const double level = std::pow(10.0, 2 * draw(r)), amp = level * std::pow(10.0, -1.5 + 1.5 * draw(r));
+        double g[2][4], G[5], G64[5];
+        for (int s = 0; s < 2; ++s) {
+            const double a = draw(r), b = 0.3 * draw(r), c = 0.1 * draw(r), jump = level * std::pow(10.0, decades) * (1 + 0.5 * draw(r));
+            const int j = (int)(r() % 4);
+            for (int m = 0; m < 4; ++m)
+                g[s][m] = (kind == 3 ? level * draw(r) : amp * (a + b * (m - 1.5) + c * (m - 1.5) * (m - 1.5))) +
+                          (kind == 1 + s && m == j ? jump : 0.0);
+        }
+        fx::u32 top = 0;
+        const fx::u32 e0 = fx::scale_of(g[0], top), eh = fx::umax(e0, fx::scale_of(g[1], top));
+        fx::Gradient q;
+        fx::correction6_taped<Z>(g[0], eh, q);
+        weno_grad_of<Z>(g[0], G64);
+        if (fx::rough(g[0], eh)) weno_grad_of<Z>(g[0], G);
+        else fx::gradient_out(q, top, G);
+        ld want[5];
+        gradient_of<Z>(g[0], want);
+        double e = 0, e64 = 0;
+        for (int m = 0; m < 5; ++m) {
+            e = std::max(e, (double)fabsl(G[m] - want[m]));
+            e64 = std::max(e64, (double)fabsl(G64[m] - want[m]));
+        }
+        err.add(e, e64);
+    }
+    printf("taped %d %d %d ", (int)Z, kind, decades);
+    err.print();
+}
+
 int main() {
+    for (int kind = 0; kind < 4; ++kind)
+        for (int decades : {-2, -1, 0, 1, 4}) { taped<false>(kind, decades); taped<true>(kind, decades); }
     for (int kind = 0; kind < 4; ++kind) change(kind);
     for (double delta : {0.0, 0.001, 0.01, 0.5, 0.9})
         for (int decades : {-3, 0, 2, 6, 10}) borrowed(delta, decades);
