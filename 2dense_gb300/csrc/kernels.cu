@@ -539,7 +539,7 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
                     fx::Gradient q;
                     const fx::i64 cs = fx::correction6_taped<Z>(gd, eh, q);
                     c += s == 0 ? cs : -cs;
-                    if (fx::rough(gd, eh)) weno_grad_of<Z>(gd, g);
+                    if (fx::rough<Z>(gd, eh)) weno_grad_of<Z>(gd, g);
                     else fx::gradient_out(q, top, g);
 #pragma unroll
                     for (int m = 0; m < 5; ++m) tape_at[((5 * s + m) * 4 + v) * ts] = g[m];

@@ -348,7 +348,7 @@ template <bool Z> void taped(int kind, int decades) {
         fx::Gradient q;
         fx::correction6_taped<Z>(g[0], eh, q);
         weno_grad_of<Z>(g[0], G64);
-        if (fx::rough(g[0], eh)) weno_grad_of<Z>(g[0], G);
+        if (fx::rough<Z>(g[0], eh)) weno_grad_of<Z>(g[0], G);
         else fx::gradient_out(q, top, G);
         ld want[5];
         gradient_of<Z>(g[0], want);
