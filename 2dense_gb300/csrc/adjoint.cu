@@ -904,8 +904,8 @@ __device__ __forceinline__ void char_face_block(const AdjParams& a, const double
                 fx::u32 top = 0;
                 const fx::u32 eh = fx::scale_of(gd, top);
                 fx::Gradient q;
-                const double cv = fx::to_double(fx::correction6_taped<true>(gd, eh, q), eh, top) * (1.0 / 6.0);
-                if (fx::rough(gd)) weno_grad_of<true>(gd, G);
+                double cv = fx::to_double(fx::correction6_taped<true>(gd, eh, q), eh, top) * (1.0 / 6.0);
+                if (fx::rough<true>(gd, eh)) cv = weno_grad_of<true>(gd, G);  // (beside a jump: value and gradient)
                 else fx::gradient_out(q, top, G);
                 const double cb = sL[20 + k][tid];
                 sL[20 + k][tid] = cv;

@@ -121,15 +121,16 @@ __device__ __forceinline__ void weno_grad(const double gd[4], const double B[3],
     g[2] = 1.0 - ((g[0] + g[1]) + (g[3] + g[4]));
 }
 
-// The gradient from a stencil's first differences alone.
+// The gradient from a stencil's first differences alone; returns h - lf_2.
 template <bool Z>
-__device__ __forceinline__ void weno_grad_of(const double gd[4], double g[5]) {
+__device__ __forceinline__ double weno_grad_of(const double gd[4], double g[5]) {
     double d0, d1, d2, B[3];
     betas_g(gd, d0, d1, d2, B);
     WenoTerms t;
     weno_terms<Z>(gd, d0, d1, d2, t);
-    const double iN = fx::rcp(t.N);
-    weno_grad<Z>(gd, B, d0, d1, d2, t, weno_num(t) * iN, iN, g);
+    const double iN = fx::rcp(t.N), corr = weno_num(t) * iN;
+    weno_grad<Z>(gd, B, d0, d1, d2, t, corr, iN, g);
+    return corr;
 }
 
 // The weights' share alone of a reconstruction's stencil gradient, for weights computed from one

@@ -8,6 +8,8 @@ import numpy as np
 import pytest
 import torch
 
+import torch_step
+
 pytestmark = pytest.mark.gpu
 
 THIN = 1e-8
@@ -70,3 +72,25 @@ def test_thin_side_characteristic(dense, split, axis, n):
     size = max(np.abs(strict).max(), THIN * 3.0 / min(c.dx, c.dy))
     assert size < 1e-4 * 3.0 / min(c.dx, c.dy)
     assert np.abs(fast - strict).max() <= 1e-12 * size
+
+
+@pytest.mark.parametrize("axis", [0, 1])
+@pytest.mark.parametrize("split,recon", [(101, 253), (101, 255), (103, 255), (104, 0), (105, 0)])
+def test_thin_side_adjoint(dense, split, recon, axis):
+    """The transposed Jacobian for weights on thin cells three and more from the jumps, at the thin cells
+    beside those, against autograd through the PyTorch step; entries there are of order one whatever
+    the density, so a field's value is needed to its own digits. 1e-10 as on smooth states."""
+    adjoint = importlib.import_module("2dense_gb300.adjoint")
+    c = dense.init_general(dense.config_default(ni=40, nj=48, benchmark=11, splitting=split, recon=recon, cfl=0.5))[0]
+    U = torch.from_numpy(np.ascontiguousarray(state(c, axis, True)[4:-4, 4:-4].transpose(2, 1, 0))).cuda()
+    m, dim = (c.ni, 2) if axis == 0 else (c.nj, 1)
+    rows = torch.arange(m // 2 + 2, m - 2, device="cuda")
+    v = torch.zeros_like(U)
+    w = torch.randn(U.shape, generator=torch.Generator().manual_seed(7), dtype=torch.float64).cuda()
+    v.index_copy_(dim, rows, w.index_select(dim, rows))
+    with adjoint.Adjoint(c) as adj:
+        out, _ = adj.rhs_vjp(U, v)
+    Ut = U.clone().requires_grad_(True)
+    (ref,) = torch.autograd.grad(torch_step.rhs(Ut, c.gamma, c.dx, c.dy, recon, split, delta=c.delta), Ut, v)
+    out, ref = (x.index_select(dim, rows) for x in (out, ref))
+    assert float((out - ref).abs().max() / ref.abs().max()) < 1e-10
