@@ -245,10 +245,12 @@ int build_step_graph(dense_handle* h) {
     return DENSE_OK;
 }
 
-// rhs[v][j][i] = -(hx[v][j][i+1] - hx[v][j][i])/dx - (he[v][j+1][i] - he[v][j][i])/dy, with 1/dx
-// and 1/dy (eight IEEE divides a cell took 33 of the 237 us of a 481 x 479 call)
-__global__ void k_rhs(const double* __restrict__ hx, const double* __restrict__ he, int ni, int nj, double idx,
-                      double idy, double* __restrict__ rhs) {
+// rhs[v][j][i] = -(hx[v][j][i+1] - hx[v][j][i])/dx - (he[v][j+1][i] - he[v][j][i])/dy: the strict variant in these
+// operations, the others with 1/dx and 1/dy in place of dx and dy (eight IEEE divides a cell took 33 of
+// the 237 us of a 481 x 479 call)
+template <bool STRICT>
+__global__ void k_rhs(const double* __restrict__ hx, const double* __restrict__ he, int ni, int nj, double dx,
+                      double dy, double* __restrict__ rhs) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= ni || j >= nj) return;
     const long long xs = (long long)nj * (ni + 1), ys = (long long)(nj + 1) * ni;
@@ -256,7 +258,8 @@ __global__ void k_rhs(const double* __restrict__ hx, const double* __restrict__ 
     for (int v = 0; v < 4; ++v) {
         const double* X = hx + v * xs + (long long)j * (ni + 1) + i;
         const double* Y = he + v * ys + (long long)j * ni + i;
-        rhs[(long long)v * ni * nj + (long long)j * ni + i] = fma(X[0] - X[1], idx, (Y[0] - Y[ni]) * idy);
+        rhs[(long long)v * ni * nj + (long long)j * ni + i] =
+            STRICT ? -(X[1] - X[0]) / dx - (Y[ni] - Y[0]) / dy : fma(X[0] - X[1], dx, (Y[0] - Y[ni]) * dy);
     }
 }
 
@@ -643,8 +646,8 @@ int dense_rhs_device(dense_handle_t* h, int irk, double* rhs, void* stream) {
     h->kt->flux(h->prm, irk, 0, h->stream);
     h->kt->flux(h->prm, irk, 1, h->stream);
     const dim3 b(32, 8), g((h->cfg.ni + 31) / 32, (h->cfg.nj + 7) / 8);
-    k_rhs<<<g, b, 0, h->stream>>>(h->hx, h->he, h->cfg.ni, h->cfg.nj, 1.0 / h->cfg.dx, 1.0 / h->cfg.dy,
-                                    rhs);
+    if (h->cfg.strict == 1) k_rhs<true><<<g, b, 0, h->stream>>>(h->hx, h->he, h->cfg.ni, h->cfg.nj, h->cfg.dx, h->cfg.dy, rhs);
+    else k_rhs<false><<<g, b, 0, h->stream>>>(h->hx, h->he, h->cfg.ni, h->cfg.nj, 1.0 / h->cfg.dx, 1.0 / h->cfg.dy, rhs);
     h->launches += 2 + h->kt->flux_launches(h->prm, 0) + h->kt->flux_launches(h->prm, 1) + 1;
     rc = launch_check(h);
     if (rc) return rc;
