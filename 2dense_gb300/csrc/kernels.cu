@@ -1543,7 +1543,9 @@ __device__ __forceinline__ void bc_block(const Params& p, int bx) {
 // the 256 x 1024 Rayleigh-Taylor case took 0.127 (xi) and 0.111 ms (eta), at 768 0.131 and 0.113,
 // unbounded 0.141 and 0.158 (now 0.106 and 0.098, the roots on the integer pipes too; 0.340 and
 // 0.293 with the reconstructions in FP64).
-constexpr int char_min_blocks(bool adapt, int nt) { return adapt ? 768 / nt : 1024 / nt; }
+// (The checked ones gain alike.) The strict 104 sweeps have 142 registers without a bound and no spill: at 64
+// they spilled 528 bytes a thread, and the eta sweep of that case took 0.854 instead of 0.849 ms.
+constexpr int char_min_blocks(bool adapt, int nt) { return adapt ? 768 / nt : FAST ? 1024 / nt : 1; }
 // The four-thread tiles: five resident blocks (48 registers), which grids of a few blocks an SM need to
 // run as one wave (200 x 200 vortex, ten steps 0.927 -> 0.897 ms).
 template <int DIR, int SPL, int REC, int TX, int TY, bool TAPE = false, int TZ = 1>
@@ -1564,7 +1566,7 @@ __global__ void k_prim(Params p, int slot) {
 // cell); with the reciprocal and root of get_primary on the integer pipes 0.356 -> 0.283 ms of a 2048 x
 // 2048 stage, with the flux change there too 0.242 at five blocks and 0.235 at six (four 0.252; the flux
 // change in FP64 0.315; 200 B a cell at the copy rate: 0.124 ms).
-constexpr int kUpdateBlocks = 6;
+constexpr int kUpdateBlocks = FAST ? 6 : 4;  // (strict spills at 42 registers, not at 64)
 template <int IRK>
 __global__ void __launch_bounds__(256, kUpdateBlocks) k_update(Params p) {
     grid_dependency_wait();
