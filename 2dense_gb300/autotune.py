@@ -14,18 +14,19 @@ so the tuner is free to pick whichever is fastest for the batch at hand.
 The search is a coordinate descent (launch mode, order, xi tile, eta tile, repeated until a pass
 changes nothing, at most three passes), each candidate timed on a scratch copy of the batch (same
 configurations, same initial states) so the caller's solution is untouched. The winner is cached
-in a JSON file keyed by device, scheme and the histogram of instance sizes, so a second batch of
-the same shape reuses it without timing.
+in a JSON file keyed by device, scheme, the histogram of instance sizes and the kernels' sources, so a
+second batch of the same shape reuses it without timing until the kernels change.
 """
 from __future__ import annotations
 
 import ctypes
+import functools
 import hashlib
 import json
 import os
 import time
 
-from . import _abi
+from . import _abi, build
 from .solver import BatchSolver, init_general
 
 CACHE = os.environ.get("DENSE2D_AUTOTUNE_CACHE",
@@ -56,11 +57,17 @@ def _device_key() -> str:
         return "cuda"
 
 
+@functools.lru_cache(maxsize=1)
+def _kernels_key() -> str:
+    """The kernels' sources: a schedule timed on other kernels is timed again."""
+    return build.source_digest()[:12]
+
+
 def batch_key(cfgs) -> str:
     sizes = sorted((c.ni, c.nj) for c in cfgs)
     h = hashlib.sha1(json.dumps(sizes).encode()).hexdigest()[:16]
     c0 = cfgs[0]
-    return f"{_device_key()}|{c0.splitting}|{c0.recon}|{c0.strict}|n{len(cfgs)}|{h}|modes"
+    return f"{_device_key()}|{c0.splitting}|{c0.recon}|{c0.strict}|n{len(cfgs)}|{h}|modes|{_kernels_key()}"
 
 
 def _load_cache() -> dict:

@@ -17,6 +17,7 @@ The ptxas resource report of each kernel (registers, spills, shared memory) is w
 """
 from __future__ import annotations
 
+import hashlib
 import os
 import shutil
 import subprocess
@@ -46,6 +47,16 @@ def _sources() -> list[str]:
             if f.endswith((".cu", ".cuh", ".h", ".cpp")):
                 out.append(os.path.join(d, f))
     return out
+
+
+def source_digest() -> str:
+    """SHA-1 of the library's sources: what a result measured on its kernels is valid for."""
+    h = hashlib.sha1()
+    for path in sorted(_sources()):
+        h.update(os.path.basename(path).encode() + b"\0")
+        with open(path, "rb") as f:
+            h.update(f.read())
+    return h.hexdigest()
 
 
 def _stale() -> bool:
