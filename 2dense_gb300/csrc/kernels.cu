@@ -1068,7 +1068,6 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
             if (smooth[s]) {
                 double F[5][4], h[4];
                 stencil(tx, ty, s, F);
-#if !FAST
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     double lf[5], q0, q1, q2;
@@ -1077,7 +1076,6 @@ __device__ __forceinline__ void flux_char_block(const Params& p, int irk, int bx
                     candidates(lf, q0, q1, q2);
                     h[c] = wsur[s][0] * q0 + wsur[s][1] * q1 + wsur[s][2] * q2;
                 }
-#endif
 #pragma unroll
                 for (int c = 0; c < 4; ++c) hbuf(s, c, tid) = h[c];
             } else {
