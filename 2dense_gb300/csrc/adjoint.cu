@@ -863,8 +863,7 @@ __device__ __forceinline__ void char_face_block(const AdjParams& a, const double
         for (int v = 0; v < 4; ++v) HB[v] = hb[(DIR == 0 ? 0 : 4 * a.xs) + v * ts + to];
         if (any_char) {  // a face whose signs are both smooth never forms its Roe average
             r = fx::rcp(sl + sr);
-            const double wr = sr * r;
-            u0 = fma(wr, ur - ul, ul); v0 = fma(wr, vr - vl, vl); h0 = fma(wr, hr - hl, hl);
+            u0 = fma(sr, ur, sl * ul) * r; v0 = fma(sr, vr, sl * vl) * r; h0 = fma(sr, hr, sl * hl) * r;
             uu0 = 0.5 * fma(u0, u0, v0 * v0);
             c2 = g1 * (h0 - uu0);
             ia = fx::rsqrt(c2); a0 = c2 * ia;

@@ -22,10 +22,12 @@ struct EigFast {
 template <int DIR>
 __device__ __forceinline__ bool roe_eig_fast(double g1, double sl, double sr, double ul, double ur,
                                              double vl, double vr, double hl, double hr, EigFast& e) {
-    const double w = sr * fx::rcp(sl + sr);
-    const double u0 = fma(w, ur - ul, ul);
-    const double v0 = fma(w, vr - vl, vl);
-    e.h0 = fma(w, hr - hl, hl);
+    // (each mean as one sum: about either side's value it would keep that value's rounding, which the other
+    // side's weight may dwarf -- of an enthalpy 1e8 times the other's at that density ratio, 1e-12 of the mean)
+    const double r = fx::rcp(sl + sr);
+    const double u0 = fma(sr, ur, sl * ul) * r;
+    const double v0 = fma(sr, vr, sl * vl) * r;
+    e.h0 = fma(sr, hr, sl * hl) * r;
     e.uu0 = 0.5 * fma(u0, u0, v0 * v0);
     const double c2 = g1 * (e.h0 - e.uu0);
     const double ia = fx::rsqrt(c2);

@@ -89,3 +89,11 @@ def test_taped_gradient(lines, z, kind, decades):
                                        if x[0] == "taped" and x[1:4] == [str(z), str(kind), str(decades)]]
     assert rms <= 1.02 * rms64
     assert worst <= 2.0 * worst64
+
+
+@pytest.mark.parametrize("decades", [0, 2, 4, 8])
+def test_roe_means(lines, decades):
+    """The Roe averages of two cells of very different density, relative to the mean of the magnitudes: two
+    products and a sum, a sum and its reciprocal, their product, half an ulp each: 6 x 2^-53."""
+    ((worst,),) = [x[2:] for x in lines if x[0] == "means" and x[1] == str(decades)]
+    assert float(worst) <= 6.0

@@ -363,7 +363,28 @@ template <bool Z> void taped(int kind, int decades) {
     err.print();
 }
 
+// the Roe means of two cells whose densities are up to 10^decades apart, the enthalpies the other way
+// round: relative to the weighted mean of the magnitudes, in units of 2^-53
+void means(int decades) {
+    std::mt19937_64 r(211 + decades);
+    double worst = 0;
+    for (int t = 0; t < 20000; ++t) {
+        const double f = std::pow(10.0, decades * draw(r)), sl = std::sqrt(1 + std::fabs(draw(r))), sr = std::sqrt(f * (1 + std::fabs(draw(r))));
+        const double ul = draw(r) * std::pow(10.0, 3 * draw(r)), ur = draw(r) * std::pow(10.0, 3 * draw(r));
+        const double hl = 20 + 1e6 * f, hr = 20 + 1e6;  // (above the velocities' squares over two)
+        EigFast e;
+        roe_eig_fast<0>(0.4, sl, sr, ul, ur, 0.5 * ur, 0.5 * ul, hl + ul * ul + ur * ur, hr + ul * ul + ur * ur, e);
+        const ld HL = hl + ul * ul + ur * ur, HR = hr + ul * ul + ur * ur;
+        auto mean = [&](ld l, ld x) { return (sl * l + sr * x) / ((ld)sl + sr); };
+        worst = std::max(worst, (double)(fabsl(e.un0 - mean(ul, ur)) / mean(std::fabs(ul), std::fabs(ur)) / 0x1p-53L));
+        worst = std::max(worst, (double)(fabsl(e.ut0 - mean(0.5 * ur, 0.5 * ul)) / mean(0.5 * std::fabs(ur), 0.5 * std::fabs(ul)) / 0x1p-53L));
+        worst = std::max(worst, (double)(fabsl(e.h0 - mean((double)HL, (double)HR)) / mean((double)HL, (double)HR) / 0x1p-53L));
+    }
+    printf("means %d %.17g\n", decades, worst);
+}
+
 int main() {
+    for (int decades : {0, 2, 4, 8}) means(decades);
     for (int kind = 0; kind < 4; ++kind)
         for (int decades : {-2, -1, 0, 1, 4}) { taped<false>(kind, decades); taped<true>(kind, decades); }
     for (int kind = 0; kind < 4; ++kind) change(kind);
