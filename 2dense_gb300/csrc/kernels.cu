@@ -399,7 +399,8 @@ struct CwTile {
     static constexpr int NC = DIR == 0 ? TX + 5 : TX;   // smem columns
     static constexpr int NCELL = NL * NC;
     static constexpr bool kStageG = FAST && REC != DENSE_RECON_UPWIND5;
-    static constexpr size_t bytes = sizeof(double) * (size_t)NCELL * (kStageG ? 16 : 8);
+    // (and the queue of the values left to FP64: its length and four 16-bit items an interface)
+    static constexpr size_t bytes = sizeof(double) * (size_t)NCELL * (kStageG ? 16 : 8) + (kStageG ? 16 + 8 * TX * TY : 0);
 };
 
 // The position of the (n + 1)-th set bit of m, which has more than n.
@@ -584,8 +585,8 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
             // took the FP64 pipe for a few lanes (steps of 240 x 240 Steger-Warming 1.78 ms; so 1.70).
             constexpr bool Z = REC == DENSE_RECON_WENOZ5;
             constexpr int NT = TX * TY * TZ;
-            __shared__ unsigned short items[4 * TX * TY];
-            __shared__ int count;
+            int& count = *(int*)(dsm + 16 * NCELL);
+            unsigned short* const items = (unsigned short*)(dsm + 16 * NCELL + 2);
             const int lane = lt & 31, s = lane & 1;
             if (lt == 0) count = 0;
             __syncthreads();
@@ -651,7 +652,7 @@ __global__ void k_flux_noop(Params p, int irk) {
 // What bounds it: the FP64 pipe. The surrogate's weights and the smooth branch run on the integer
 // pipes (weno_fixed.cuh), which leaves some 55 FP64 instructions an interface of 150 and took the
 // 1920 x 480 double Mach reflection's sweeps from 0.282 and 0.305 ms to 0.149 and 0.172 (0.139 and 0.141
-// with tiles of 128 threads).
+// with tiles of 128 threads; 0.147 both with the fields left to FP64 beside its shocks).
 // Dynamic shared memory of one characteristic sweep block, in doubles: the tile's split fluxes
 // sF[8][NL][NC] and primitives sQ[4][NL][NC]; per-cell sqrt(rho) sS (104, fast); the split fluxes'
 // forward differences along the sweep sDF[8][NL][NC] (fast); and one region R that AdaWENO uses
@@ -1535,14 +1536,13 @@ __device__ __forceinline__ void bc_block(const Params& p, int bx) {
 // blocks stall on the barriers of their work queue, which 768 resident threads per SM hide (80
 // registers, a few bytes spilled; sweeps of the 1920 x 480 double Mach reflection in blocks of 256, xi
 // and eta: 0.159 and 0.180 ms at 768, 0.180 and 0.203 at 512, 0.162 and 0.188 at 1024; steps in blocks
-// of 128: 3.97 ms at 768, 4.00 at 640). The 104
-// sweeps' four inlined integer
-// reconstructions would take 160 registers; at 1024 resident threads (64 registers) the sweeps of
-// the 256 x 1024 Rayleigh-Taylor case took 0.127 (xi) and 0.111 ms (eta), at 768 0.131 and 0.113,
-// unbounded 0.141 and 0.158 (now 0.106 and 0.098, the roots on the integer pipes too; 0.340 and
-// 0.293 with the reconstructions in FP64).
-// (The checked ones gain alike.) The strict 104 sweeps have 142 registers without a bound and no spill: at 64
-// they spilled 528 bytes a thread, and the eta sweep of that case took 0.854 instead of 0.849 ms.
+// of 128: 3.97 ms at 768, 4.00 at 640). The 104 sweeps' four inlined integer reconstructions would
+// take 160 registers; at 1024 resident threads (64 registers) the sweeps of the 256 x 1024
+// Rayleigh-Taylor case took 0.127 (xi) and 0.111 ms (eta), at 768 0.131 and 0.113, unbounded 0.141
+// and 0.158 (now 0.109 and 0.094, the roots on the integer pipes too; 0.340 and 0.293 with the
+// reconstructions in FP64; the checked ones gain alike). The strict 104 sweeps have 142 registers
+// without a bound and no spill: at 64 they spilled 528 bytes a thread, and the eta sweep of that case
+// took 0.854 instead of 0.849 ms.
 constexpr int char_min_blocks(bool adapt, int nt) { return adapt ? 768 / nt : FAST ? 1024 / nt : 1; }
 // The four-thread tiles: five resident blocks (48 registers), which grids of a few blocks an SM need to
 // run as one wave (200 x 200 vortex, ten steps 0.927 -> 0.897 ms).
@@ -1782,7 +1782,8 @@ kb_persist(const Params* tab, PersistLaunch L, int xi_variant, int eta_variant) 
 // slowest warp. Sweeps (xi, eta) against tiles of 32 x 4 and 8 x 32: 2048 x 2048 LLF + WENO-JS 0.682 and
 // 0.668 -> 0.675 and 0.657 ms, 1024 x 1024 GLF + upwind 0.157 and 0.131 -> 0.143 and 0.131, 481 x 479
 // Steger-Warming + WENO-Z 0.069 and 0.071 -> 0.067 and 0.064. Steps, the last: 4.26 -> 4.08 ms (xi 128 x 1:
-// 4.01, but 5 % slower on a 512 x 512 vortex; 96 x 1: 4.21; eta 4 x 16: 4.36; 8 x 64: 4.75).
+// 4.01, but 5 % slower on a 512 x 512 vortex; 96 x 1: 4.21; eta 4 x 16: 4.36; 8 x 64: 4.75). (All tiles
+// were compared before the values beside jumps went to FP64, which adds 1 to 5 % to each.)
 constexpr int kXTX = 64, kXTY = 2, kXSTX = 32, kXSTY = 2;  // xi tile; on small grids
 constexpr int kETX = 4, kETY = 32, kESTX = 8, kESTY = 8;   // eta tile; on small grids
 // 104 sweeps: 32 interfaces x 4 rows, 4 columns x 32 interfaces. Steps of the Rayleigh-Taylor case
