@@ -789,7 +789,7 @@ __device__ __forceinline__ void fetch_cell(const AdjParams& a, const double* __r
 // and split computed once, not once per reading face), and each thread parks its fields'
 // differences, then their gradients there too: the field loop is not unrolled, so that its one
 // copy of the integer gradient stays in the instruction cache. The transposed Jacobian of the 128 x
-// 512 Rayleigh-Taylor case, where both directions' face kernels took 0.43 of 0.75 ms, takes 0.58 ms.
+// 512 Rayleigh-Taylor case, where both directions' face kernels took 0.43 of 0.75 ms, takes 0.52 ms.
 template <int DIR>
 __device__ __forceinline__ void char_face_block(const AdjParams& a, const double* __restrict__ u,
                                                 const double* __restrict__ hb, const double* __restrict__ lamv,

@@ -42,10 +42,10 @@ struct Scalars {
     double dt_save;
 };
 
-// Everything a kernel needs, passed by value.
 // Cells below which an AdaWENO grid takes its sweeps' small-grid tiles and programmatic graph edges.
 constexpr long long kAdaptiveSmall = 80000;
 
+// Everything a kernel needs, passed by value.
 struct Params {
     double* cons;    // [4][NJp][P] padded conserved variables
     double* prim;    // [5][NJp][P] padded rho,u,v,p,alpha

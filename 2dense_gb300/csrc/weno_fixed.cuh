@@ -6,12 +6,12 @@
 // product. A reconstruction in FP64 is about 34 instructions, 556 (JS) to 668 (Z) cycles with the
 // integer pipes idle; the same value in 64-bit integers takes 172 and 205, and leaves the FP64 pipe
 // to the split fluxes of other warps. The component-wise xi sweep of a 2048 x 2048 LLF stage went
-// from 2.414 to 0.684 ms (JS) and from 2.773 to 0.778 ms (Z), the eta sweep from 2.301 to 0.663 and
-// from 2.657 to 0.772 ms; what bounds them now is the integer ALU (72 % busy, 340 instructions a
-// reconstruction before its last trimming). The words carry 57 to
-// 64 significant bits where a double carries 53, but counted from a stencil's largest difference; on
-// the small side of a jump, where that says too little, FP64 takes over (enough, weno_value.cuh: 1 to
-// 2 % of the time of a step, the test above all).
+// from 2.414 to 0.684 ms (JS) and from 2.773 to 0.780 ms (Z), the eta sweep from 2.301 to 0.655 and
+// from 2.657 to 0.754 ms; what bounds them now is the integer ALU (71 % busy) and issue. A word
+// carries 57 to 64 significant bits where a double carries 53, but they count from a stencil's largest
+// difference; on the small side of a jump, where that says too little, FP64 takes over (enough,
+// weno_value.cuh): 1 % of these sweeps for the test alone, 2 to 4 % of the time of the steps of a
+// captured shock.
 //
 // The value. With g_m = lf_m - lf_(m+1), A_k = g_k - g_(k+1), B_0 = A_0 - 2 g_1, B_1 = g_1 + g_2,
 // B_2 = A_2 + 2 g_2 and d_k = 4 (ss + beta_k) = 4 ss + 13/3 A_k^2 + B_k^2 (weno_fast.cuh), the
@@ -29,7 +29,8 @@
 //    third-order step;
 //  * every rounding is a truncation of magnitudes, so a change of sign of the data changes the
 //    sign of the result and nothing else: mirror-symmetric flows stay so bit for bit.
-// A NaN or infinity among the differences gives NaN. Against long double over random smooth,
+// A NaN or infinity among the differences, or a difference from 2^977 on, gives NaN (in FP64 the
+// indicators' products overflow from 2^75 on). Against long double over random smooth,
 // discontinuous and rough stencils the error's rms is 0.57 to 0.86 of the FP64 form's, its maximum
 // 0.58 to 1.0; relative to the small side of a jump, where FP64 takes over, 0.6 to 1.0 and 0.6 to 1.1.
 //

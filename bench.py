@@ -16,7 +16,8 @@ Reported on one JSON line (rank 0):
                the state back (dense_download);
   roofline     the dominant kernel (the xi-direction flux sweep) against the FP64 peak measured
                live on this GPU (dense_measure_fp64, an FMA-throughput probe): achieved = the
-               reference algorithm's FLOPs for that sweep per launch / its mean CUDA-event time;
+               reference algorithm's FLOPs for that sweep per launch / its mean CUDA-event time (no
+               bound: the reconstructions are done in integers);
   cpu_baseline the CPU oracle (a line-faithful C++ restatement of the reference, OpenMP) on
                this host's cores, on a bounded sample of the same workload.
 With --impl reference the CPU restatement of the reference (the Fortran itself cannot be built
@@ -51,6 +52,8 @@ WORKLOADS = {
 }
 METRIC = "FP64 WENO5-RK3 cell-updates/s"
 UNIT = "cell-updates/s"
+# what the profiles show the sweeps to be bound by; "peak" and "frac" are the FP64 pipe's
+BOUND = "integer pipes and issue"
 
 
 def dist_info():
@@ -335,7 +338,7 @@ def run_batched(args, dense, lib):
                                   "what": "every instance's state after the warm-up and timed steps, "
                                           "batched against its own plain solve"},
             "gpu_launches": launches,
-            "roofline": {"bound": "fp64", "achieved": fl["flops_per_cell_update"] * value / 1e12,
+            "roofline": {"bound": BOUND, "achieved": fl["flops_per_cell_update"] * value / 1e12,
                          "peak": peak.value / 1e12, "unit": "TFLOP/s",
                          "frac": fl["flops_per_cell_update"] * value / peak.value,
                          "flops_per_cell_update": fl["flops_per_cell_update"], "traffic": None},
@@ -494,7 +497,7 @@ def run_adjoint(args, dense, lib):
                     "d2h_bytes_per_step": (g_host[0].numel() + g_host[1].numel()) * 8,
                     "note": "perturbation field from pinned host memory, forward, backward, gradients to host"},
             "gpu_launches": launches,
-            "roofline": {"bound": "fp64", "achieved": fl["flops_per_cell_update"] * cells * n / (plain_ms * 1e-3) / 1e12,
+            "roofline": {"bound": BOUND, "achieved": fl["flops_per_cell_update"] * cells * n / (plain_ms * 1e-3) / 1e12,
                          "peak": peak.value / 1e12, "unit": "TFLOP/s",
                          "frac": fl["flops_per_cell_update"] * cells * n / (plain_ms * 1e-3) / peak.value,
                          "of": "the plain forward's reference FLOPs", "traffic": None},
@@ -676,11 +679,11 @@ def main():
         xi_flops = fl["flux_xi_per_cell_update"] / 3.0 * cells
     achieved = xi_flops / (xi_ms * 1e-3) / 1e12
     kname = {104: "k_flux_char<0,false>", 105: "k_flux_char<0,true>"}.get(split, "k_flux_cw<0,...>")
-    roofline = {"bound": "fp64", "kernel": f"xi flux sweep ({kname})",
+    roofline = {"bound": BOUND, "kernel": f"xi flux sweep ({kname})",
                 "achieved": achieved, "peak": peak.value / 1e12, "unit": "TFLOP/s",
                 "frac": achieved * 1e12 / peak.value,
-                "frac_note": "the reference's FP64 operations over the FP64 peak; the default kernels do the "
-                             "reconstructions in 64-bit integers beside that pipe, so it can exceed 1",
+                "frac_note": "the reference's FP64 operations over the FP64 peak, which is no bound: the default "
+                             "kernels do the reconstructions in 64-bit integers beside that pipe, so it can exceed 1",
                 "peak_source": "measured live: dense_measure_fp64 FMA-throughput probe on this GPU "
                                "(MEASURED_PEAKS.json has no FP64 figure)",
                 "traffic": None,
