@@ -1545,9 +1545,11 @@ __device__ __forceinline__ void bc_block(const Params& p, int bx) {
 // took 0.854 instead of 0.849 ms.
 constexpr int char_min_blocks(bool adapt, int nt) { return adapt ? 768 / nt : FAST ? 1024 / nt : 1; }
 // The four-thread tiles: five resident blocks (48 registers), which grids of a few blocks an SM need to
-// run as one wave (200 x 200 vortex, ten steps 0.927 -> 0.897 ms).
+// run as one wave (200 x 200 vortex, ten steps 0.927 -> 0.897 ms). (The strict ones take 58 and 72
+// registers and would spill 8 to 96 bytes a thread; they have no bound.)
+constexpr int cw_min_blocks(int tz, bool tape) { return FAST && tz == 4 && !tape ? 5 : 0; }
 template <int DIR, int SPL, int REC, int TX, int TY, bool TAPE = false, int TZ = 1>
-__global__ void __launch_bounds__(TX* TY* TZ, TZ == 4 && !TAPE ? 5 : 0) k_flux_cw(Params p, int irk) {
+__global__ void __launch_bounds__(TX* TY* TZ, cw_min_blocks(TZ, TAPE)) k_flux_cw(Params p, int irk) {
     grid_dependency_wait();
     flux_cw_block<DIR, SPL, REC, TX, TY, TAPE, TZ>(p, irk, blockIdx.x, blockIdx.y + gridDim.y * blockIdx.z);
 }

@@ -1,5 +1,5 @@
-"""The register bounds of the launch configurations were chosen on the fast kernels; the strict 104 sweeps
-and update keep theirs. Read from the compiler's resource report of the build."""
+"""The register bounds of the launch configurations were chosen on the fast kernels; the strict 104 sweeps,
+four-thread component-wise sweeps and update keep theirs. Read from the compiler's resource report of the build."""
 import os
 import re
 
@@ -21,6 +21,6 @@ def spills(dense, unit, kernel):
 
 
 # (k_flux_char<DIR, ADAPT = false, ...>: 104; AdaWENO's 80 registers bind every variant, as measured)
-@pytest.mark.parametrize("kernel", ["k_flux_charILi0ELb0", "k_flux_charILi1ELb0", "8k_update"])
+@pytest.mark.parametrize("kernel", ["k_flux_charILi0ELb0", "k_flux_charILi1ELb0", "9k_flux_cw", "8k_update"])
 def test_strict_kernels_do_not_spill(dense, kernel):
     assert set(spills(dense, "kernels_strict", kernel).values()) == {0}
