@@ -1564,8 +1564,8 @@ __global__ void k_prim(Params p, int slot) {
 }
 // Update: six resident blocks (42 registers). What bounded it was the FP64 pipe (50 instructions a
 // cell); with the reciprocal and root of get_primary on the integer pipes 0.356 -> 0.283 ms of a 2048 x
-// 2048 stage, with the flux change there too 0.242 at five blocks and 0.235 at six (four 0.252; the flux
-// change in FP64 0.315; 200 B a cell at the copy rate: 0.124 ms).
+// 2048 stage, with the flux change there too 0.242 at five blocks and 0.235 at six (four 0.252; its clamp
+// to infinity as an FP64 product 0.262, the whole in FP64 0.315; 200 B a cell at the copy rate: 0.124 ms).
 constexpr int kUpdateBlocks = FAST ? 6 : 4;  // (strict spills at 42 registers, not at 64)
 template <int IRK>
 __global__ void __launch_bounds__(256, kUpdateBlocks) k_update(Params p) {

@@ -469,11 +469,15 @@ DENSE_FX double flux_change(double xl, double xr, double yl, double yr, const Ra
     const int e = imax(x.e, y.e);
     const u64 a = shr(x.m, (u32)(e - x.e) + 1), b = shr(y.m, (u32)(e - y.e) + 1);
     const i64 t = (i64)((a ^ x.sign) - x.sign) + (i64)((b ^ y.sign) - y.sign);   // below 2^63
-    double d = to_double(t, (u32)imin(imax(e + 1, 64), 2040) << 20, 0);
-    if (e + 1 < 64) d = 0.0;
-    if (e + 1 > 2040) d = d * from_bits((u64)(1023 + imin(e + 1 - 2040, 1000)) << 52);  // (towards infinity)
-    if (top >= 0x7ff00000u || umax((u32)q.x.e, (u32)q.y.e) == (u32)kNoRate) d = from_bits(0x7ff8000000000000ull);
-    return from_bits(bits(d) ^ ((u64)q.sign << 32));
+    const u64 m = abs64(t);
+    const int n = clz64(m) & 63;
+    // (as to_double, with an infinity from 2^1024 on: a product in its place would take the FP64 pipe)
+    u64 r = ((u64)(imin(e, 3000) + 6 - n) << 52) + ((((m << n) >> 10) + 1) >> 1);
+    if (r >= 0x7ff0000000000000ull) r = 0x7ff0000000000000ull;
+    r |= (u64)t & 0x8000000000000000ull;
+    if (e + 1 < 64 || m == 0) r = 0;
+    if (top >= 0x7ff00000u || umax((u32)q.x.e, (u32)q.y.e) == (u32)kNoRate) r = 0x7ff8000000000000ull;
+    return from_bits(r ^ ((u64)q.sign << 32));
 }
 
 }  // namespace fx
