@@ -597,7 +597,8 @@ __device__ __forceinline__ void flux_cw_block(const Params& p, int irk, int bx, 
                 int base = 0;
                 if (lane == 0) base = atomicAdd(&count, __popc(m));
                 base = __shfl_sync(0xffffffffu, base, 0);
-                if (redo >> vz & 1u) items[base + __popc(m & ((1u << lane) - 1u))] = (unsigned short)((lt % (TX * TY)) * 4 + tz + vz * TZ);
+                if (redo >> vz & 1u)
+                    items[chk(p, base + __popc(m & ((1u << lane) - 1u)), 4 * TX * TY)] = (unsigned short)((lt % (TX * TY)) * 4 + tz + vz * TZ);
             }
             __syncthreads();
             const int n = count;
