@@ -653,7 +653,8 @@ __global__ void k_flux_noop(Params p, int irk) {
 // What bounds it: the FP64 pipe. The surrogate's weights and the smooth branch run on the integer
 // pipes (weno_fixed.cuh), which leaves some 55 FP64 instructions an interface of 150 and took the
 // 1920 x 480 double Mach reflection's sweeps from 0.282 and 0.305 ms to 0.149 and 0.172 (0.139 and 0.141
-// with tiles of 128 threads; 0.147 both with the fields left to FP64 beside its shocks).
+// with tiles of 128 threads; at the flow's middle, t = 0.1, 0.153 and 0.148, and with the fields left to
+// FP64 beside its shocks 0.166 and 0.154).
 // Dynamic shared memory of one characteristic sweep block, in doubles: the tile's split fluxes
 // sF[8][NL][NC] and primitives sQ[4][NL][NC]; per-cell sqrt(rho) sS (104, fast); the split fluxes'
 // forward differences along the sweep sDF[8][NL][NC] (fast); and one region R that AdaWENO uses
